@@ -43,13 +43,16 @@ def listed():
         # The headline workload, both modes: a large terrain at full HD.
         _frame("terrain_100m_1080p", points=100_000_000, w=1920, h=1080),
         _frame("terrain_100m_nearest_1080p", points=100_000_000, w=1920, h=1080, mode="nearest"),
-        # An export without level of detail (every point of the view drawn),
-        # in a window of odd size with a ragged last batch.
-        _frame("terrain_20m_all_points", points=19_999_981, w=1913, h=1077, clod=False),
+        # Without level of detail (every point of the view drawn), at an odd
+        # size, with a ragged last batch, for a consumer on the GPU (the copy
+        # of an image this cheap to draw would take longer than drawing it).
+        _frame("terrain_20m_all_points", points=19_999_981, w=1913, h=1077, clod=False,
+               out="planes"),
         # World-sized splats and hole filling: a closed surface.
         _frame("terrain_20m_splats", points=20_000_000, w=1920, h=1080, splat=0.5, fill=2),
         # The per-point effects (displacement and tint buffers).
-        _frame("terrain_10m_effects", points=10_000_000, w=1920, h=1080, effects=True),
+        _frame("terrain_10m_effects", points=10_000_000, w=1920, h=1080, effects=True,
+               out="planes"),
         # Many views of mixed sizes of one cloud in a call.
         {"name": "views_64_50m", "kind": "views", "points": 50_000_000, "views": 64},
         # The point under the cursor.
