@@ -42,8 +42,6 @@ struct PackScratch {
     uint32_t *idx[2] = {nullptr, nullptr};  // sort payload, ping-pong
     float4 *sorted = nullptr;               // positions in Morton order
     uint8_t *lv_morton = nullptr;           // levels in Morton order
-    uint8_t *lv_out = nullptr;              // levels in final order
-    uint32_t *perm = nullptr;               // final order -> Morton position
     uint32_t *grid = nullptr;               // dense LOD occupancy grid
     RadixScratch radix;                     // the sort's look-back words and histograms
     uint32_t *bounds = nullptr;             // 6 flipped words: min xyz, max xyz

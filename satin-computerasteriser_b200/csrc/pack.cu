@@ -17,12 +17,12 @@
 //                   to occupy an empty voxel"); the claims of a level ride
 //                   in the kernel before (the gather, or the previous
 //                   level's assignment)
-//   6 batches       one CTA per batch, a contiguous segment per warp:
-//                   AABB, level counts, stable level-ascending scatter (warp
-//                   ballots, no block barrier), RasterBatch with the
-//                   cumulative LOD counts
-//   7 emit          gather in final order, 30-bit quantisation into three
-//                   10-bit/axis words, colours, levels, source indices.
+//   6-7 batches     one CTA per batch, a contiguous segment per warp:
+//                   AABB, level counts, RasterBatch with the cumulative LOD
+//                   counts; stable level-ascending scatter (warp ballots, no
+//                   block barrier) of the points, quantised to 30 bits an
+//                   axis in three 10-bit/axis words, with colours, levels
+//                   and source indices.
 // Host-side float math (scale, voxel sizes, grid dims) is compiled without
 // contraction and uses the same operation order as the CPU oracle.
 #include <algorithm>
@@ -249,43 +249,57 @@ __global__ void __launch_bounds__(kThreads)
     lod_claim_one(left, p, (uint32_t)i, next, grid_next);
 }
 
-// Stage 6: per batch AABB + stable level bucketing + RasterBatch
-// (packBatchAABB + packBucketLOD, GPUPacker/Shaders.metal:243-284, 383-414).
+// Stages 6 and 7: per batch AABB, RasterBatch and stable level bucketing
+// (packBatchAABB + packBucketLOD, GPUPacker/Shaders.metal:243-284, 383-414),
+// then final order and quantisation (packQuantize, Shaders.metal:288-309).
 // One CTA per batch; each warp owns a contiguous segment of the batch's
 // points.  Pass 1: the AABB and the warp's per-level counts (ballots).  The
 // counts give every warp its first slot per level (the batch's exclusive
 // level prefix plus the counts of the warps before it), so pass 2 needs no
 // block barrier: each warp walks its segment in order, 32 points a round,
-// placing each point after the earlier points of its level (ballot rank).
-// Both passes load four rounds ahead.
+// places each point after the earlier points of its level (ballot rank) and
+// writes it there quantised.  Both passes load kBatchRounds rounds ahead.
+// Bound by memory: pass 1 reads the batch from DRAM (17 bytes a point), pass
+// 2 reads it again from L2 (two or three 10,240-point batches of 164 KB an
+// SM are in flight), and the points of a level land next to each other, so
+// the stores of a round fill one run per level.
+// NL: the levels there can be (4, the default, or 8): a ballot each in both
+// passes.
 constexpr int kBatchRounds = 4;
-__global__ void __launch_bounds__(kThreads)
+constexpr int kBatchThreads = 512;
+template <int NL>
+__global__ void __launch_bounds__(kBatchThreads)
     pack_batches(const float4 *__restrict__ sorted, const uint8_t *__restrict__ lv, uint64_t n,
                  uint32_t ppb, uint32_t first_slot, cr_raster_batch *__restrict__ batches,
-                 uint32_t *__restrict__ perm, uint8_t *__restrict__ lv_out) {
-    constexpr int kWarps = kThreads / 32;
+                 const uint32_t *__restrict__ idx_sorted, uint32_t *__restrict__ low,
+                 uint32_t *__restrict__ med, uint32_t *__restrict__ high,
+                 uint32_t *__restrict__ colors, uint8_t *__restrict__ levels,
+                 uint32_t *__restrict__ src_out) {
+    constexpr int kWarps = kBatchThreads / 32;
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ uint32_t red[6][kWarps];
-    __shared__ uint32_t wcnt[kWarps][8];
+    __shared__ uint32_t wcnt[kWarps][NL];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint64_t start = (uint64_t)blockIdx.x * ppb;
     const uint64_t end = (start + ppb < n) ? start + ppb : n;
     const uint32_t total = (uint32_t)(end - start);
     const uint32_t seg = (total + kWarps - 1u) / kWarps;
-    const uint64_t s0 = start + min((uint64_t)total, (uint64_t)warp * seg);
-    const uint64_t s1 = start + min((uint64_t)total, (uint64_t)(warp + 1) * seg);
+    const uint32_t s0 = min(total, (uint32_t)warp * seg);
+    const uint32_t s1 = min(total, (uint32_t)(warp + 1) * seg);
+    const float4 *bsorted = sorted + start;
+    const uint8_t *blv = lv + start;
     // 1. AABB and level counts of the warp's segment.
     uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
-    uint32_t c[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-    for (uint64_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
+    uint32_t c[NL] = {};
+    for (uint32_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
         float4 p[kBatchRounds];
         uint32_t l[kBatchRounds];
 #pragma unroll
         for (int k = 0; k < kBatchRounds; ++k) {
-            const uint64_t i = r0 + 32u * k + lane;
-            l[k] = i < s1 ? (lv[i] & 7u) : 8u;
-            p[k] = i < s1 ? sorted[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const uint32_t i = r0 + 32u * k + lane;
+            l[k] = i < s1 ? (blv[i] & 7u) : 8u;
+            p[k] = i < s1 ? bsorted[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int k = 0; k < kBatchRounds; ++k) {
@@ -298,7 +312,7 @@ __global__ void __launch_bounds__(kThreads)
                 }
             }
 #pragma unroll
-            for (int L = 0; L < 8; ++L) c[L] += __popc(__ballot_sync(kFull, l[k] == (uint32_t)L));
+            for (int L = 0; L < NL; ++L) c[L] += __popc(__ballot_sync(kFull, l[k] == (uint32_t)L));
         }
     }
 #pragma unroll
@@ -310,47 +324,46 @@ __global__ void __launch_bounds__(kThreads)
             red[3 + a][warp] = y;
         }
     }
-    if (lane < 8) {
+    if (lane < NL) {
         uint32_t mine = 0;
 #pragma unroll
-        for (int L = 0; L < 8; ++L)
+        for (int L = 0; L < NL; ++L)
             if (lane == L) mine = c[L];
         wcnt[warp][lane] = mine;
     }
     __syncthreads();
-    // 2. This warp's first slot (from the batch start) per level.
-    uint32_t run[8], cum[8];
+    // 2. This warp's first slot (from the batch start) per level; the box.
+    uint32_t run[NL], cum[8];
     {
         uint32_t acc = 0;
 #pragma unroll
-        for (int L = 0; L < 8; ++L) {
-            uint32_t tot = 0, before = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t x = wcnt[w][L];
-                tot += x;
-                if (w < warp) before += x;
-            }
+        for (int L = 0; L < NL; ++L) {
+            const uint32_t x = lane < kWarps ? wcnt[lane][L] : 0u;
+            const uint32_t tot = __reduce_add_sync(kFull, x);
+            const uint32_t before = __reduce_add_sync(kFull, lane < warp ? x : 0u);
             run[L] = acc + before;
             acc += tot;
             cum[L] = acc;
         }
+#pragma unroll
+        for (int L = NL; L < 8; ++L) cum[L] = acc;
+    }
+    float bmin[3], size[3], bmax[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        bmin[a] = unflip(__reduce_min_sync(kFull, lane < kWarps ? red[a][lane] : 0xffffffffu));
+        bmax[a] = unflip(__reduce_max_sync(kFull, lane < kWarps ? red[3 + a][lane] : 0u));
+        size[a] = fmaxf(bmax[a] - bmin[a], 0.000001f);
     }
     if (threadIdx.x == 0) {
-        uint32_t m[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-        for (int w = 0; w < kWarps; ++w)
-            for (int a = 0; a < 3; ++a) {
-                m[a] = min(m[a], red[a][w]);
-                m[3 + a] = max(m[3 + a], red[3 + a][w]);
-            }
         cr_raster_batch rb;
         rb.state = 1;
-        rb.minX = unflip(m[0]);
-        rb.minY = unflip(m[1]);
-        rb.minZ = unflip(m[2]);
-        rb.maxX = unflip(m[3]);
-        rb.maxY = unflip(m[4]);
-        rb.maxZ = unflip(m[5]);
+        rb.minX = bmin[0];
+        rb.minY = bmin[1];
+        rb.minZ = bmin[2];
+        rb.maxX = bmax[0];
+        rb.maxY = bmax[1];
+        rb.maxZ = bmax[2];
         rb.numPoints = total;
         rb.firstPoint = (first_slot + blockIdx.x) * ppb;
         rb.fileIndex = 0;
@@ -362,67 +375,49 @@ __global__ void __launch_bounds__(kThreads)
         rb.padding8 = 0;
         batches[blockIdx.x] = rb;
     }
-    // 3. Stable bucketing of the warp's segment.
-    for (uint64_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
+    // 3. Stable bucketing of the warp's segment, each point quantised into
+    // its final place.
+    for (uint32_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
+        float4 p[kBatchRounds];
         uint32_t raw[kBatchRounds];
 #pragma unroll
         for (int k = 0; k < kBatchRounds; ++k) {
-            const uint64_t i = r0 + 32u * k + lane;
-            raw[k] = i < s1 ? (uint32_t)lv[i] : 0xffu;
+            const uint32_t i = r0 + 32u * k + lane;
+            raw[k] = i < s1 ? (uint32_t)blv[i] : 0xffu;
+            p[k] = i < s1 ? bsorted[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int k = 0; k < kBatchRounds; ++k) {
-            const uint64_t i = r0 + 32u * k + lane;
+            const uint32_t i = r0 + 32u * k + lane;
             const bool v = i < s1;
             const uint32_t l = v ? (raw[k] & 7u) : 8u;
             uint32_t dst = 0;
 #pragma unroll
-            for (int L = 0; L < 8; ++L) {
+            for (int L = 0; L < NL; ++L) {
                 const uint32_t b = __ballot_sync(kFull, l == (uint32_t)L);
                 if (l == (uint32_t)L) dst = run[L] + __popc(b & lt);
                 run[L] += __popc(b);
             }
             if (v && dst < total) {  // always true: the ranks come from the same levels
-                perm[start + dst] = (uint32_t)i;
-                lv_out[start + dst] = (uint8_t)raw[k];
+                const float nx = fminf(fmaxf((p[k].x - bmin[0]) / size[0], 0.0f), 0.99999994f);
+                const float ny = fminf(fmaxf((p[k].y - bmin[1]) / size[1], 0.0f), 0.99999994f);
+                const float nz = fminf(fmaxf((p[k].z - bmin[2]) / size[2], 0.0f), 0.99999994f);
+                // Float(2^30 - 1) rounds to 2^30 in f32.
+                const uint32_t qx = (uint32_t)(nx * 1073741824.0f);
+                const uint32_t qy = (uint32_t)(ny * 1073741824.0f);
+                const uint32_t qz = (uint32_t)(nz * 1073741824.0f);
+                const uint64_t j = start + dst;
+                low[j] = ((qx >> 20) & 1023u) | (((qy >> 20) & 1023u) << 10) |
+                         (((qz >> 20) & 1023u) << 20);
+                med[j] = ((qx >> 10) & 1023u) | (((qy >> 10) & 1023u) << 10) |
+                         (((qz >> 10) & 1023u) << 20);
+                high[j] = (qx & 1023u) | ((qy & 1023u) << 10) | ((qz & 1023u) << 20);
+                colors[j] = __float_as_uint(p[k].w);
+                levels[j] = (uint8_t)raw[k];
+                if (src_out) src_out[j] = idx_sorted[start + i];
             }
         }
     }
-}
-
-// Stage 7: final order, quantisation (packQuantize, GPUPacker/Shaders.metal:288-309).
-__global__ void __launch_bounds__(kThreads)
-    pack_emit(uint64_t n, uint32_t ppb, const uint32_t *__restrict__ perm,
-              const uint32_t *__restrict__ idx_sorted, const float4 *__restrict__ sorted,
-              const uint8_t *__restrict__ lv_out,
-              const cr_raster_batch *__restrict__ batches, uint32_t *__restrict__ low,
-              uint32_t *__restrict__ med, uint32_t *__restrict__ high,
-              uint32_t *__restrict__ colors, uint8_t *__restrict__ levels,
-              uint32_t *__restrict__ src_out) {
-    const uint64_t j = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (j >= n) return;
-    // perm only reorders points within their batch (level bucketing), so
-    // the Morton-ordered arrays are read nearly in order.
-    const uint32_t pj = perm[j];
-    if (pj >= n) return;  // unreachable for a complete permutation
-    const float4 p = sorted[pj];
-    const cr_raster_batch &b = batches[j / ppb];
-    const float sx = fmaxf(b.maxX - b.minX, 0.000001f);
-    const float sy = fmaxf(b.maxY - b.minY, 0.000001f);
-    const float sz = fmaxf(b.maxZ - b.minZ, 0.000001f);
-    const float nx = fminf(fmaxf((p.x - b.minX) / sx, 0.0f), 0.99999994f);
-    const float ny = fminf(fmaxf((p.y - b.minY) / sy, 0.0f), 0.99999994f);
-    const float nz = fminf(fmaxf((p.z - b.minZ) / sz, 0.0f), 0.99999994f);
-    // Float(2^30 - 1) rounds to 2^30 in f32.
-    const uint32_t qx = (uint32_t)(nx * 1073741824.0f);
-    const uint32_t qy = (uint32_t)(ny * 1073741824.0f);
-    const uint32_t qz = (uint32_t)(nz * 1073741824.0f);
-    low[j] = ((qx >> 20) & 1023u) | (((qy >> 20) & 1023u) << 10) | (((qz >> 20) & 1023u) << 20);
-    med[j] = ((qx >> 10) & 1023u) | (((qy >> 10) & 1023u) << 10) | (((qz >> 10) & 1023u) << 20);
-    high[j] = (qx & 1023u) | ((qy & 1023u) << 10) | ((qz & 1023u) << 20);
-    colors[j] = __float_as_uint(p.w);
-    levels[j] = lv_out[j];
-    if (src_out) src_out[j] = idx_sorted[pj];
 }
 
 unsigned grid_for(uint64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
@@ -463,8 +458,6 @@ cr_status ensure_points(PackScratch &s, uint64_t n) {
     ALLOC(s.idx[1], m * 4);
     ALLOC(s.sorted, m * sizeof(float4));
     ALLOC(s.lv_morton, (m + 15) & ~15ull);
-    ALLOC(s.lv_out, (m + 15) & ~15ull);
-    ALLOC(s.perm, m * 4);
     ALLOC(s.src_idx, m * 4);
     ALLOC(s.bounds, 8 * 4);
 #undef ALLOC
@@ -476,7 +469,7 @@ cr_status ensure_points(PackScratch &s, uint64_t n) {
 
 void pack_scratch_free(PackScratch &s) {
     void *ptrs[] = {s.raw, s.pos, s.keys[0], s.keys[1], s.idx[0], s.idx[1], s.sorted,
-                    s.lv_morton, s.lv_out, s.perm, s.grid, s.bounds, s.src_idx};
+                    s.lv_morton, s.grid, s.bounds, s.src_idx};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     radix_scratch_free(s.radix);
@@ -635,16 +628,14 @@ cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const cr_pack_input *in, ui
         CR_CUDA(cudaGetLastError());
     }
 
-    // Stage 6-7: batches, final order, quantisation into the pool.
+    // Stages 6-7: batches, final order, quantisation into the pool.
     cr_raster_batch *dst_batches = cloud->d_batches + first_slot;
-    pack_batches<<<nb, kThreads, 0, s>>>(sc.sorted, sc.lv_morton, count, ppb, first_slot,
-                                         dst_batches, sc.perm, sc.lv_out);
-    CR_CUDA(cudaGetLastError());
     const uint64_t p0 = (uint64_t)first_slot * ppb;
-    pack_emit<<<grid_for(count), kThreads, 0, s>>>(
-        count, ppb, sc.perm, idx_sorted, sc.sorted, sc.lv_out, dst_batches,
-        cloud->d_low + p0,
-        cloud->d_med + p0, cloud->d_high + p0, cloud->d_colors + p0, cloud->d_levels + p0,
+    auto *batch_kernel = L <= 4 ? pack_batches<4> : pack_batches<8>;
+    batch_kernel<<<nb, kBatchThreads, 0, s>>>(
+        sc.sorted, sc.lv_morton, count, ppb, first_slot, dst_batches, idx_sorted,
+        cloud->d_low + p0, cloud->d_med + p0, cloud->d_high + p0, cloud->d_colors + p0,
+        cloud->d_levels + p0,
         src_idx_host ? sc.src_idx : nullptr);  // source indices only when asked for
     CR_CUDA(cudaGetLastError());
     if (src_idx_host)
