@@ -110,109 +110,191 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
 template <typename K>
 size_t onesweep_smem_bytes() {
     return (size_t)kTileKeys * (sizeof(K) + sizeof(uint32_t)) +
-           (size_t)kWarps * 256 * sizeof(WarpCount) + (256 + 256 + 32) * sizeof(uint32_t);
+           (size_t)kWarps * 256 * sizeof(WarpCount) + (256 + 32) * sizeof(uint32_t);
+}
+
+// Digit of a key: a byte of the 32-bit word that holds it (a digit never
+// straddles the words: the shifts are multiples of 8).
+struct DigitOf {
+    uint32_t word;  // word of the key (0 low, 1 high)
+    uint32_t sel;   // byte selector: that byte, then three zero bytes
+    __device__ __forceinline__ explicit DigitOf(int shift)
+        : word((uint32_t)shift >> 5), sel(0x4440u | (((uint32_t)shift >> 3) & 3u)) {}
+    __device__ __forceinline__ uint32_t of_word(uint32_t w) const {
+        return __byte_perm(w, 0u, sel);
+    }
+    // Digit of key i of an array in global or shared memory.
+    __device__ __forceinline__ uint32_t at(const uint32_t *keys, uint32_t i) const {
+        return of_word(keys[i]);
+    }
+    __device__ __forceinline__ uint32_t at(const unsigned long long *keys, uint32_t i) const {
+        return of_word(reinterpret_cast<const uint32_t *>(keys)[2u * i + word]);
+    }
+    __device__ __forceinline__ uint32_t of(uint32_t k) const { return of_word(k); }
+    __device__ __forceinline__ uint32_t of(unsigned long long k) const {
+        return of_word(word ? (uint32_t)(k >> 32) : (uint32_t)k);
+    }
+};
+
+// Ranks a warp's keys (512, in warp-striped order: key 32 j + lane) among
+// equal digits, in input order, against the warp's running digit counts wc.
+// rd[j] = rank | digit << 16.  FULL: the tile has all of its keys.
+template <typename K, bool FULL>
+__device__ __forceinline__ void rank_keys(const K *keys, uint32_t w0, uint32_t tile_n,
+                                          const DigitOf &dig, WarpCount *wc, uint32_t lt,
+                                          uint32_t (&rd)[kKeysPerLane]) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < kKeysPerLane; ++j) {
+        const uint32_t li = w0 + (uint32_t)j * 32u + lane;
+        const bool v = FULL || li < tile_n;
+        const uint32_t d = v ? dig.at(keys, li) : 0u;
+        // Lanes with the same digit: the lanes that agree with this lane's
+        // bit, for every bit (eight ballots cost less than
+        // __match_any_sync when a warp holds many distinct digits).  A lane
+        // differs from this one where its bit of some ballot does.
+        uint32_t differ = FULL ? 0u : ~__ballot_sync(0xffffffffu, v);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const bool bit = (d >> b) & 1u;
+            const uint32_t m = __ballot_sync(0xffffffffu, bit);
+            differ |= m ^ (bit ? 0xffffffffu : 0u);
+        }
+        const uint32_t lower = ~differ & lt;
+        const uint32_t before = wc[d];
+        rd[j] = (before + __popc(lower)) | (d << 16);
+        __syncwarp();
+        if (v && lower == 0u) wc[d] = (WarpCount)(before + __popc(~differ));
+        __syncwarp();
+    }
+}
+
+// Moves a warp's keys and values to their places in the tile sorted by digit.
+template <typename K, bool kIota, bool FULL>
+__device__ __forceinline__ void move_keys(const K *keys, const uint32_t *vals, uint32_t tile0,
+                                          uint32_t w0, uint32_t tile_n, const WarpCount *wc,
+                                          const uint32_t (&rd)[kKeysPerLane], K *skey,
+                                          uint32_t *sval) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < kKeysPerLane; ++j) {
+        const uint32_t li = w0 + (uint32_t)j * 32u + lane;
+        if (FULL || li < tile_n) {
+            const uint32_t slot = wc[rd[j] >> 16] + (rd[j] & 0xffffu);
+            skey[slot] = keys[li];
+            sval[slot] = kIota ? tile0 + li : vals[li];
+        }
+    }
+}
+
+// Writes the sorted tile to global memory: gbase[d] + (slot in the tile).
+template <typename K, bool FULL>
+__device__ __forceinline__ void write_keys(const K *skey, const uint32_t *sval,
+                                           const uint32_t *gbase, const DigitOf &dig,
+                                           uint32_t tile_n, uint32_t n, K *keys_out,
+                                           uint32_t *vals_out) {
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < (FULL ? (uint32_t)kTileKeys : tile_n); i += kThreads) {
+        const K k = skey[i];
+        const uint32_t dst = gbase[dig.of(k)] + i;
+        if (dst < n) {  // always true when the counts are consistent
+            keys_out[dst] = k;
+            vals_out[dst] = sval[i];
+        }
+    }
 }
 
 // One pass: a tile of kTileKeys keys per CTA, in ticket order.
 //   1. each warp takes 512 consecutive keys, 16 per lane in warp-striped order
 //      (key j*32 + lane), and ranks them among equal digits (peer lanes found
 //      by ballots) against running per-warp digit counts, in input order;
-//   2. thread d: the tile's count of digit d (published at once) and the
-//      exclusive bases of the warps;
-//   3. exclusive scan over the digits gives each key its slot in a tile
-//      sorted by digit; keys and values move there in shared memory; then
-//      thread d sums the counts of the tiles before it (look-back) and
-//      publishes the inclusive prefix;
+//   2. thread d: the tile's count of digit d (published at once); an
+//      exclusive scan over the digits, and with it the first slot of every
+//      (warp, digit) in a tile sorted by digit;
+//   3. keys and values move there in shared memory; then thread d sums the
+//      counts of the tiles before it (look-back) and publishes the inclusive
+//      prefix;
 //   4. threads read the sorted tile in order and write each key to its
 //      digit's global offset: keys of one digit are consecutive in shared
 //      memory and land at consecutive addresses (coalesced runs).
+// Bound by the integer pipe (ballots, selects and address arithmetic; it was
+// 83 % busy), so the full tiles have code without bounds (every tile but the
+// last), a digit is one byte permute of the word that holds it, offsets are
+// 32 bits and one shared word gives a key's place.
 template <typename K, bool kIota>
 __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
     radix_onesweep(const K *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
-                   K *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint64_t n,
+                   K *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n,
                    int shift, const uint32_t *__restrict__ digit_base,
                    unsigned long long *__restrict__ lookback, uint32_t epoch,
                    uint32_t *__restrict__ tile_counter, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char smem[];
     K *skey = reinterpret_cast<K *>(smem);
     uint32_t *sval = reinterpret_cast<uint32_t *>(skey + kTileKeys);
-    // [kWarps][256]: per-warp digit counts, then the warps' digit bases.
+    // [kWarps][256]: per-warp digit counts, then the warps' first slots.
     WarpCount *wcnt = reinterpret_cast<WarpCount *>(sval + kTileKeys);
-    // Global offset of the tile's run of each digit.
-    uint32_t *offset = reinterpret_cast<uint32_t *>(wcnt + kWarps * 256);
-    uint32_t *tbase = offset + 256;          // tile-local digit base
-    uint32_t *misc = tbase + 256;            // [0] ticket, [1..8] warp sums of the digit scan
+    // Per digit: global place of the tile's run less its first slot in the tile.
+    uint32_t *gbase = reinterpret_cast<uint32_t *>(wcnt + kWarps * 256);
+    uint32_t *misc = gbase + 256;            // [0] ticket, [1..8] warp sums of the digit scan
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
+    const DigitOf dig(shift);
     if (threadIdx.x == 0) misc[0] = atomicAdd(tile_counter, 1u);
-    for (int i = threadIdx.x; i < kWarps * 256; i += kThreads) wcnt[i] = 0u;
+    static_assert(kWarps * 256 * sizeof(WarpCount) == kThreads * sizeof(uint4), "one store each");
+    reinterpret_cast<uint4 *>(wcnt)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const uint32_t tile = misc[0];
-    const uint64_t tile0 = (uint64_t)tile * kTileKeys;
-    const uint32_t tile_n =
-        (n - tile0 < (uint64_t)kTileKeys) ? (uint32_t)(n - tile0) : (uint32_t)kTileKeys;
+    const uint32_t tile0 = tile * (uint32_t)kTileKeys;  // below n
+    const uint32_t tile_n = min(n - tile0, (uint32_t)kTileKeys);
+    const bool full = tile_n == (uint32_t)kTileKeys;
+    keys_in += tile0;
+    if (!kIota) vals_in += tile0;
+    const uint32_t w0 = (uint32_t)warp * (32 * kKeysPerLane);
     // 1. Warp-level ranking in input order; a key's rank within its warp
     //    (< 512) and digit are kept packed, the key and value are read again
-    //    (from L1 / L2) when they move.
+    //    (from L2) when they move.
     uint32_t rd[kKeysPerLane];
     WarpCount *wc = wcnt + warp * 256;
-#pragma unroll
-    for (int j = 0; j < kKeysPerLane; ++j) {
-        const uint32_t li = (uint32_t)warp * (32 * kKeysPerLane) + (uint32_t)j * 32 + lane;
-        const bool v = li < tile_n;
-        const K key = v ? keys_in[tile0 + li] : K(0);
-        const uint32_t d = v ? ((uint32_t)(key >> shift) & 0xffu) : 256u;
-        // Lanes with the same digit (9 bits: the digit and the no-key flag):
-        // the intersection, over the bits, of the lanes that agree with this
-        // lane's bit.  (Nine ballots cost less than __match_any_sync when a
-        // warp holds many distinct digits.)
-        uint32_t peers = 0xffffffffu;
-#pragma unroll
-        for (int b = 0; b < 9; ++b) {
-            const uint32_t m = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-            peers &= ((d >> b) & 1u) ? m : ~m;
-        }
-        const uint32_t before = v ? wc[d] : 0u;
-        rd[j] = (before + __popc(peers & lt)) | (d << 16);
-        __syncwarp();
-        if (v && (peers & lt) == 0u) wc[d] = (WarpCount)(before + __popc(peers));
-        __syncwarp();
-    }
+    if (full)
+        rank_keys<K, true>(keys_in, w0, tile_n, dig, wc, lt, rd);
+    else
+        rank_keys<K, false>(keys_in, w0, tile_n, dig, wc, lt, rd);
     __syncthreads();
-    // 2. Digit d = thread: the tile's count and the warps' exclusive bases.
+    // 2. Digit d = thread: the tile's count and the warps' first slots.
     const uint32_t dd = threadIdx.x;
-    uint32_t total = 0;
+    uint32_t cw[kWarps], total = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-        const uint32_t c = wcnt[w * 256 + dd];
-        wcnt[w * 256 + dd] = (WarpCount)total;
-        total += c;
+        cw[w] = wcnt[w * 256 + dd];
+        total += cw[w];
     }
     unsigned long long *my = lookback + (size_t)tile * 256 + dd;
     // Publish the tile's count first (tile 0: its prefix), so that the tiles
     // after it can go on while this one sorts its keys.
     st_relaxed64(my, lookback_word(epoch, tile == 0 ? kFlagPrefix : kFlagAgg, total));
-    // 3. Exclusive scan of the tile's digit counts (a warp scan per 32
-    //    digits, then over the warps).
+    // Exclusive scan of the tile's digit counts (a warp scan per 32 digits,
+    // then over the warps).
     const uint32_t incl = warp_inclusive(total, lane);
     if (lane == 31) misc[1 + warp] = incl;
     __syncthreads();
-    uint32_t wbase = 0;
+    uint32_t tbase = incl - total;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w)
-        if (w < warp) wbase += misc[1 + w];
-    tbase[dd] = wbase + incl - total;
-    __syncthreads();
+        if (w < warp) tbase += misc[1 + w];
+    {
+        uint32_t slot = tbase;
 #pragma unroll
-    for (int j = 0; j < kKeysPerLane; ++j) {
-        const uint32_t li = (uint32_t)warp * (32 * kKeysPerLane) + (uint32_t)j * 32 + lane;
-        if (li < tile_n) {
-            const uint32_t d = rd[j] >> 16;
-            const uint32_t slot = tbase[d] + wcnt[warp * 256 + d] + (rd[j] & 0xffffu);
-            skey[slot] = keys_in[tile0 + li];
-            sval[slot] = kIota ? (uint32_t)(tile0 + li) : vals_in[tile0 + li];
+        for (int w = 0; w < kWarps; ++w) {
+            wcnt[w * 256 + dd] = (WarpCount)slot;
+            slot += cw[w];
         }
     }
+    __syncthreads();
+    // 3. The tile sorted by digit.
+    if (full)
+        move_keys<K, kIota, true>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
+    else
+        move_keys<K, kIota, false>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
     // The look-back (thread d, digit d) over the tiles before this one, after
     // the tile-local work so that its waits overlap it.
     unsigned long long excl = 0;
@@ -269,18 +351,13 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
         if (gave_up && status) *(volatile uint32_t *)status = kErrSortWait;
         st_relaxed64(my, lookback_word(epoch, kFlagPrefix, excl + total));
     }
-    offset[dd] = digit_base[dd] + (uint32_t)excl;
-    __syncthreads();  // every digit's offset; the sorted tile complete
+    gbase[dd] = digit_base[dd] + (uint32_t)excl - tbase;
+    __syncthreads();  // every digit's place; the sorted tile complete
     // 4. Coalesced runs per digit to the global output.
-    for (uint32_t i = threadIdx.x; i < tile_n; i += kThreads) {
-        const K k = skey[i];
-        const uint32_t d = (uint32_t)(k >> shift) & 0xffu;
-        const uint64_t dst = (uint64_t)offset[d] + (i - tbase[d]);
-        if (dst < n) {  // always true when the counts are consistent
-            keys_out[dst] = k;
-            vals_out[dst] = sval[i];
-        }
-    }
+    if (full)
+        write_keys<K, true>(skey, sval, gbase, dig, tile_n, n, keys_out, vals_out);
+    else
+        write_keys<K, false>(skey, sval, gbase, dig, tile_n, n, keys_out, vals_out);
 }
 
 }  // namespace
@@ -361,7 +438,7 @@ cr_status radix_sort_pairs(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_
         // The first pass of an index sort makes the indices (kIota).
         auto *kern = vals_iota && p == run.front() ? radix_onesweep<K, true>
                                                    : radix_onesweep<K, false>;
-        kern<<<(unsigned)ntiles, kThreads, smem, s>>>(kin, vin, kout, vout, n, 8 * p,
+        kern<<<(unsigned)ntiles, kThreads, smem, s>>>(kin, vin, kout, vout, (uint32_t)n, 8 * p,
                                                      rs.bases + p * 256, rs.lookback, rs.epoch,
                                                      rs.tiles + p, status);
         CR_CUDA(cudaGetLastError());
