@@ -1534,7 +1534,7 @@ CR_API cr_status cr_pack(cr_context *ctx, cr_cloud *c, const cr_pack_input *in, 
     c->points = count;
     mark_dirty(c, 0, (int64_t)c->mirror.size() - 1);
     if ((st = flush_mirror(c))) return st;
-    if ((st = pack_run(ctx, c, in, count, prm, on_device, 0, src_idx))) return st;
+    if ((st = pack_run(ctx, c, {PackJob{in, count, 0u}}, prm, on_device, src_idx))) return st;
     return adopt_batches(c, 0, nb);
 }
 
@@ -1589,13 +1589,20 @@ CR_API cr_status cr_pack_chunks(cr_context *ctx, cr_cloud *c, const cr_pack_inpu
         if (first < 0) continue;
         placed.push_back(Placed{(uint32_t)first, (uint32_t)nb, i});
     }
+    std::vector<PackJob> jobs;
     for (const Placed &p : placed)
-        if ((st = pack_run(ctx, c, &chunks[p.index], counts[p.index], prm, on_device, p.first,
-                           nullptr)))
-            return st;
+        jobs.push_back(PackJob{&chunks[p.index], counts[p.index], p.first});
+    if ((st = pack_run(ctx, c, jobs, prm, on_device, nullptr))) return st;
+    // The batches come back with one copy per run of neighbouring slots.
+    for (size_t k = 0; k < placed.size();) {
+        uint32_t n = placed[k].nb;
+        size_t e = k + 1;
+        while (e < placed.size() && placed[e].first == placed[k].first + n) n += placed[e++].nb;
+        if ((st = adopt_batches(c, placed[k].first, n))) return st;
+        k = e;
+    }
     for (size_t k = 0; k < placed.size(); ++k) {
         const Placed &p = placed[k];
-        if ((st = adopt_batches(c, p.first, p.nb))) return st;
         c->resident += p.nb;
         c->points += counts[p.index];
         if (first_slots) first_slots[k] = (int32_t)p.first;

@@ -519,6 +519,11 @@ cr_status launch_split_nearest(const unsigned long long *keys, uint32_t *depth_o
                                uint32_t *index_out, size_t n, cudaStream_t s);
 
 
-cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const cr_pack_input *in, uint64_t count,
-                   const cr_pack_params *prm, int on_device, uint32_t first_slot,
-                   uint32_t *src_idx_host);
+// One cloud or chunk to pack: count points into the slots from first_slot.
+struct PackJob {
+    const cr_pack_input *in;
+    uint64_t count;
+    uint32_t first_slot;
+};
+cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const std::vector<PackJob> &jobs,
+                   const cr_pack_params *prm, int on_device, uint32_t *src_idx_host);

@@ -6,29 +6,53 @@
 
 #include "cr/cr.h"
 
+// One segment of a sort: keys [begin, begin + n) of the arrays, sorted by
+// itself; tile0 is its first tile in the numbering of all segments' tiles.
+struct RadixSeg {
+    uint64_t begin;
+    uint32_t n, tile0;
+};
+constexpr int kRadixMaxPasses = 8;  // 8-bit digits of a 64-bit key
+
+// The sort's ping-pong buffers: the keys start in keys[0].  A segment whose
+// set of passes (RadixScratch::runs) has k members ends in buffer k & 1; with
+// k = 0 no values were written, and key i's value is i.
+template <typename K>
+struct RadixBuffers {
+    K *keys[2];
+    uint32_t *vals[2];
+};
+
 // Grow-only scratch of the radix sort: look-back words (256 per 4096-key
-// tile), the histograms and digit bases of up to 8 passes, one tile ticket
-// counter per pass, and the epoch of the last pass (look-back words carry it).
+// tile), per segment the histograms and digit bases of up to 8 passes and
+// the set of passes to run, one tile ticket counter per pass, and the epoch
+// of the last pass (look-back words carry it).
 struct RadixScratch {
     unsigned long long *lookback = nullptr;
     uint64_t cap_tiles = 0;
-    uint32_t *hist = nullptr;
-    uint32_t *bases = nullptr;
+    uint32_t cap_segs = 0;
+    uint32_t *hist = nullptr;   // [segment][kRadixMaxPasses][256], filled by the caller
+    uint32_t *bases = nullptr;  // the same shape
+    uint32_t *runs = nullptr;   // per segment: bit p set = pass p runs
     uint32_t *tiles = nullptr;
     uint32_t epoch = 0;
 };
 void radix_scratch_free(RadixScratch &r);
-
-// Stable sort of n (key, value) pairs by the low key_bits bits of the keys;
-// the result is in (keys_alt, vals_alt) when *result_in_alt.  With
-// vals_iota the values are the keys' input positions and `vals` is not read
-// (the first pass makes them).  Synchronises once (the histograms are read
-// back to skip constant digits).  A bounded wait that gives up stores
-// kErrSortWait into *status.
+// Tiles of n keys.
+uint32_t radix_tiles(uint32_t n);
+// Makes room for nseg segments of ntiles tiles in all and zeroes the
+// histograms; the caller then fills them and calls radix_sort.
+cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStream_t s);
+// Stable sort of every segment's keys by their low key_bits bits (the bits
+// above them are zero), with the keys' places in the segment as values.
+// segs is device memory.  A bounded wait that gives up stores kErrSortWait
+// into *status.
 template <typename K>
-cr_status radix_sort_pairs(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_alt, uint64_t n,
-                           int key_bits, bool vals_iota, RadixScratch &rs, uint32_t *status,
-                           int sm_count, cudaStream_t s, bool *result_in_alt);
+cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
+                     uint64_t ntiles, int key_bits, RadixScratch &rs, uint32_t *status,
+                     cudaStream_t s);
+
+struct PackSeg;
 
 // Grow-only device scratch of the packer, owned by the context (the
 // reference's PackScratch, GPUPacker.swift:453-484).
@@ -36,15 +60,19 @@ struct PackScratch {
     uint64_t cap_points = 0;
     uint64_t cap_raw_bytes = 0;
     uint64_t cap_grid = 0;
+    uint64_t cap_segs = 0;
     void *raw = nullptr;                    // staged host input
     float4 *pos = nullptr;                  // input x, y, z and RGBA8 bits in w
     void *keys[2] = {nullptr, nullptr};     // Morton keys (u32 or u64), ping-pong
     uint32_t *idx[2] = {nullptr, nullptr};  // sort payload, ping-pong
     float4 *sorted = nullptr;               // positions in Morton order
     uint8_t *lv_morton = nullptr;           // levels in Morton order
-    uint32_t *grid = nullptr;               // dense LOD occupancy grid
+    uint32_t *grid = nullptr;               // dense LOD occupancy grids
+    PackSeg *segs = nullptr;                // the segments of a run
+    RadixSeg *rsegs = nullptr;              //   and what the sort needs of them
     RadixScratch radix;                     // the sort's look-back words and histograms
-    uint32_t *bounds = nullptr;             // 6 flipped words: min xyz, max xyz
+    uint32_t *bounds = nullptr;             // per segment: 3 flipped minima, 3 complements of
+                                            // flipped maxima
     uint32_t *src_idx = nullptr;            // final order -> input index
 };
 

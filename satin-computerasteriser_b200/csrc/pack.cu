@@ -4,10 +4,13 @@
 // Restates GPUPacker.encodePack (GPUPacker.swift:204-392) and its kernels
 // (Pipelines/GPUPacker/Shaders.metal:41-414), which in turn mirror the CPU
 // PackedPointCloudFixtures.pack (PackedPointCloudFixtures.swift:30-344):
-//   1 bounds        global AABB (order-preserving flipped-bit min/max)
-//   2 morton        10 bits/axis (30-bit key) or 21 bits/axis (63-bit key)
-//   3 sort          stable LSD radix of (key, input index), one read of the
-//                   keys for every digit's histogram, then one single-sweep
+//   1 load, bounds  raw input to 16-byte records {x, y, z, rgba8} (records on
+//                   the device are read in place), and the AABB of every
+//                   segment (order-preserving flipped-bit min/max), read back
+//                   once for the Morton scales and the LOD grids
+//   2 morton        10 bits/axis (30-bit key) or 21 bits/axis (63-bit key),
+//                   with the histograms of every 8-bit digit
+//   3 sort          stable LSD radix of (key, input index), one single-sweep
 //                   pass per digit (decoupled look-back; the first pass
 //                   makes the input indices)                     [radix.cu]
 //   4 gather        positions in Morton order, levels = maxLevel
@@ -23,6 +26,11 @@
 //                   block barrier) of the points, quantised to 30 bits an
 //                   axis in three 10-bit/axis words, with colours, levels
 //                   and source indices.
+// Every stage is one launch over all segments of a run (the chunks of one
+// cr_pack_chunks call, or the one cloud of cr_pack): a streamed node of 140
+// thousand points fills a quarter of the GPU, and launches and read-backs
+// took longer than its kernels (ten nodes: 2.04 ms one after the other, 0.45
+// ms together).
 // Host-side float math (scale, voxel sizes, grid dims) is compiled without
 // contraction and uses the same operation order as the CPU oracle.
 #include <algorithm>
@@ -60,22 +68,14 @@ __host__ __device__ __forceinline__ float unflip(uint32_t u) {
 #endif
 }
 
+// Ten bits spread to every third place.  The copies do not overlap, so a
+// shift and an or are one multiplication.
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
     uint32_t x = v & 0x3ffu;
-    x = (x | (x << 16)) & 0x030000ffu;
-    x = (x | (x << 8)) & 0x0300f00fu;
-    x = (x | (x << 4)) & 0x030c30c3u;
-    x = (x | (x << 2)) & 0x09249249u;
-    return x;
-}
-
-__device__ __forceinline__ unsigned long long spread21(unsigned long long v) {
-    unsigned long long x = v & 0x1fffffull;
-    x = (x | (x << 32)) & 0x1f00000000ffffull;
-    x = (x | (x << 16)) & 0x1f0000ff0000ffull;
-    x = (x | (x << 8)) & 0x100f00f00f00f00full;
-    x = (x | (x << 4)) & 0x10c30c30c30c30c3ull;
-    x = (x | (x << 2)) & 0x1249249249249249ull;
+    x = (x * 0x10001u) & 0x030000ffu;
+    x = (x * 0x101u) & 0x0300f00fu;
+    x = (x * 0x11u) & 0x030c30c3u;
+    x = (x * 0x5u) & 0x09249249u;
     return x;
 }
 
@@ -87,166 +87,279 @@ struct LoadArgs {
     int col_format;
 };
 
-// Stage 0: raw input -> float4 positions + packed RGBA8 (GPUPacker/Shaders.metal:219-235
-// colour rule: uint(clamp(c, 0, 1) * 255), truncating).
-// One 16-byte record per point: x, y, z and the packed RGBA8 colour's bits
-// in w (moved, never computed on), so the Morton-order gather brings both
-// with one access.
-__global__ void __launch_bounds__(kThreads)
-    pack_load(LoadArgs a, uint64_t n, float4 *__restrict__ pos) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    const float *p = reinterpret_cast<const float *>(a.pos + i * a.pos_stride);
-    uint32_t col;
-    if (a.col_format == 1) {
-        col = *reinterpret_cast<const uint32_t *>(a.col + i * a.col_stride);
-    } else {
-        const float *c = reinterpret_cast<const float *>(a.col + i * a.col_stride);
-        const uint32_t r = (uint32_t)(fminf(fmaxf(c[0], 0.0f), 1.0f) * 255.0f);
-        const uint32_t g = (uint32_t)(fminf(fmaxf(c[1], 0.0f), 1.0f) * 255.0f);
-        const uint32_t b = (uint32_t)(fminf(fmaxf(c[2], 0.0f), 1.0f) * 255.0f);
-        const uint32_t al = (uint32_t)(fminf(fmaxf(c[3], 0.0f), 1.0f) * 255.0f);
-        col = r | (g << 8) | (b << 16) | (al << 24);
-    }
-    pos[i] = make_float4(p[0], p[1], p[2], __uint_as_float(col));
-}
-
-// Stage 1: global bounds (packBounds, GPUPacker/Shaders.metal:71-105).
-__global__ void __launch_bounds__(kThreads)
-    pack_bounds(const float4 *__restrict__ pos, uint64_t n, uint32_t *__restrict__ bounds) {
-    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * kThreads) {
-        const float4 p = pos[i];
-        const uint32_t f[3] = {flip(p.x), flip(p.y), flip(p.z)};
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            mn[k] = min(mn[k], f[k]);
-            mx[k] = max(mx[k], f[k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t a = __reduce_min_sync(0xffffffffu, mn[k]);
-        const uint32_t b = __reduce_max_sync(0xffffffffu, mx[k]);
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&bounds[k], a);
-            atomicMax(&bounds[3 + k], b);
-        }
-    }
-}
-
 struct MortonArgs {
     float bmin[3];
     float scale[3];
     float top;
 };
 
-// Stage 2: Morton key (packMorton, GPUPacker/Shaders.metal:109-126); the
-// identity index the reference writes beside it is made by the sort's first
-// pass instead.
-template <typename K>
-__global__ void __launch_bounds__(kThreads)
-    pack_morton(const float4 *__restrict__ pos, uint64_t n, MortonArgs m, K *__restrict__ keys) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    const uint32_t qx = (uint32_t)fminf(fmaxf((p.x - m.bmin[0]) * m.scale[0], 0.0f), m.top);
-    const uint32_t qy = (uint32_t)fminf(fmaxf((p.y - m.bmin[1]) * m.scale[1], 0.0f), m.top);
-    const uint32_t qz = (uint32_t)fminf(fmaxf((p.z - m.bmin[2]) * m.scale[2], 0.0f), m.top);
-    if (sizeof(K) == 8)
-        keys[i] = (K)((spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz));
-    else
-        keys[i] = (K)((spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz));
-}
-
-// Stage 4: gather into Morton order, all levels at maxLevel (packLODInit).
-__global__ void __launch_bounds__(kThreads)
-    pack_gather(const float4 *__restrict__ pos, const uint32_t *__restrict__ idx, uint64_t n,
-                float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint8_t max_level) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    sorted[i] = pos[idx[i]];
-    lv[i] = max_level;
-}
-
 struct LodArgs {
     float bmin[3];
     float inv;
     uint32_t dims[3];
-    uint8_t max_level;
-    uint8_t level;
+    uint32_t level;
+    uint32_t *grid;  // this level's voxels
 };
 
-__device__ __forceinline__ uint64_t lod_cell(const float4 &p, const LodArgs &a) {
+constexpr int kMaxLevels = 8;
+
+}  // namespace
+
+// One segment of a run: points packed into slots of their own.  Its keys,
+// indices, levels and sorted points are elements [begin, begin + n) of the
+// scratch arrays.
+struct PackSeg {
+    LoadArgs la;
+    const float4 *pos;  // the records: the staged copy, or the caller's
+    float4 *stage;      // where the load writes them (null: read in place)
+    uint64_t begin;
+    uint32_t n;
+    uint32_t block0;      // first 256-point block of the per-point kernels
+    uint32_t batch0;      // first CTA of the batch kernel
+    uint32_t first_slot;  // first slot of the pool
+    MortonArgs m;
+    LodArgs lod[kMaxLevels - 1];
+};
+
+namespace {
+
+// The segments of a launch: one rides in the kernel's parameters (ONE), more
+// are read from device memory.
+struct Segs {
+    PackSeg one;
+    const PackSeg *list;
+    uint32_t n;
+};
+
+// Segment of block b among the segments' first blocks.
+template <bool ONE, uint32_t PackSeg::*FIRST>
+__device__ __forceinline__ uint32_t seg_of(const Segs &s, uint32_t b) {
+    uint32_t lo = 0;
+    if (!ONE)
+        for (uint32_t hi = s.n; hi - lo > 1u;) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (s.list[mid].*FIRST <= b)
+                lo = mid;
+            else
+                hi = mid;
+        }
+    return lo;
+}
+template <bool ONE>
+__device__ __forceinline__ const PackSeg &seg_at(const Segs &s, uint32_t i) {
+    if constexpr (ONE)
+        return s.one;
+    else
+        return s.list[i];
+}
+
+// Stages 0 and 1: raw input -> float4 positions + packed RGBA8
+// (GPUPacker/Shaders.metal:219-235; colour rule: uint(clamp(c, 0, 1) * 255),
+// truncating) and the bounds (packBounds, Shaders.metal:71-105).  One 16-byte
+// record per point: x, y, z and the packed RGBA8 colour's bits in w (moved,
+// never computed on), so the Morton-order gather brings both with one access.
+// blockIdx.y = segment.  One set of bounds atomics per CTA (a set per warp
+// kept the six words of a 140-thousand-point node busy for 18 us).
+constexpr int kLoadRounds = 4;
+template <bool ONE>
+__global__ void __launch_bounds__(kThreads)
+    pack_load_bounds(const __grid_constant__ Segs segs, uint32_t *__restrict__ bounds) {
+    const PackSeg &sg = seg_at<ONE>(segs, blockIdx.y);
+    const uint32_t n = sg.n;
+    const LoadArgs a = sg.la;
+    const float4 *pos = sg.pos;
+    float4 *stage = sg.stage;
+    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
+    const uint64_t step = (uint64_t)gridDim.x * kThreads;
+    auto widen = [&](const float4 &p) {
+        const uint32_t f[3] = {flip(p.x), flip(p.y), flip(p.z)};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            mn[d] = min(mn[d], f[d]);
+            mx[d] = max(mx[d], f[d]);
+        }
+    };
+    uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (!stage) {
+        for (; i + step * (kLoadRounds - 1) < n; i += step * kLoadRounds) {
+            float4 p[kLoadRounds];
+#pragma unroll
+            for (int k = 0; k < kLoadRounds; ++k) p[k] = pos[i + step * k];
+#pragma unroll
+            for (int k = 0; k < kLoadRounds; ++k) widen(p[k]);
+        }
+        for (; i < n; i += step) widen(pos[i]);
+    } else {
+        for (; i < n; i += step) {
+            const float *q = reinterpret_cast<const float *>(a.pos + i * a.pos_stride);
+            uint32_t col;
+            if (a.col_format == 1) {
+                col = *reinterpret_cast<const uint32_t *>(a.col + i * a.col_stride);
+            } else {
+                const float *c = reinterpret_cast<const float *>(a.col + i * a.col_stride);
+                const uint32_t r = (uint32_t)(fminf(fmaxf(c[0], 0.0f), 1.0f) * 255.0f);
+                const uint32_t g = (uint32_t)(fminf(fmaxf(c[1], 0.0f), 1.0f) * 255.0f);
+                const uint32_t b = (uint32_t)(fminf(fmaxf(c[2], 0.0f), 1.0f) * 255.0f);
+                const uint32_t al = (uint32_t)(fminf(fmaxf(c[3], 0.0f), 1.0f) * 255.0f);
+                col = r | (g << 8) | (b << 16) | (al << 24);
+            }
+            const float4 p = make_float4(q[0], q[1], q[2], __uint_as_float(col));
+            stage[i] = p;
+            widen(p);
+        }
+    }
+    __shared__ uint32_t part[6][kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const uint32_t x = __reduce_min_sync(0xffffffffu, mn[d]);
+        const uint32_t y = __reduce_min_sync(0xffffffffu, ~mx[d]);
+        if (lane == 0) {
+            part[d][warp] = x;
+            part[3 + d][warp] = y;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        uint32_t x = 0xffffffffu;
+        for (int w = 0; w < kThreads / 32; ++w) x = min(x, part[threadIdx.x][w]);
+        atomicMin(&bounds[8 * blockIdx.y + threadIdx.x], x);
+    }
+}
+
+// Morton keys.  63 bits: the low ten bits and the high eleven of each axis
+// are spread apart as 32-bit words, which the integer pipe does in fewer
+// operations than 64-bit shifts and masks.
+__device__ __forceinline__ uint32_t interleave10(uint32_t x, uint32_t y, uint32_t z) {
+    return (spread10(x) << 2) | (spread10(y) << 1) | spread10(z);
+}
+__device__ __forceinline__ void morton_key(uint32_t x, uint32_t y, uint32_t z, uint32_t &key) {
+    key = interleave10(x, y, z);
+}
+__device__ __forceinline__ void morton_key(uint32_t x, uint32_t y, uint32_t z,
+                                           unsigned long long &key) {
+    const uint32_t lo = interleave10(x, y, z);                    // key bits 0..29
+    const uint32_t mid = interleave10(x >> 10, y >> 10, z >> 10);  // key bits 30..59
+    const uint32_t top = ((x >> 20) << 2) | ((y >> 20) << 1) | (z >> 20);  // key bits 60..62
+    key = ((unsigned long long)((top << 28) | (mid >> 2)) << 32) | (lo | (mid << 30));
+}
+
+// Stage 2: Morton keys (packMorton, GPUPacker/Shaders.metal:109-126) and the
+// histograms of their 8-bit digits (a CTA counts in shared memory and adds
+// its counts once); the identity index the reference writes beside the keys
+// is made by the sort's first pass instead.  blockIdx.y = segment.  100M
+// 63-bit keys: 480 us, where the keys (577 us) and their histograms (362 us,
+// reading them again) were two kernels.
+template <typename K, bool ONE>
+__global__ void __launch_bounds__(kThreads)
+    pack_morton(const __grid_constant__ Segs segs, K *__restrict__ keys,
+                uint32_t *__restrict__ hist) {
+    constexpr int kPasses = sizeof(K) == 8 ? 8 : 4;
+    __shared__ uint32_t sh[kPasses * 256];
+    for (int i = threadIdx.x; i < kPasses * 256; i += kThreads) sh[i] = 0u;
+    __syncthreads();
+    const PackSeg &sg = seg_at<ONE>(segs, blockIdx.y);
+    const uint32_t n = sg.n;
+    const float4 *pos = sg.pos;
+    const MortonArgs m = sg.m;
+    keys += sg.begin;
+    const uint64_t step = (uint64_t)gridDim.x * kThreads;
+    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += step) {
+        const float4 p = pos[i];
+        const uint32_t qx = (uint32_t)fminf(fmaxf((p.x - m.bmin[0]) * m.scale[0], 0.0f), m.top);
+        const uint32_t qy = (uint32_t)fminf(fmaxf((p.y - m.bmin[1]) * m.scale[1], 0.0f), m.top);
+        const uint32_t qz = (uint32_t)fminf(fmaxf((p.z - m.bmin[2]) * m.scale[2], 0.0f), m.top);
+        K k;
+        morton_key(qx, qy, qz, k);
+        keys[i] = k;
+#pragma unroll
+        for (int d = 0; d < kPasses; ++d)
+            atomicAdd(&sh[d * 256 + ((uint32_t)(k >> (8 * d)) & 0xffu)], 1u);
+    }
+    __syncthreads();
+    uint32_t *out = hist + (size_t)blockIdx.y * kRadixMaxPasses * 256;
+    for (int i = threadIdx.x; i < kPasses * 256; i += kThreads)
+        if (sh[i]) atomicAdd(&out[i], sh[i]);
+}
+
+__device__ __forceinline__ uint32_t lod_cell(const float4 &p, const LodArgs &a) {
     const float lx = (p.x - a.bmin[0]) * a.inv;
     const float ly = (p.y - a.bmin[1]) * a.inv;
     const float lz = (p.z - a.bmin[2]) * a.inv;
     const uint32_t cx = min((uint32_t)max(0, (int)floorf(lx)), a.dims[0] - 1u);
     const uint32_t cy = min((uint32_t)max(0, (int)floorf(ly)), a.dims[1] - 1u);
     const uint32_t cz = min((uint32_t)max(0, (int)floorf(lz)), a.dims[2] - 1u);
-    return (uint64_t)cx + (uint64_t)a.dims[0] * ((uint64_t)cy + (uint64_t)a.dims[1] * cz);
+    return cx + a.dims[0] * (cy + a.dims[1] * cz);  // a grid has at most kLodCellCap cells
 }
 
 // Stage 5 (packLODClaim / packLODAssign, GPUPacker/Shaders.metal:337-371).
 // The points are in Morton order, so neighbouring lanes often share a cell;
 // lanes carry increasing indices, so the lowest lane of each group of lanes
 // with the same cell holds the group's minimum and alone does the atomicMin
-// (the grid ends the same: min is order-independent).  The last level's
-// assignment:
-__global__ void __launch_bounds__(kThreads)
-    pack_lod_assign(const float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint64_t n,
-                    LodArgs a, const uint32_t *__restrict__ grid) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n || lv[i] != a.max_level) return;
-    if (grid[lod_cell(sorted[i], a)] == (uint32_t)i) lv[i] = a.level;
-}
-
-// The claims are fused into the kernels that read the Morton-ordered points
-// anyway: the gather also claims the coarsest level (every point is still
-// unassigned there), and the assignment of level L also claims level L + 1
-// for the points it leaves unassigned (each level has its own grid), so the
-// points are read once per level instead of twice.
+// (the grid ends the same: min is order-independent).  The claims are fused
+// into the kernels that read the Morton-ordered points anyway: the gather
+// also claims the coarsest level (every point is still unassigned there),
+// and the assignment of level L also claims level L + 1 for the points it
+// leaves unassigned (each level has its own grid), so the points are read
+// once per level instead of twice.
 __device__ __forceinline__ void lod_claim_one(bool part, const float4 &p, uint32_t i,
-                                              const LodArgs &a, uint32_t *grid) {
+                                              const LodArgs &a) {
     const unsigned act = __ballot_sync(0xffffffffu, part);
     if (!part) return;
-    const uint64_t cell = lod_cell(p, a);
-    const unsigned same = __match_any_sync(act, (unsigned long long)cell);
-    if ((int)(__ffs(same) - 1) == (int)(threadIdx.x & 31u)) atomicMin(&grid[cell], i);
+    const uint32_t cell = lod_cell(p, a);
+    const unsigned same = __match_any_sync(act, cell);
+    if ((int)(__ffs(same) - 1) == (int)(threadIdx.x & 31u)) atomicMin(&a.grid[cell], i);
 }
 
+// The sort's values of a segment: where its indices ended up (null: the
+// input order stands).
+__device__ __forceinline__ const uint32_t *sorted_index(const uint32_t *vals0,
+                                                        const uint32_t *vals1, uint32_t set,
+                                                        uint64_t begin) {
+    return set == 0u ? nullptr : ((__popc(set) & 1) ? vals1 : vals0) + begin;
+}
+
+// Stage 4: gather into Morton order, all levels at max_level (packLODInit),
+// and the coarsest level's claims when there is more than one level.
+template <bool ONE>
 __global__ void __launch_bounds__(kThreads)
-    pack_gather_claim(const float4 *__restrict__ pos, const uint32_t *__restrict__ idx, uint64_t n,
-                      float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint8_t max_level,
-                      LodArgs a0, uint32_t *__restrict__ grid0) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool v = i < n;
+    pack_gather_claim(const __grid_constant__ Segs segs, const uint32_t *__restrict__ vals0,
+                      const uint32_t *__restrict__ vals1, const uint32_t *__restrict__ runs,
+                      float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint32_t max_level) {
+    const uint32_t si = seg_of<ONE, &PackSeg::block0>(segs, blockIdx.x);
+    const PackSeg &sg = seg_at<ONE>(segs, si);
+    const uint64_t i = (uint64_t)(blockIdx.x - sg.block0) * kThreads + threadIdx.x;
+    const bool v = i < sg.n;
+    const uint32_t *idx = sorted_index(vals0, vals1, runs[si], sg.begin);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     if (v) {
-        p = pos[idx[i]];
-        sorted[i] = p;
-        lv[i] = max_level;
+        p = sg.pos[idx ? idx[i] : (uint32_t)i];
+        sorted[sg.begin + i] = p;
+        lv[sg.begin + i] = (uint8_t)max_level;
     }
-    lod_claim_one(v, p, (uint32_t)i, a0, grid0);
+    if (max_level > 0u) lod_claim_one(v, p, (uint32_t)i, sg.lod[0]);
 }
 
+// Assignment of a level and, unless it is the last, the claims of the next.
+template <bool ONE, bool CLAIM>
 __global__ void __launch_bounds__(kThreads)
-    pack_lod_assign_claim(const float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint64_t n,
-                          LodArgs a, const uint32_t *__restrict__ grid, LodArgs next,
-                          uint32_t *__restrict__ grid_next) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool v = i < n && lv[i] == a.max_level;
+    pack_lod_assign(const __grid_constant__ Segs segs, const float4 *__restrict__ sorted,
+                    uint8_t *__restrict__ lv, uint32_t level, uint32_t max_level) {
+    const PackSeg &sg = seg_at<ONE>(segs, seg_of<ONE, &PackSeg::block0>(segs, blockIdx.x));
+    const uint64_t i = (uint64_t)(blockIdx.x - sg.block0) * kThreads + threadIdx.x;
+    const uint64_t at = sg.begin + i;
+    const bool v = i < sg.n && lv[at] == max_level;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     bool left = false;
     if (v) {
-        p = sorted[i];
-        if (grid[lod_cell(p, a)] == (uint32_t)i)
-            lv[i] = a.level;
+        p = sorted[at];
+        const LodArgs &a = sg.lod[level];
+        if (a.grid[lod_cell(p, a)] == (uint32_t)i)
+            lv[at] = (uint8_t)level;
         else
             left = true;
     }
-    lod_claim_one(left, p, (uint32_t)i, next, grid_next);
+    if (CLAIM) lod_claim_one(left, p, (uint32_t)i, sg.lod[level + 1]);
 }
 
 // Stages 6 and 7: per batch AABB, RasterBatch and stable level bucketing
@@ -267,28 +380,33 @@ __global__ void __launch_bounds__(kThreads)
 // passes.
 constexpr int kBatchRounds = 4;
 constexpr int kBatchThreads = 512;
-template <int NL>
+template <int NL, bool ONE>
 __global__ void __launch_bounds__(kBatchThreads)
-    pack_batches(const float4 *__restrict__ sorted, const uint8_t *__restrict__ lv, uint64_t n,
-                 uint32_t ppb, uint32_t first_slot, cr_raster_batch *__restrict__ batches,
-                 const uint32_t *__restrict__ idx_sorted, uint32_t *__restrict__ low,
-                 uint32_t *__restrict__ med, uint32_t *__restrict__ high,
-                 uint32_t *__restrict__ colors, uint8_t *__restrict__ levels,
-                 uint32_t *__restrict__ src_out) {
+    pack_batches(const __grid_constant__ Segs segs, const float4 *__restrict__ sorted,
+                 const uint8_t *__restrict__ lv, uint32_t ppb,
+                 const uint32_t *__restrict__ vals0, const uint32_t *__restrict__ vals1,
+                 const uint32_t *__restrict__ runs, cr_raster_batch *__restrict__ batches,
+                 uint32_t *__restrict__ low, uint32_t *__restrict__ med,
+                 uint32_t *__restrict__ high, uint32_t *__restrict__ colors,
+                 uint8_t *__restrict__ levels, uint32_t *__restrict__ src_out) {
     constexpr int kWarps = kBatchThreads / 32;
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ uint32_t red[6][kWarps];
     __shared__ uint32_t wcnt[kWarps][NL];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint64_t start = (uint64_t)blockIdx.x * ppb;
-    const uint64_t end = (start + ppb < n) ? start + ppb : n;
-    const uint32_t total = (uint32_t)(end - start);
+    const uint32_t si = seg_of<ONE, &PackSeg::batch0>(segs, blockIdx.x);
+    const PackSeg &sg = seg_at<ONE>(segs, si);
+    const uint32_t batch = blockIdx.x - sg.batch0;
+    const uint64_t start = (uint64_t)batch * ppb;  // in the segment
+    const uint32_t total = (uint32_t)min((uint64_t)sg.n - start, (uint64_t)ppb);
+    const uint32_t slot = sg.first_slot + batch;
+    const uint64_t pool = (uint64_t)slot * ppb;
     const uint32_t seg = (total + kWarps - 1u) / kWarps;
     const uint32_t s0 = min(total, (uint32_t)warp * seg);
     const uint32_t s1 = min(total, (uint32_t)(warp + 1) * seg);
-    const float4 *bsorted = sorted + start;
-    const uint8_t *blv = lv + start;
+    const float4 *bsorted = sorted + sg.begin + start;
+    const uint8_t *blv = lv + sg.begin + start;
     // 1. AABB and level counts of the warp's segment.
     uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
     uint32_t c[NL] = {};
@@ -365,7 +483,7 @@ __global__ void __launch_bounds__(kBatchThreads)
         rb.maxY = bmax[1];
         rb.maxZ = bmax[2];
         rb.numPoints = total;
-        rb.firstPoint = (first_slot + blockIdx.x) * ppb;
+        rb.firstPoint = slot * ppb;
         rb.fileIndex = 0;
         rb.lodCum01 = cum[0] | (cum[1] << 16);
         rb.lodCum23 = cum[2] | (cum[3] << 16);
@@ -373,10 +491,11 @@ __global__ void __launch_bounds__(kBatchThreads)
         rb.lodCum67 = cum[6] | (cum[7] << 16);
         rb.padding7 = 0;
         rb.padding8 = 0;
-        batches[blockIdx.x] = rb;
+        batches[slot] = rb;
     }
     // 3. Stable bucketing of the warp's segment, each point quantised into
     // its final place.
+    const uint32_t *idx = src_out ? sorted_index(vals0, vals1, runs[si], sg.begin) : nullptr;
     for (uint32_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
         float4 p[kBatchRounds];
         uint32_t raw[kBatchRounds];
@@ -406,7 +525,7 @@ __global__ void __launch_bounds__(kBatchThreads)
                 const uint32_t qx = (uint32_t)(nx * 1073741824.0f);
                 const uint32_t qy = (uint32_t)(ny * 1073741824.0f);
                 const uint32_t qz = (uint32_t)(nz * 1073741824.0f);
-                const uint64_t j = start + dst;
+                const uint64_t j = pool + dst;
                 low[j] = ((qx >> 20) & 1023u) | (((qy >> 20) & 1023u) << 10) |
                          (((qz >> 20) & 1023u) << 20);
                 med[j] = ((qx >> 10) & 1023u) | (((qy >> 10) & 1023u) << 10) |
@@ -414,7 +533,9 @@ __global__ void __launch_bounds__(kBatchThreads)
                 high[j] = (qx & 1023u) | ((qy & 1023u) << 10) | ((qz & 1023u) << 20);
                 colors[j] = __float_as_uint(p[k].w);
                 levels[j] = (uint8_t)raw[k];
-                if (src_out) src_out[j] = idx_sorted[start + i];
+                if (src_out)
+                    src_out[sg.begin + start + dst] =
+                        idx ? idx[start + i] : (uint32_t)(start + i);
             }
         }
     }
@@ -459,186 +580,323 @@ cr_status ensure_points(PackScratch &s, uint64_t n) {
     ALLOC(s.sorted, m * sizeof(float4));
     ALLOC(s.lv_morton, (m + 15) & ~15ull);
     ALLOC(s.src_idx, m * 4);
-    ALLOC(s.bounds, 8 * 4);
 #undef ALLOC
     s.cap_points = n;
     return CR_OK;
+}
+
+cr_status ensure_segs(PackScratch &s, uint64_t n) {
+    if (s.segs && s.cap_segs >= n) return CR_OK;
+    uint64_t have[3] = {0, 0, 0};  // grow() keeps a capacity per array; these three go together
+    s.cap_segs = 0;
+    cr_status st;
+    if ((st = grow(&s.segs, have[0], n)) || (st = grow(&s.rsegs, have[1], n)) ||
+        (st = grow(&s.bounds, have[2], 8 * n)))
+        return st;
+    s.cap_segs = n;
+    return CR_OK;
+}
+
+// Elements of a segment in the scratch arrays: whole 16-byte words of bytes.
+uint64_t padded(uint64_t n) { return (n + 15) & ~15ull; }
+
+// Launches kern<true> with the one segment in the parameters, or kern<false>
+// with the list.
+#define PACK_LAUNCH(nseg, grid, threads, stream, kern1, kernN, ...)      \
+    do {                                                                 \
+        if ((nseg) == 1u)                                                \
+            kern1<<<(grid), (threads), 0, (stream)>>>(__VA_ARGS__);      \
+        else                                                             \
+            kernN<<<(grid), (threads), 0, (stream)>>>(__VA_ARGS__);      \
+        CR_CUDA(cudaGetLastError());                                     \
+    } while (0)
+
+// The LOD grids of a segment from its bounds: level `level` has its own
+// dense grid.  Returns the cells of all levels in *cells.
+cr_status lod_args(PackSeg &sg, const float bmin[3], const float ext[3], int levels, int divs,
+                   uint64_t *cells_out) {
+    uint64_t total = 0;
+    const float longest = std::fmax(ext[0], std::fmax(ext[1], ext[2]));
+    const float base_voxel = longest / (float)divs;
+    for (int level = 0; level + 1 < levels; ++level) {
+        LodArgs &a = sg.lod[level];
+        const float voxel = base_voxel * std::pow(0.5f, (float)level);
+        a.inv = 1.0f / std::fmax(voxel, 0.000001f);
+        uint64_t cells = 1;
+        for (int k = 0; k < 3; ++k) {
+            a.bmin[k] = bmin[k];
+            const float d = std::floor(ext[k] * a.inv);
+            if (!(d < 2097151.0f))
+                return cri::fail(CR_ERR_CAPACITY, "LOD grid exceeds 2^21 cells per axis");
+            a.dims[k] = (uint32_t)d + 1u;
+            cells *= a.dims[k];
+        }
+        if (cells > kLodCellCap)
+            return cri::fail(CR_ERR_CAPACITY,
+                             "LOD grid of " + std::to_string(cells) + " cells exceeds the cap");
+        a.level = (uint32_t)level;
+        total += cells;
+    }
+    *cells_out = total;
+    return CR_OK;
+}
+
+// Packs jobs [0, njobs) in one run; *done = the jobs packed, fewer than
+// njobs when the grids of all would be too large together (at least one), or
+// when a job's grid is refused (an error, after packing the jobs before it).
+cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint32_t njobs,
+                    const cr_pack_params *prm, int on_device, uint32_t *src_idx_host,
+                    uint32_t *done) {
+    cudaStream_t s = ctx->stream;
+    PackScratch &sc = *ctx->pack;
+    const bool wide = prm->mortonBits == 21;
+    const uint32_t ppb = cloud->cap.pointsPerBatch;
+    uint64_t points = 0;
+    uint32_t largest = 0;
+    for (uint32_t j = 0; j < njobs; ++j) {
+        points += padded(jobs[j].count);
+        largest = std::max(largest, (uint32_t)jobs[j].count);
+    }
+    cr_status st = ensure_points(sc, points);
+    if (st) return st;
+    if ((st = ensure_segs(sc, njobs))) return st;
+    std::vector<PackSeg> segs(njobs);
+    std::vector<RadixSeg> rsegs(njobs);
+
+    // Stage 0: stage host input (one copy when the colour sits inside the
+    // position record).
+    std::vector<uint64_t> raw_off(njobs, 0);
+    uint64_t raw_bytes = 0;
+    auto layout = [](const cr_pack_input *in, uint64_t count, uint64_t &pbytes, uint64_t &cbytes,
+                     bool &inside) -> uint64_t {
+        const uint64_t csize = in->colorFormat == CR_COLOR_RGBA8 ? 4 : 16;
+        const uint8_t *hp = static_cast<const uint8_t *>(in->positions);
+        const uint8_t *hc = static_cast<const uint8_t *>(in->colors);
+        pbytes = (count - 1) * in->positionStrideBytes + 12;
+        cbytes = (count - 1) * in->colorStrideBytes + csize;
+        inside = hc >= hp && in->colorStrideBytes == in->positionStrideBytes &&
+                 (uint64_t)(hc - hp) + csize <= in->positionStrideBytes;
+        return inside ? std::max(pbytes, (uint64_t)(hc - hp) + cbytes)
+                      : ((pbytes + 255) & ~255ull) + cbytes;
+    };
+    if (!on_device) {
+        for (uint32_t j = 0; j < njobs; ++j) {
+            uint64_t pb, cb;
+            bool inside;
+            raw_off[j] = raw_bytes;
+            raw_bytes += (layout(jobs[j].in, jobs[j].count, pb, cb, inside) + 255) & ~255ull;
+        }
+        if ((st = grow(reinterpret_cast<uint8_t **>(&sc.raw), sc.cap_raw_bytes, raw_bytes)))
+            return st;
+    }
+    uint64_t begin = 0, blocks = 0, tiles = 0, batches = 0;
+    for (uint32_t j = 0; j < njobs; ++j) {
+        const cr_pack_input *in = jobs[j].in;
+        const uint64_t count = jobs[j].count;
+        PackSeg &sg = segs[j];
+        sg = PackSeg{};
+        sg.begin = begin;
+        sg.n = (uint32_t)count;
+        sg.block0 = (uint32_t)blocks;
+        sg.batch0 = (uint32_t)batches;
+        sg.first_slot = jobs[j].first_slot;
+        rsegs[j] = RadixSeg{begin, (uint32_t)count, (uint32_t)tiles};
+        LoadArgs &la = sg.la;
+        la.pos_stride = in->positionStrideBytes;
+        la.col_stride = in->colorStrideBytes;
+        la.col_format = in->colorFormat;
+        if (on_device) {
+            la.pos = static_cast<const uint8_t *>(in->positions);
+            la.col = static_cast<const uint8_t *>(in->colors);
+        } else {
+            const uint8_t *hp = static_cast<const uint8_t *>(in->positions);
+            const uint8_t *hc = static_cast<const uint8_t *>(in->colors);
+            uint64_t pbytes, cbytes;
+            bool inside;
+            const uint64_t need = layout(in, count, pbytes, cbytes, inside);
+            uint8_t *raw = static_cast<uint8_t *>(sc.raw) + raw_off[j];
+            la.pos = raw;
+            if (inside) {
+                CR_CUDA(cudaMemcpyAsync(raw, hp, need, cudaMemcpyHostToDevice, s));
+                la.col = raw + (hc - hp);
+            } else {
+                const uint64_t coff = (pbytes + 255) & ~255ull;
+                CR_CUDA(cudaMemcpyAsync(raw, hp, pbytes, cudaMemcpyHostToDevice, s));
+                CR_CUDA(cudaMemcpyAsync(raw + coff, hc, cbytes, cudaMemcpyHostToDevice, s));
+                la.col = raw + coff;
+            }
+        }
+        // Device-resident 16-byte records {x, y, z, rgba8} already have the
+        // layout of the staged positions: read them in place.
+        const bool in_place = on_device && in->positionStrideBytes == 16 &&
+                              in->colorStrideBytes == 16 && in->colorFormat == CR_COLOR_RGBA8 &&
+                              static_cast<const uint8_t *>(in->colors) ==
+                                  static_cast<const uint8_t *>(in->positions) + 12 &&
+                              ((uintptr_t)in->positions & 15) == 0;
+        sg.stage = in_place ? nullptr : sc.pos + begin;
+        sg.pos = in_place ? static_cast<const float4 *>(in->positions) : sc.pos + begin;
+        begin += padded(count);
+        blocks += grid_for(count);
+        tiles += radix_tiles((uint32_t)count);
+        batches += (count + ppb - 1) / ppb;
+    }
+    Segs arg;
+    arg.list = sc.segs;
+    auto upload = [&](uint32_t n) -> cr_status {
+        arg.n = n;
+        arg.one = segs[0];
+        if (n > 1)  // one segment travels in the kernels' parameters
+            CR_CUDA(cudaMemcpyAsync(sc.segs, segs.data(), n * sizeof(PackSeg),
+                                    cudaMemcpyHostToDevice, s));
+        return CR_OK;
+    };
+    if ((st = upload(njobs))) return st;
+    CR_CUDA(cudaMemcpyAsync(sc.rsegs, rsegs.data(), njobs * sizeof(RadixSeg),
+                            cudaMemcpyHostToDevice, s));
+
+    // Stage 1: bounds, read back once.
+    CR_CUDA(cudaMemsetAsync(sc.bounds, 0xff, (size_t)njobs * 8 * 4, s));
+    const unsigned sms = (unsigned)std::max(ctx->sm_count, 1);
+    auto rows = [&](uint32_t n) {  // CTAs of a segment in the two-dimensional launches
+        return std::max(1u, std::min(grid_for(largest), std::max(sms * 8u / n, 32u)));
+    };
+    PACK_LAUNCH(njobs, dim3(rows(njobs), njobs), kThreads, s, pack_load_bounds<true>,
+                pack_load_bounds<false>, arg, sc.bounds);
+    std::vector<uint32_t> bflip((size_t)njobs * 8);
+    CR_CUDA(cudaMemcpyAsync(bflip.data(), sc.bounds, bflip.size() * 4, cudaMemcpyDeviceToHost, s));
+    CR_CUDA(cudaStreamSynchronize(s));
+    const int L = std::max(1, std::min(prm->lodLevels, kMaxLevels));
+    const int divs = std::max(1, prm->coarseVoxelDivisions);
+    const uint32_t max_level = (uint32_t)(L - 1);
+    std::vector<uint64_t> cells(njobs, 0);
+    uint64_t cell_sum = 0;
+    uint32_t nseg = 0;
+    cr_status refused = CR_OK;
+    for (uint32_t j = 0; j < njobs; ++j) {
+        PackSeg &sg = segs[j];
+        float bmin[3], bmax[3], ext[3];
+        for (int k = 0; k < 3; ++k) {
+            bmin[k] = unflip(bflip[8 * j + k]);
+            bmax[k] = unflip(~bflip[8 * j + 3 + k]);
+            ext[k] = std::fmax(bmax[k] - bmin[k], 0.000001f);
+        }
+        sg.m.top = wide ? 2097151.0f : 1023.0f;
+        for (int k = 0; k < 3; ++k) {
+            sg.m.bmin[k] = bmin[k];
+            sg.m.scale[k] = sg.m.top / ext[k];
+        }
+        if ((refused = lod_args(sg, bmin, ext, L, divs, &cells[j]))) break;
+        if (j > 0 && cell_sum + cells[j] > kLodCellCap) break;
+        cell_sum += cells[j];
+        nseg = j + 1;
+    }
+    *done = nseg;
+    if (nseg == 0) return refused;
+    if (nseg < njobs) {
+        blocks = segs[nseg].block0;
+        batches = segs[nseg].batch0;
+        tiles = rsegs[nseg].tile0;
+    }
+    if ((st = grow(&sc.grid, sc.cap_grid, cell_sum))) return st;
+    uint64_t goff = 0;
+    for (uint32_t j = 0; j < nseg; ++j)
+        for (int level = 0; level + 1 < L; ++level) {
+            LodArgs &a = segs[j].lod[level];
+            a.grid = sc.grid + goff;
+            goff += (uint64_t)a.dims[0] * a.dims[1] * a.dims[2];
+        }
+    if ((st = upload(nseg))) return st;
+
+    // Stages 2-3: Morton keys and their digits' histograms, stable sort.
+    if ((st = radix_begin(sc.radix, nseg, tiles, s))) return st;
+    if (wide) {
+        using K = unsigned long long;
+        const RadixBuffers<K> buf{{static_cast<K *>(sc.keys[0]), static_cast<K *>(sc.keys[1])},
+                                  {sc.idx[0], sc.idx[1]}};
+        PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
+                    (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
+        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, 63, sc.radix, ctx->d_status, s);
+    } else {
+        using K = uint32_t;
+        const RadixBuffers<K> buf{{static_cast<K *>(sc.keys[0]), static_cast<K *>(sc.keys[1])},
+                                  {sc.idx[0], sc.idx[1]}};
+        PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
+                    (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
+        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, 30, sc.radix, ctx->d_status, s);
+    }
+    if (st) return st;
+
+    // Stages 4-5: gather, LOD levels (each level its own dense grid).
+    if (cell_sum) CR_CUDA(cudaMemsetAsync(sc.grid, 0xff, cell_sum * 4, s));
+    PACK_LAUNCH(nseg, (unsigned)blocks, kThreads, s, pack_gather_claim<true>,
+                pack_gather_claim<false>, arg, sc.idx[0], sc.idx[1], sc.radix.runs, sc.sorted,
+                sc.lv_morton, max_level);
+    for (uint32_t level = 0; level < max_level; ++level) {
+        if (level + 1 < max_level)
+            PACK_LAUNCH(nseg, (unsigned)blocks, kThreads, s, (pack_lod_assign<true, true>),
+                        (pack_lod_assign<false, true>), arg, sc.sorted, sc.lv_morton, level,
+                        max_level);
+        else
+            PACK_LAUNCH(nseg, (unsigned)blocks, kThreads, s, (pack_lod_assign<true, false>),
+                        (pack_lod_assign<false, false>), arg, sc.sorted, sc.lv_morton, level,
+                        max_level);
+    }
+
+    // Stages 6-7: batches, final order, quantisation into the pool; source
+    // indices only when asked for.
+    uint32_t *src = src_idx_host ? sc.src_idx : nullptr;
+    if (L <= 4)
+        PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<4, true>),
+                    (pack_batches<4, false>), arg, sc.sorted, sc.lv_morton, ppb, sc.idx[0],
+                    sc.idx[1], sc.radix.runs, cloud->d_batches, cloud->d_low, cloud->d_med,
+                    cloud->d_high, cloud->d_colors, cloud->d_levels, src);
+    else
+        PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<8, true>),
+                    (pack_batches<8, false>), arg, sc.sorted, sc.lv_morton, ppb, sc.idx[0],
+                    sc.idx[1], sc.radix.runs, cloud->d_batches, cloud->d_low, cloud->d_med,
+                    cloud->d_high, cloud->d_colors, cloud->d_levels, src);
+    if (src)
+        CR_CUDA(cudaMemcpyAsync(src_idx_host, src, jobs[0].count * 4, cudaMemcpyDeviceToHost, s));
+    return refused;
 }
 
 }  // namespace
 
 void pack_scratch_free(PackScratch &s) {
     void *ptrs[] = {s.raw, s.pos, s.keys[0], s.keys[1], s.idx[0], s.idx[1], s.sorted,
-                    s.lv_morton, s.grid, s.bounds, s.src_idx};
+                    s.lv_morton, s.grid, s.segs, s.rsegs, s.bounds, s.src_idx};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     radix_scratch_free(s.radix);
     s = PackScratch{};
 }
 
-// Packs `count` points into slots [first_slot, first_slot + ceil(count/ppb)) of
-// the cloud's pool.  Enqueues on the context stream; one synchronisation reads
-// the global bounds back to size the Morton scale and the LOD grid.
-cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const cr_pack_input *in, uint64_t count,
-                   const cr_pack_params *prm, int on_device, uint32_t first_slot,
-                   uint32_t *src_idx_host) {
-    cudaStream_t s = ctx->stream;
-    PackScratch &sc = *ctx->pack;
-    const bool wide = prm->mortonBits == 21;
-    cr_status st = ensure_points(sc, count);
-    if (st) return st;
-    const uint32_t ppb = cloud->cap.pointsPerBatch;
-    const uint32_t nb = (uint32_t)((count + ppb - 1) / ppb);
-
-    // Stage 0: stage host input (one copy when the colour sits inside the position record).
-    LoadArgs la;
-    la.pos_stride = in->positionStrideBytes;
-    la.col_stride = in->colorStrideBytes;
-    la.col_format = in->colorFormat;
-    const uint64_t csize = in->colorFormat == CR_COLOR_RGBA8 ? 4 : 16;
-    if (on_device) {
-        la.pos = static_cast<const uint8_t *>(in->positions);
-        la.col = static_cast<const uint8_t *>(in->colors);
-    } else {
-        const uint8_t *hp = static_cast<const uint8_t *>(in->positions);
-        const uint8_t *hc = static_cast<const uint8_t *>(in->colors);
-        const uint64_t pbytes = (count - 1) * in->positionStrideBytes + 12;
-        const uint64_t cbytes = (count - 1) * in->colorStrideBytes + csize;
-        const bool inside = hc >= hp && in->colorStrideBytes == in->positionStrideBytes &&
-                            (uint64_t)(hc - hp) + csize <= in->positionStrideBytes;
-        const uint64_t need = inside ? std::max(pbytes, (uint64_t)(hc - hp) + cbytes)
-                                     : ((pbytes + 255) & ~255ull) + cbytes;
-        if ((st = grow(reinterpret_cast<uint8_t **>(&sc.raw), sc.cap_raw_bytes, need))) return st;
-        uint8_t *raw = static_cast<uint8_t *>(sc.raw);
-        if (inside) {
-            CR_CUDA(cudaMemcpyAsync(raw, hp, need, cudaMemcpyHostToDevice, s));
-            la.pos = raw;
-            la.col = raw + (hc - hp);
-        } else {
-            const uint64_t coff = (pbytes + 255) & ~255ull;
-            CR_CUDA(cudaMemcpyAsync(raw, hp, pbytes, cudaMemcpyHostToDevice, s));
-            CR_CUDA(cudaMemcpyAsync(raw + coff, hc, cbytes, cudaMemcpyHostToDevice, s));
-            la.pos = raw;
-            la.col = raw + coff;
-        }
+// Packs every job into its slots of the cloud's pool.  Enqueues on the
+// context stream; one synchronisation per wave reads the segments' bounds
+// back to size the Morton scales and the LOD grids.  src_idx_host (one job
+// only): the input index of every packed point.  A wave takes jobs while
+// they hold at most kWavePoints points together, so that a long list of
+// chunks needs no more scratch than one chunk of that size.
+cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const std::vector<PackJob> &jobs,
+                   const cr_pack_params *prm, int on_device, uint32_t *src_idx_host) {
+    constexpr uint64_t kWavePoints = 1ull << 24;
+    constexpr size_t kWaveJobs = 4096;  // the launches' second grid dimension is bounded
+    if (src_idx_host && jobs.size() != 1)
+        return cri::fail(CR_ERR_INTERNAL, "pack_run: source indices of one job only");
+    size_t first = 0;
+    while (first < jobs.size()) {
+        size_t last = first;
+        uint64_t points = 0;
+        do {
+            points += padded(jobs[last].count);
+            ++last;
+        } while (last < jobs.size() && last - first < kWaveJobs &&
+                 points + padded(jobs[last].count) <= kWavePoints);
+        uint32_t done = 0;
+        const cr_status st = pack_wave(ctx, cloud, jobs.data() + first, (uint32_t)(last - first),
+                                       prm, on_device, src_idx_host, &done);
+        if (st) return st;
+        first += done;
     }
-    // Device-resident 16-byte records {x, y, z, rgba8} already have the
-    // layout of the staged positions: read them in place.
-    const bool in_place = on_device && in->positionStrideBytes == 16 &&
-                          in->colorStrideBytes == 16 && in->colorFormat == CR_COLOR_RGBA8 &&
-                          static_cast<const uint8_t *>(in->colors) ==
-                              static_cast<const uint8_t *>(in->positions) + 12 &&
-                          ((uintptr_t)in->positions & 15) == 0;
-    const float4 *pos = in_place ? static_cast<const float4 *>(in->positions) : sc.pos;
-    if (!in_place) {
-        pack_load<<<grid_for(count), kThreads, 0, s>>>(la, count, sc.pos);
-        CR_CUDA(cudaGetLastError());
-    }
-
-    // Stage 1: bounds, read back once.
-    const uint32_t binit[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    CR_CUDA(cudaMemcpyAsync(sc.bounds, binit, sizeof(binit), cudaMemcpyHostToDevice, s));
-    pack_bounds<<<std::min<unsigned>(grid_for(count), (unsigned)ctx->sm_count * 8), kThreads, 0,
-                  s>>>(pos, count, sc.bounds);
-    CR_CUDA(cudaGetLastError());
-    uint32_t bflip[6];
-    CR_CUDA(cudaMemcpyAsync(bflip, sc.bounds, sizeof(bflip), cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaStreamSynchronize(s));
-    float bmin[3], bmax[3], ext[3];
-    for (int k = 0; k < 3; ++k) {
-        bmin[k] = unflip(bflip[k]);
-        bmax[k] = unflip(bflip[3 + k]);
-        ext[k] = std::fmax(bmax[k] - bmin[k], 0.000001f);
-    }
-
-    // Stage 2-3: Morton keys, stable sort.
-    MortonArgs ma;
-    ma.top = wide ? 2097151.0f : 1023.0f;
-    for (int k = 0; k < 3; ++k) {
-        ma.bmin[k] = bmin[k];
-        ma.scale[k] = ma.top / ext[k];
-    }
-    bool in_alt = false;
-    if (wide) {
-        auto *k0 = static_cast<unsigned long long *>(sc.keys[0]);
-        auto *k1 = static_cast<unsigned long long *>(sc.keys[1]);
-        pack_morton<unsigned long long><<<grid_for(count), kThreads, 0, s>>>(pos, count, ma, k0);
-        CR_CUDA(cudaGetLastError());
-        st = radix_sort_pairs<unsigned long long>(k0, sc.idx[0], k1, sc.idx[1], count, 63, true,
-                                                  sc.radix, ctx->d_status, ctx->sm_count, s,
-                                                  &in_alt);
-    } else {
-        auto *k0 = static_cast<uint32_t *>(sc.keys[0]);
-        auto *k1 = static_cast<uint32_t *>(sc.keys[1]);
-        pack_morton<uint32_t><<<grid_for(count), kThreads, 0, s>>>(pos, count, ma, k0);
-        CR_CUDA(cudaGetLastError());
-        st = radix_sort_pairs<uint32_t>(k0, sc.idx[0], k1, sc.idx[1], count, 30, true, sc.radix,
-                                        ctx->d_status, ctx->sm_count, s, &in_alt);
-    }
-    if (st) return st;
-    const uint32_t *idx_sorted = sc.idx[in_alt ? 1 : 0];
-
-    // Stage 4-5: gather, LOD levels (each level its own dense grid).
-    const int L = std::max(1, std::min(prm->lodLevels, 8));
-    const int divs = std::max(1, prm->coarseVoxelDivisions);
-    const uint8_t max_level = (uint8_t)(L - 1);
-    if (L == 1) {
-        pack_gather<<<grid_for(count), kThreads, 0, s>>>(pos, idx_sorted, count, sc.sorted,
-                                                         sc.lv_morton, max_level);
-        CR_CUDA(cudaGetLastError());
-    } else {
-        const float longest = std::fmax(ext[0], std::fmax(ext[1], ext[2]));
-        const float base_voxel = longest / (float)divs;
-        std::vector<LodArgs> la_(L - 1);
-        std::vector<uint64_t> goff(L);
-        goff[0] = 0;
-        for (int level = 0; level < L - 1; ++level) {
-            LodArgs &a = la_[level];
-            const float voxel = base_voxel * std::pow(0.5f, (float)level);
-            a.inv = 1.0f / std::fmax(voxel, 0.000001f);
-            uint64_t cells = 1;
-            for (int k = 0; k < 3; ++k) {
-                a.bmin[k] = bmin[k];
-                const float d = std::floor(ext[k] * a.inv);
-                if (!(d < 2097151.0f))
-                    return cri::fail(CR_ERR_CAPACITY, "LOD grid exceeds 2^21 cells per axis");
-                a.dims[k] = (uint32_t)d + 1u;
-                cells *= a.dims[k];
-            }
-            if (cells > kLodCellCap)
-                return cri::fail(CR_ERR_CAPACITY,
-                                 "LOD grid of " + std::to_string(cells) + " cells exceeds the cap");
-            a.max_level = max_level;
-            a.level = (uint8_t)level;
-            goff[level + 1] = goff[level] + cells;
-        }
-        if ((st = grow(&sc.grid, sc.cap_grid, goff[L - 1]))) return st;
-        CR_CUDA(cudaMemsetAsync(sc.grid, 0xff, goff[L - 1] * 4, s));
-        pack_gather_claim<<<grid_for(count), kThreads, 0, s>>>(
-            pos, idx_sorted, count, sc.sorted, sc.lv_morton, max_level, la_[0], sc.grid);
-        CR_CUDA(cudaGetLastError());
-        for (int level = 0; level + 1 < L - 1; ++level) {
-            pack_lod_assign_claim<<<grid_for(count), kThreads, 0, s>>>(
-                sc.sorted, sc.lv_morton, count, la_[level], sc.grid + goff[level],
-                la_[level + 1], sc.grid + goff[level + 1]);
-            CR_CUDA(cudaGetLastError());
-        }
-        pack_lod_assign<<<grid_for(count), kThreads, 0, s>>>(sc.sorted, sc.lv_morton, count,
-                                                             la_[L - 2], sc.grid + goff[L - 2]);
-        CR_CUDA(cudaGetLastError());
-    }
-
-    // Stages 6-7: batches, final order, quantisation into the pool.
-    cr_raster_batch *dst_batches = cloud->d_batches + first_slot;
-    const uint64_t p0 = (uint64_t)first_slot * ppb;
-    auto *batch_kernel = L <= 4 ? pack_batches<4> : pack_batches<8>;
-    batch_kernel<<<nb, kBatchThreads, 0, s>>>(
-        sc.sorted, sc.lv_morton, count, ppb, first_slot, dst_batches, idx_sorted,
-        cloud->d_low + p0, cloud->d_med + p0, cloud->d_high + p0, cloud->d_colors + p0,
-        cloud->d_levels + p0,
-        src_idx_host ? sc.src_idx : nullptr);  // source indices only when asked for
-    CR_CUDA(cudaGetLastError());
-    if (src_idx_host)
-        CR_CUDA(cudaMemcpyAsync(src_idx_host, sc.src_idx, count * 4, cudaMemcpyDeviceToHost, s));
     return CR_OK;
 }

@@ -3,23 +3,27 @@
 // The reference packer (Pipelines/GPUPacker/Shaders.metal:134-215) sorts
 // 30-bit Morton keys with four 8-bit passes, one *thread* per 1024-key tile
 // walking the tile serially so histogram and scatter agree on order.  Here
-// the sort reads the keys once for the histograms of every digit, then runs
-// one kernel per 8-bit digit that reads each key and value once and writes
-// them once (a single-sweep pass with decoupled look-back):
-//   radix_histograms  one read of all keys: the 256-bin histogram of every
-//                     digit position; the host reads them back, skips the
-//                     passes whose digit is the same for every key and turns
-//                     the rest into digit bases (exclusive scans);
+// one kernel per 8-bit digit reads each key and value once and writes them
+// once (a single-sweep pass with decoupled look-back).  The arrays hold one
+// or more segments (the clouds of one call), each sorted by itself:
+//   (caller)          the 256-bin histograms of every digit of every segment,
+//                     beside the keys it makes (RadixScratch::hist);
+//   radix_bases       per segment: exclusive scans into digit bases, and the
+//                     set of digits that its keys do not all share (a pass
+//                     over the others would move nothing and is skipped);
 //   radix_onesweep    per pass, 4096-key tiles taken in ticket order: a tile
 //                     ranks its keys among equal digits in input order (warp
 //                     multisplit with ballots, then scans over warps and
 //                     digits), publishes its per-digit counts, sums the
-//                     counts of the tiles before it per digit (look-back over
-//                     their published counts and inclusive prefixes, a
-//                     thread per digit), sorts the tile by digit in shared
-//                     memory and writes one coalesced run per digit.  Equal
-//                     keys keep their input order (stable), as the CPU's
-//                     stable sort does.
+//                     counts of its segment's tiles before it per digit
+//                     (look-back over their published counts and inclusive
+//                     prefixes, a thread per digit), sorts the tile by digit
+//                     in shared memory and writes one coalesced run per
+//                     digit.  Equal keys keep their input order (stable), as
+//                     the CPU's stable sort does.
+// Nothing is read back: which of the two buffers a segment's pass reads
+// follows from the segment's set of digits (bit p: pass p runs), and so does
+// where its sorted keys and indices end up.
 // A tile waits only for tiles with smaller tickets, which started before it,
 // so the waits end whatever the GPU schedules; each wait is nevertheless
 // bounded (kLookbackLimit polls), after which the tile counts the missing
@@ -71,32 +75,6 @@ constexpr int kLookbackBatch = CR_LOOKBACK_BATCH;  // predecessor words one roun
 using WarpCount = uint16_t;
 constexpr int kSortBlocksPerSM = 4;
 
-// Histograms of every 8-bit digit of the keys (grid-stride, per-CTA shared
-// counts added to global memory once per CTA).
-template <typename K>
-__global__ void __launch_bounds__(kThreads)
-    radix_histograms(const K *__restrict__ keys, uint64_t n, int passes,
-                     uint32_t *__restrict__ hist) {
-    __shared__ uint32_t sh[8 * 256];
-    for (int i = threadIdx.x; i < passes * 256; i += kThreads) sh[i] = 0u;
-    __syncthreads();
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * kThreads) {
-        const K k = keys[i];
-        for (int p = 0; p < passes; ++p)
-            atomicAdd(&sh[p * 256 + ((uint32_t)(k >> (8 * p)) & 0xffu)], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * 256; i += kThreads)
-        if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
-
-// The values of a sort that ran no pass: their input positions.
-__global__ void __launch_bounds__(kThreads) radix_iota(uint32_t *__restrict__ vals, uint64_t n) {
-    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) vals[i] = (uint32_t)i;
-}
-
 // Inclusive warp scan.
 __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
 #pragma unroll
@@ -105,6 +83,38 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
         if (lane >= o) x += y;
     }
     return x;
+}
+
+// A segment's digit bases and the set of its passes: one CTA per segment, a
+// thread per digit.
+__global__ void __launch_bounds__(kThreads)
+    radix_bases(const uint32_t *__restrict__ hist, const RadixSeg *__restrict__ segs, int passes,
+                uint32_t *__restrict__ bases, uint32_t *__restrict__ runs) {
+    __shared__ uint32_t sums[kRadixMaxPasses][kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t n = segs[blockIdx.x].n;
+    const size_t row = (size_t)blockIdx.x * kRadixMaxPasses * 256;
+    uint32_t set = 0, incl[kRadixMaxPasses], mine[kRadixMaxPasses];
+#pragma unroll
+    for (int p = 0; p < kRadixMaxPasses; ++p)
+        mine[p] = p < passes ? hist[row + p * 256 + threadIdx.x] : 0u;
+#pragma unroll
+    for (int p = 0; p < kRadixMaxPasses; ++p) {
+        incl[p] = warp_inclusive(mine[p], lane);
+        if (lane == 31) sums[p][warp] = incl[p];
+        // Every key has this digit: the pass is a copy.
+        const bool constant = __syncthreads_or(mine[p] == n);
+        if (p < passes && !constant) set |= 1u << p;
+    }
+#pragma unroll
+    for (int p = 0; p < kRadixMaxPasses; ++p) {
+        uint32_t base = incl[p] - mine[p];
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w)
+            if (w < warp) base += sums[p][w];
+        if (p < passes) bases[row + p * 256 + threadIdx.x] = base;
+    }
+    if (threadIdx.x == 0) runs[blockIdx.x] = set;
 }
 
 template <typename K>
@@ -123,12 +133,15 @@ struct DigitOf {
     __device__ __forceinline__ uint32_t of_word(uint32_t w) const {
         return __byte_perm(w, 0u, sel);
     }
-    // Digit of key i of an array in global or shared memory.
+    // Digit of key i of an array in global memory that the kernel only reads
+    // (__ldg, here and where the keys move: a plain load cannot pass the
+    // barriers and shared-memory stores between two keys; a pass over 100M
+    // keys took 975 us instead of 750 us with them).
     __device__ __forceinline__ uint32_t at(const uint32_t *keys, uint32_t i) const {
-        return of_word(keys[i]);
+        return of_word(__ldg(keys + i));
     }
     __device__ __forceinline__ uint32_t at(const unsigned long long *keys, uint32_t i) const {
-        return of_word(reinterpret_cast<const uint32_t *>(keys)[2u * i + word]);
+        return of_word(__ldg(reinterpret_cast<const uint32_t *>(keys) + (2u * i + word)));
     }
     __device__ __forceinline__ uint32_t of(uint32_t k) const { return of_word(k); }
     __device__ __forceinline__ uint32_t of(unsigned long long k) const {
@@ -170,7 +183,9 @@ __device__ __forceinline__ void rank_keys(const K *keys, uint32_t w0, uint32_t t
 }
 
 // Moves a warp's keys and values to their places in the tile sorted by digit.
-template <typename K, bool kIota, bool FULL>
+// vals null: the values are the keys' places in their segment (tile0: the
+// tile's).
+template <typename K, bool FULL>
 __device__ __forceinline__ void move_keys(const K *keys, const uint32_t *vals, uint32_t tile0,
                                           uint32_t w0, uint32_t tile_n, const WarpCount *wc,
                                           const uint32_t (&rd)[kKeysPerLane], K *skey,
@@ -181,8 +196,8 @@ __device__ __forceinline__ void move_keys(const K *keys, const uint32_t *vals, u
         const uint32_t li = w0 + (uint32_t)j * 32u + lane;
         if (FULL || li < tile_n) {
             const uint32_t slot = wc[rd[j] >> 16] + (rd[j] & 0xffffu);
-            skey[slot] = keys[li];
-            sval[slot] = kIota ? tile0 + li : vals[li];
+            skey[slot] = __ldg(keys + li);
+            sval[slot] = vals ? __ldg(vals + li) : tile0 + li;
         }
     }
 }
@@ -221,11 +236,12 @@ __device__ __forceinline__ void write_keys(const K *skey, const uint32_t *sval,
 // 83 % busy), so the full tiles have code without bounds (every tile but the
 // last), a digit is one byte permute of the word that holds it, offsets are
 // 32 bits and one shared word gives a key's place.
-template <typename K, bool kIota>
+// The first pass that a segment runs makes the values (the keys' places in
+// the segment); the pass before it wrote none.
+template <typename K>
 __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
-    radix_onesweep(const K *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
-                   K *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n,
-                   int shift, const uint32_t *__restrict__ digit_base,
+    radix_onesweep(RadixBuffers<K> buf, const RadixSeg *__restrict__ segs, uint32_t nseg, int pass,
+                   const uint32_t *__restrict__ bases, const uint32_t *__restrict__ runs,
                    unsigned long long *__restrict__ lookback, uint32_t epoch,
                    uint32_t *__restrict__ tile_counter, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -238,17 +254,36 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
     uint32_t *misc = gbase + 256;            // [0] ticket, [1..8] warp sums of the digit scan
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const DigitOf dig(shift);
+    const DigitOf dig(8 * pass);
     if (threadIdx.x == 0) misc[0] = atomicAdd(tile_counter, 1u);
     static_assert(kWarps * 256 * sizeof(WarpCount) == kThreads * sizeof(uint4), "one store each");
     reinterpret_cast<uint4 *>(wcnt)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    const uint32_t tile = misc[0];
+    const uint32_t gtile = misc[0];
+    // The segment of the tile, and its tile in the segment.
+    uint32_t si = 0;
+    for (uint32_t hi = nseg; hi - si > 1u;) {
+        const uint32_t mid = (si + hi) >> 1;
+        if (segs[mid].tile0 <= gtile)
+            si = mid;
+        else
+            hi = mid;
+    }
+    const RadixSeg sg = segs[si];
+    const uint32_t set = runs[si];
+    if (!(set >> pass & 1u)) return;  // every key of the segment has this digit
+    const uint32_t done = __popc(set & ((1u << pass) - 1u));  // passes before this one
+    const uint32_t n = sg.n, tile = gtile - sg.tile0;
     const uint32_t tile0 = tile * (uint32_t)kTileKeys;  // below n
     const uint32_t tile_n = min(n - tile0, (uint32_t)kTileKeys);
     const bool full = tile_n == (uint32_t)kTileKeys;
-    keys_in += tile0;
-    if (!kIota) vals_in += tile0;
+    const bool odd = done & 1u;
+    const K *keys_in = (odd ? buf.keys[1] : buf.keys[0]) + sg.begin + tile0;
+    const uint32_t *vals_in =
+        done ? (odd ? buf.vals[1] : buf.vals[0]) + sg.begin + tile0 : nullptr;
+    K *keys_out = (odd ? buf.keys[0] : buf.keys[1]) + sg.begin;
+    uint32_t *vals_out = (odd ? buf.vals[0] : buf.vals[1]) + sg.begin;
+    const uint32_t *digit_base = bases + ((size_t)si * kRadixMaxPasses + pass) * 256;
     const uint32_t w0 = (uint32_t)warp * (32 * kKeysPerLane);
     // 1. Warp-level ranking in input order; a key's rank within its warp
     //    (< 512) and digit are kept packed, the key and value are read again
@@ -268,6 +303,7 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
         cw[w] = wcnt[w * 256 + dd];
         total += cw[w];
     }
+    lookback += (size_t)sg.tile0 * 256;  // the segment's words
     unsigned long long *my = lookback + (size_t)tile * 256 + dd;
     // Publish the tile's count first (tile 0: its prefix), so that the tiles
     // after it can go on while this one sorts its keys.
@@ -292,9 +328,9 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
     __syncthreads();
     // 3. The tile sorted by digit.
     if (full)
-        move_keys<K, kIota, true>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
+        move_keys<K, true>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
     else
-        move_keys<K, kIota, false>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
+        move_keys<K, false>(keys_in, vals_in, tile0, w0, tile_n, wc, rd, skey, sval);
     // The look-back (thread d, digit d) over the tiles before this one, after
     // the tile-local work so that its waits overlap it.
     unsigned long long excl = 0;
@@ -363,71 +399,50 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
 }  // namespace
 
 void radix_scratch_free(RadixScratch &r) {
-    void *ptrs[] = {r.lookback, r.hist, r.bases, r.tiles};
+    void *ptrs[] = {r.lookback, r.hist, r.bases, r.runs, r.tiles};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     r = RadixScratch{};
 }
 
-template <typename K>
-cr_status radix_sort_pairs(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_alt, uint64_t n,
-                           int key_bits, bool vals_iota, RadixScratch &rs, uint32_t *status,
-                           int sm_count, cudaStream_t s, bool *result_in_alt) {
-    *result_in_alt = false;
-    if (n <= 1) {
-        if (vals_iota && n == 1) CR_CUDA(cudaMemsetAsync(vals, 0, sizeof(uint32_t), s));
-        return CR_OK;
-    }
-    if (n >= (1ull << 32)) return cri::fail(CR_ERR_CAPACITY, "radix sort: at most 2^32 - 1 keys");
-    const int passes = (key_bits + 7) / 8;
-    const uint64_t ntiles = (n + kTileKeys - 1) / kTileKeys;
-    // Scratch: look-back words (tiles x 256), histograms and bases (8 x 256),
-    // tile tickets (one per pass).
-    if (!rs.lookback || rs.cap_tiles < ntiles) {
+uint32_t radix_tiles(uint32_t n) {
+    return n / (uint32_t)kTileKeys + (n % (uint32_t)kTileKeys != 0u ? 1u : 0u);
+}
+
+cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStream_t s) {
+    if (!rs.lookback || rs.cap_tiles < ntiles || rs.cap_segs < nseg) {
+        const uint64_t tiles = std::max(ntiles, rs.cap_tiles);
+        const uint32_t segs = std::max(nseg, rs.cap_segs);
         radix_scratch_free(rs);
-        CR_CUDA(cudaMalloc((void **)&rs.lookback, ntiles * 256 * sizeof(unsigned long long)));
-        CR_CUDA(cudaMalloc((void **)&rs.hist, 8 * 256 * sizeof(uint32_t)));
-        CR_CUDA(cudaMalloc((void **)&rs.bases, 8 * 256 * sizeof(uint32_t)));
-        CR_CUDA(cudaMalloc((void **)&rs.tiles, 8 * sizeof(uint32_t)));
-        CR_CUDA(cudaMemsetAsync(rs.lookback, 0, ntiles * 256 * sizeof(unsigned long long), s));
-        rs.cap_tiles = ntiles;
+        const size_t rows = (size_t)segs * kRadixMaxPasses * 256;
+        CR_CUDA(cudaMalloc((void **)&rs.lookback, tiles * 256 * sizeof(unsigned long long)));
+        CR_CUDA(cudaMalloc((void **)&rs.hist, rows * sizeof(uint32_t)));
+        CR_CUDA(cudaMalloc((void **)&rs.bases, rows * sizeof(uint32_t)));
+        CR_CUDA(cudaMalloc((void **)&rs.runs, segs * sizeof(uint32_t)));
+        CR_CUDA(cudaMalloc((void **)&rs.tiles, kRadixMaxPasses * sizeof(uint32_t)));
+        CR_CUDA(cudaMemsetAsync(rs.lookback, 0, tiles * 256 * sizeof(unsigned long long), s));
+        rs.cap_tiles = tiles;
+        rs.cap_segs = segs;
         rs.epoch = 0;
     }
-    CR_CUDA(cudaMemsetAsync(rs.hist, 0, 8 * 256 * sizeof(uint32_t), s));
-    CR_CUDA(cudaMemsetAsync(rs.tiles, 0, 8 * sizeof(uint32_t), s));
-    const unsigned hgrid = (unsigned)std::min<uint64_t>((n + kThreads - 1) / kThreads,
-                                                        (uint64_t)std::max(sm_count, 1) * 8);
-    radix_histograms<K><<<hgrid, kThreads, 0, s>>>(keys, n, passes, rs.hist);
+    CR_CUDA(cudaMemsetAsync(rs.hist, 0, (size_t)nseg * kRadixMaxPasses * 256 * sizeof(uint32_t), s));
+    CR_CUDA(cudaMemsetAsync(rs.tiles, 0, kRadixMaxPasses * sizeof(uint32_t), s));
+    return CR_OK;
+}
+
+template <typename K>
+cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
+                     uint64_t ntiles, int key_bits, RadixScratch &rs, uint32_t *status,
+                     cudaStream_t s) {
+    const int passes = (key_bits + 7) / 8;
+    if (nseg == 0 || passes > kRadixMaxPasses || ntiles > rs.cap_tiles || nseg > rs.cap_segs)
+        return cri::fail(CR_ERR_INTERNAL, "radix_sort: arguments");
+    radix_bases<<<nseg, kThreads, 0, s>>>(rs.hist, segs, passes, rs.bases, rs.runs);
     CR_CUDA(cudaGetLastError());
-    // The histograms on the host: skip the passes whose digit every key
-    // shares, exclusive scans into the digit bases of the others.
-    std::vector<uint32_t> hist(8 * 256), bases(8 * 256, 0u);
-    CR_CUDA(cudaMemcpyAsync(hist.data(), rs.hist, passes * 256 * sizeof(uint32_t),
-                            cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> run;
-    for (int p = 0; p < passes; ++p) {
-        uint32_t acc = 0;
-        bool constant = false;
-        for (int d = 0; d < 256; ++d) {
-            bases[p * 256 + d] = acc;
-            acc += hist[p * 256 + d];
-            if (hist[p * 256 + d] == n) constant = true;
-        }
-        if (!constant) run.push_back(p);
-    }
-    CR_CUDA(cudaMemcpyAsync(rs.bases, bases.data(), passes * 256 * sizeof(uint32_t),
-                            cudaMemcpyHostToDevice, s));
     const size_t smem = onesweep_smem_bytes<K>();
-    for (auto *f : {radix_onesweep<K, false>, radix_onesweep<K, true>})
-        CR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (run.empty() && vals_iota) {
-        radix_iota<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(vals, n);
-        CR_CUDA(cudaGetLastError());
-    }
-    K *kin = keys, *kout = keys_alt;
-    uint32_t *vin = vals, *vout = vals_alt;
-    for (int p : run) {
+    CR_CUDA(cudaFuncSetAttribute(radix_onesweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    for (int p = 0; p < passes; ++p) {
         // A fresh epoch per pass, so the look-back words never need clearing;
         // after 65534 epochs the words are cleared once.
         if (++rs.epoch >= 0xffffu) {
@@ -435,24 +450,15 @@ cr_status radix_sort_pairs(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_
                                     rs.cap_tiles * 256 * sizeof(unsigned long long), s));
             rs.epoch = 1;
         }
-        // The first pass of an index sort makes the indices (kIota).
-        auto *kern = vals_iota && p == run.front() ? radix_onesweep<K, true>
-                                                   : radix_onesweep<K, false>;
-        kern<<<(unsigned)ntiles, kThreads, smem, s>>>(kin, vin, kout, vout, (uint32_t)n, 8 * p,
-                                                     rs.bases + p * 256, rs.lookback, rs.epoch,
-                                                     rs.tiles + p, status);
+        radix_onesweep<K><<<(unsigned)ntiles, kThreads, smem, s>>>(
+            buf, segs, nseg, p, rs.bases, rs.runs, rs.lookback, rs.epoch, rs.tiles + p, status);
         CR_CUDA(cudaGetLastError());
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-        *result_in_alt = !*result_in_alt;
     }
     return CR_OK;
 }
 
-template cr_status radix_sort_pairs<uint32_t>(uint32_t *, uint32_t *, uint32_t *, uint32_t *,
-                                              uint64_t, int, bool, RadixScratch &, uint32_t *,
-                                              int, cudaStream_t, bool *);
-template cr_status radix_sort_pairs<unsigned long long>(unsigned long long *, uint32_t *,
-                                                        unsigned long long *, uint32_t *, uint64_t,
-                                                        int, bool, RadixScratch &, uint32_t *, int,
-                                                        cudaStream_t, bool *);
+template cr_status radix_sort<uint32_t>(const RadixBuffers<uint32_t> &, const RadixSeg *, uint32_t,
+                                        uint64_t, int, RadixScratch &, uint32_t *, cudaStream_t);
+template cr_status radix_sort<unsigned long long>(const RadixBuffers<unsigned long long> &,
+                                                  const RadixSeg *, uint32_t, uint64_t, int,
+                                                  RadixScratch &, uint32_t *, cudaStream_t);

@@ -24,3 +24,45 @@ def test_batch_sizes_and_levels(cr, orc, ctx, n, ppb, lod):
                    coarseVoxelDivisions=5)
     cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, ppb=ppb, lod=lod, divs=5)
     check_region(cloud, ref, 0, ppb, src)
+
+
+@pytest.mark.parametrize("bits", [10, 21])
+@pytest.mark.parametrize("device", [False, True])
+def test_many_chunks_in_one_call(cr, orc, ctx, bits, device):
+    """Chunks around the tile and block sizes, one of a single point, one
+    whose points all coincide (no sort pass moves anything) and one of a
+    plane, packed by shared launches: each as the CPU packs it alone."""
+    torch = pytest.importorskip("torch")
+    ppb = 1000
+    chunks = []
+    for k, n in enumerate((1, 255, 4096, 4097, 9000, 300, 12288)):
+        pos, rgba = blob_cloud(n, 40 + k, scale=0.5 + k)
+        if k == 4:
+            pos[:] = pos[0]
+        if k == 5:
+            pos[:, 2] = 0.25
+        chunks.append((pos, rgba))
+    cloud = cr.ComputeRasteriserPointCloud(ctx, cr.ComputeRasteriserCapacity(40, ppb))
+    given = chunks
+    if device:
+        given = [(torch.from_numpy(p).cuda(), torch.from_numpy(c.view("int32")).cuda())
+                 for p, c in chunks]
+        torch.cuda.synchronize()
+    first = cloud.addRawChunksGPU(cr.GPUPacker(ctx, mortonBits=bits), given)
+    assert len(first) == len(chunks)
+    for f, (pos, rgba) in zip(first, chunks):
+        ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=ppb, morton_bits=bits)
+        check_region(cloud, ref, f, ppb)
+    assert cloud.pointCount == sum(len(p) for p, _ in chunks)
+
+
+def test_refused_chunk_is_still_refused(cr, ctx):
+    """A chunk with an infinite coordinate has no LOD grid: the call fails and
+    nothing of it becomes resident, as before."""
+    pos, rgba = blob_cloud(500, 3)
+    bad = pos.copy()
+    bad[7, 1] = float("inf")
+    cloud = cr.ComputeRasteriserPointCloud(ctx, cr.ComputeRasteriserCapacity(8, 256))
+    with pytest.raises(cr.CRError):
+        cloud.addRawChunksGPU(cr.GPUPacker(ctx), [(pos, rgba), (bad, rgba)])
+    assert cloud.residentBatchCount == 0
