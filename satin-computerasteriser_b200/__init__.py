@@ -18,7 +18,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import os
-from dataclasses import dataclass, field, fields
+from dataclasses import dataclass, field
 
 import numpy as np
 
@@ -46,11 +46,16 @@ SCREEN_SPACE = 0  # PointSizeMode.screenSpace
 WORLD_SPACE = 1   # PointSizeMode.worldSpace
 
 
+_F32 = np.dtype(np.float32)
+
+
 def _mat16(m) -> np.ndarray:
     """A 4x4 matrix as the column-major float[16] the ABI takes.
 
     Accepts a flat 16-vector (already column-major) or a 4x4 array in
     row-major math notation (m[row][col]), which is transposed."""
+    if type(m) is np.ndarray and m.dtype == _F32 and m.shape == (16,) and m.flags.c_contiguous:
+        return m
     a = np.asarray(m, dtype=np.float32)
     if a.shape == (4, 4):
         a = a.T
@@ -62,11 +67,12 @@ def matrix_multiply(a, b) -> np.ndarray:
     operation order (rows summed k = 0..3 left to right, no FMA)."""
     A, B = _mat16(a).reshape(4, 4), _mat16(b).reshape(4, 4)  # A[k][r] = a[4k + r]
     # Element (c, r): ((a[r] b[4c] + a[4+r] b[4c+1]) + a[8+r] b[4c+2]) + a[12+r] b[4c+3],
-    # every product and sum rounded to float32, for all 16 elements at once.
-    s = np.multiply.outer(B[:, 0], A[0]) + np.multiply.outer(B[:, 1], A[1])
-    s = s + np.multiply.outer(B[:, 2], A[2])
-    s = s + np.multiply.outer(B[:, 3], A[3])
-    return np.ascontiguousarray(s, dtype=np.float32).reshape(16)
+    # every product and sum rounded to float32; p[c, k, r] = b[4c+k] a[4k+r].
+    p = B[:, :, None] * A
+    s = p[:, 0] + p[:, 1]
+    s += p[:, 2]
+    s += p[:, 3]
+    return s.reshape(16)
 
 
 def identity_files(n: int = 1) -> np.ndarray:
@@ -290,15 +296,29 @@ class ComputeRasteriserConfiguration:
     motionBlurMaxSpread: float = 64.0
 
     def to_c(self) -> N.cr_config:
+        # Spelled out: a render loop converts its configuration every frame.
         c = N.cr_config()
-        for f in fields(self):
-            v = getattr(self, f.name)
-            if f.name == "backgroundColor":
-                c.backgroundColor[:] = [float(x) for x in v]
-            elif isinstance(getattr(c, f.name), float):
-                setattr(c, f.name, float(v))
-            else:
-                setattr(c, f.name, int(v))
+        c.mode = int(self.mode)
+        c.depthTolerance = float(self.depthTolerance)
+        c.backgroundColor[:] = [float(x) for x in self.backgroundColor]
+        c.enableFrustumCulling = int(self.enableFrustumCulling)
+        c.lodBias = int(self.lodBias)
+        c.enableCLOD = int(self.enableCLOD)
+        c.enableLODDither = int(self.enableLODDither)
+        c.holeFillIterations = int(self.holeFillIterations)
+        c.colorizeChunks = int(self.colorizeChunks)
+        c.colorizeOverdraw = int(self.colorizeOverdraw)
+        c.pointSizeMode = int(self.pointSizeMode)
+        c.minimumPointSize = float(self.minimumPointSize)
+        c.maximumPointSize = float(self.maximumPointSize)
+        c.pointSizeScale = float(self.pointSizeScale)
+        c.applyDisplacement = int(self.applyDisplacement)
+        c.applyTint = int(self.applyTint)
+        c.tintAlphaIsCoverage = int(self.tintAlphaIsCoverage)
+        c.writesSceneDepth = int(self.writesSceneDepth)
+        c.motionBlur = float(self.motionBlur)
+        c.motionBlurSamples = int(self.motionBlurSamples)
+        c.motionBlurMaxSpread = float(self.motionBlurMaxSpread)
         return c
 
 
@@ -594,11 +614,10 @@ class ComputeRasteriserPointCloud:
     def updateFiles(self, viewProjection, modelMatrix, frustumTransform=None,
                     prevViewProjection=None):
         """updateFiles (ComputeRasteriserPointCloud.swift:487-515)."""
-        vp, mm = _mat16(viewProjection), _mat16(modelMatrix)
-        fr = None if frustumTransform is None else _mat16(frustumTransform)
-        pv = None if prevViewProjection is None else _mat16(prevViewProjection)
-        N.check(N.lib().cr_cloud_update_files(self._h, N.ptr(vp), N.ptr(mm), N.ptr(fr),
-                                              N.ptr(pv)))
+        vp, mm = _mat16(viewProjection).tobytes(), _mat16(modelMatrix).tobytes()
+        fr = None if frustumTransform is None else _mat16(frustumTransform).tobytes()
+        pv = None if prevViewProjection is None else _mat16(prevViewProjection).tobytes()
+        N.check(N.lib().cr_cloud_update_files(self._h, vp, mm, fr, pv))
 
     # --- read-backs (for tests and tools) ---
     def files(self) -> np.ndarray:
@@ -673,8 +692,9 @@ class PackInput:
         self.c = N.cr_pack_input(pb, prow, cb, crow, fmt)
 
     def _view(self, a):
-        if hasattr(a, "__cuda_array_interface__"):
-            ai = a.__cuda_array_interface__
+        # Asked for once: a torch tensor builds the dict at every access.
+        ai = getattr(a, "__cuda_array_interface__", None)
+        if ai is not None:
             shape = ai["shape"]
             itemsize = np.dtype(ai["typestr"]).itemsize
             if ai.get("strides") not in (None,) and ai["strides"] is not None:
@@ -683,7 +703,7 @@ class PackInput:
                     exp.insert(0, exp[0] * d)
                 if tuple(ai["strides"]) != tuple(exp):
                     raise CRError(1, "device arrays must be C-contiguous")
-            row = itemsize * (int(np.prod(shape[1:])) if len(shape) > 1 else 1)
+            row = itemsize * math.prod(int(d) for d in shape[1:])
             self._keep.append(a)
             return int(ai["data"][0]), True, int(shape[0]) if shape else 0, row
         arr = np.ascontiguousarray(a)
@@ -820,9 +840,8 @@ class PerspectiveCamera:
     # render loop reads them several times per frame).
     @property
     def viewMatrix(self) -> np.ndarray:
-        key = (np.asarray(self.position, np.float64).tobytes(),
-               np.asarray(self.target, np.float64).tobytes(),
-               np.asarray(self.up, np.float64).tobytes())
+        key = b"".join([np.asarray(v, np.float64).tobytes()
+                        for v in (self.position, self.target, self.up)])
         if getattr(self, "_view_key", None) != key:
             self._view = self._compute_view()
             self._view_key = key
@@ -860,10 +879,8 @@ class PerspectiveCamera:
 
 
 def _camera_c(camera) -> N.cr_camera:
-    c = N.cr_camera()
-    C.memmove(c.view, _mat16(camera.viewMatrix).ctypes.data, 64)
-    C.memmove(c.projection, _mat16(camera.projectionMatrix).ctypes.data, 64)
-    return c
+    return N.cr_camera.from_buffer_copy(_mat16(camera.viewMatrix).tobytes() +
+                                        _mat16(camera.projectionMatrix).tobytes())
 
 
 class ComputeRasteriser:

@@ -878,8 +878,7 @@ CR_API cr_status cr_frame_destroy(cr_frame *f) {
     DeviceGuard g(f->ctx->device);
     cudaStreamSynchronize(f->ctx->stream);
     if (f->ev_copied) {
-        cudaEventSynchronize(f->ev_copied);
-        cudaEventDestroy(f->ev_copied);
+        cudaEventSynchronize(f->ev_copied);  // the last of the ring's, destroyed below
     }
     for (cudaEvent_t e : f->ev_copy_ring)
         if (e) cudaEventDestroy(e);
@@ -1116,15 +1115,14 @@ CR_API cr_status cr_frame_read_rgba8_async(cr_frame *f, uint8_t *out) {
     if (!ctx->copy_stream)
         CR_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
     if (!f->ev_rendered) CR_CUDA(cudaEventCreateWithFlags(&f->ev_rendered, cudaEventDisableTiming));
-    if (!f->ev_copied) CR_CUDA(cudaEventCreateWithFlags(&f->ev_copied, cudaEventDisableTiming));
     CR_CUDA(cudaEventRecord(f->ev_rendered, ctx->stream));
     CR_CUDA(cudaStreamWaitEvent(ctx->copy_stream, f->ev_rendered, 0));
     CR_CUDA(cudaMemcpyAsync(out, f->d_rgba[f->final_rgba], (size_t)f->width * f->height * 4,
                             cudaMemcpyDeviceToHost, ctx->copy_stream));
-    CR_CUDA(cudaEventRecord(f->ev_copied, ctx->copy_stream));
     cudaEvent_t &slot = f->ev_copy_ring[f->copies % cr_frame::kCopyRing];
     if (!slot) CR_CUDA(cudaEventCreateWithFlags(&slot, cudaEventDisableTiming));
     CR_CUDA(cudaEventRecord(slot, ctx->copy_stream));
+    f->ev_copied = slot;
     ++f->copies;
     f->copy_pending = true;
     return CR_OK;

@@ -227,8 +227,9 @@ struct cr_frame {
     int final_rgba = 0;                     // which d_rgba holds the final image
     int last_mode = -1;                     // 0 HQS, 1 nearest, -1 none
     // Asynchronous read-back: `rendered` is recorded on the context stream
-    // and waited on by the copy stream; `copied` is recorded after the copy
-    // and waited on by the next write of the RGBA8 planes.
+    // and waited on by the copy stream; `copied` (the ring's latest event) is
+    // recorded after the copy and waited on by the next write of the RGBA8
+    // planes.
     cudaEvent_t ev_rendered = nullptr, ev_copied = nullptr;
     bool copy_pending = false;
     // The last kCopyRing read-backs' completion events (copy n in slot
