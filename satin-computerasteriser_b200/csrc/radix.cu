@@ -66,10 +66,7 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long *p, unsigned lon
 __device__ __forceinline__ bool lookback_ready(unsigned long long v, uint32_t epoch) {
     return (uint32_t)(v >> 48) == epoch && ((v >> 46) & 3ull) != 0ull;
 }
-#ifndef CR_LOOKBACK_BATCH
-#define CR_LOOKBACK_BATCH 8
-#endif
-constexpr int kLookbackBatch = CR_LOOKBACK_BATCH;  // predecessor words one round loads at once
+constexpr int kLookbackBatch = 8;  // predecessor words one round loads at once
 // Per-warp digit counts and bases (at most kTileKeys) in 16 bits: 55.4 KB of
 // shared memory and at most 64 registers let four sort CTAs share an SM.
 using WarpCount = uint16_t;

@@ -40,20 +40,9 @@
 // predicated single instructions rather than branches around code.
 // Integer max and sum are associative and commutative: the planes are
 // bit-identical to a per-point atomic order either way.
-#include "cr_bulk.cuh"
 #include "cr_device.cuh"
 #include "cr_internal.h"
 #include "cr_resolve.cuh"
-
-#ifndef CR_TILE_REJECT
-#define CR_TILE_REJECT 0
-#endif
-#ifndef CR_DIV64
-#define CR_DIV64 0
-#endif
-#ifndef CR_TILE_PX_PER_POINT
-#define CR_TILE_PX_PER_POINT 1
-#endif
 
 namespace {
 
@@ -78,17 +67,10 @@ struct TileCfg<PASS_NEAREST> {
     static constexpr int kBytes = kPx * 8;
 };
 
-// The depth pass that writes fragments keeps two words per tile pixel: the
-// running maximum (seeded with the frame's depth plane) and the plane value
-// it was seeded with, so that the flush writes back only raised pixels.
-#ifndef CR_BULK_STAGE
-#define CR_BULK_STAGE 0
-#endif
 template <>
 struct TileCfg<PASS_DEPTH_FRAG> {
     static constexpr int kPx = 4096;
-    static constexpr int kTileBytes = kPx * (CR_TILE_REJECT ? 8 : 4);
-    static constexpr int kBytes = kTileBytes + (CR_BULK_STAGE ? 2 * 2048 * 9 : 0);  // + stage buffers
+    static constexpr int kBytes = kPx * 4;
 };
 template <>
 struct TileCfg<PASS_COLOR_FRAG> : TileCfg<PASS_COLOR> {};
@@ -133,7 +115,6 @@ struct RasterArgs {
     const uint32_t *chunk_poff;
     unsigned long long frag_cap;
     uint32_t *frag_overflow;
-    uint32_t *status;  // the context's device-side status word
 };
 
 // The frame and camera of the view whose chunk a CTA is drawing (MV kernels).
@@ -237,7 +218,6 @@ struct BatchShared {
 
 struct PointOut {
     bool ok;
-    bool doomed;  // depth pass: the fragment cannot pass the colour pass's depth test
     int ix, iy;  // pixel after the y flip
     uint32_t depth;
     float nz;
@@ -286,12 +266,7 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
     const crd::f4 clip = crd::mulp(sb.T, o.px, o.py, o.pz);
     bool ok = o.ok;
     if (clip.w <= 0.0f) ok = false;
-#if CR_DIV64
-    float nx, ny, nz;
-    crd::div3_shared(clip.x, clip.y, clip.z, clip.w, nx, ny, nz);
-#else
     const float nx = clip.x / clip.w, ny = clip.y / clip.w, nz = clip.z / clip.w;
-#endif
     // |x| > 1 is x < -1 || x > 1 for every float (false for NaN either way).
     if (fabsf(nx) > 1.0f || fabsf(ny) > 1.0f || nz > 1.0f) ok = false;
     if (PASS == PASS_NEAREST ? (nz <= 0.0f) : (nz < 0.0f)) ok = false;
@@ -334,14 +309,6 @@ __device__ __forceinline__ void red_add_u64(unsigned long long *p, unsigned long
 __device__ __forceinline__ void red_max_u32(uint32_t *p, uint32_t v) {
     asm volatile("red.global.max.u32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(v)
                  : "memory");
-}
-__device__ __forceinline__ uint32_t atom_max_u32(uint32_t *p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.global.max.u32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "l"(__cvta_generic_to_global(p)), "r"(v)
-                 : "memory");
-    return old;
 }
 __device__ __forceinline__ void red_max_u64(unsigned long long *p, unsigned long long v) {
     asm volatile("red.global.max.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "l"(v)
@@ -403,17 +370,10 @@ __device__ __forceinline__ void color_global(const RasterArgs &a, const ViewRegs
 
 // Direct path, radius 0: one global atomic per point (batches large on
 // screen, where points rarely share a pixel).
-#ifndef CR_DIRECT_EARLY_REJECT
-#define CR_DIRECT_EARLY_REJECT 0
-#endif
 template <int PASS, bool MV>
 __device__ __forceinline__ void emit_direct(const RasterArgs &a, const ViewRegsT<MV> &vr, PointOut &o) {
     const uint32_t pix = (uint32_t)(o.iy * vw<MV>(vr) + o.ix);
-    if (PASS == PASS_DEPTH_FRAG && CR_DIRECT_EARLY_REJECT) {
-        uint32_t seen = 0u;
-        if (o.ok) seen = atom_max_u32(&vdepth<MV>(vr)[pix], o.depth);
-        o.doomed = o.nz < crd::uint_to_depth(seen) * a.keep_scale;
-    } else if (is_depth(PASS)) {
+    if (is_depth(PASS)) {
         if (o.ok) red_max_u32(&vdepth<MV>(vr)[pix], o.depth);
     } else if (is_color(PASS)) {
         const uint32_t closest = o.ok ? vdepth<MV>(vr)[pix] : 0u;
@@ -438,15 +398,6 @@ __device__ __forceinline__ void emit_direct(const RasterArgs &a, const ViewRegsT
 // Tile path, radius 0: shared-memory accumulation, global atomics for points
 // that round outside the rectangle.  Colour tiles hold R | count << 20, G and
 // B per pixel in 32-bit words (exact while a chunk has at most 4095 points).
-//
-// Depth pass with fragments: the tile starts from the frame's depth plane, so
-// the value a point's shared max returns is a lower bound of the pixel's
-// final depth (depths only grow during the pass).  The colour pass keeps a
-// fragment iff z >= uint_to_depth(final) * (1 - tolerance), which is
-// monotone in the depth word for a positive factor (and true for every
-// fragment when the factor is not positive), so a fragment with
-// z < uint_to_depth(running maximum) * (1 - tolerance) fails it with the
-// final depth too and is not written (o.doomed).
 template <int PASS, bool MV>
 __device__ __forceinline__ void emit_tile(const RasterArgs &a, const ViewRegsT<MV> &vr, const ChunkRec &c,
                                           unsigned char *smem, PointOut &o) {
@@ -455,12 +406,7 @@ __device__ __forceinline__ void emit_tile(const RasterArgs &a, const ViewRegsT<M
     const bool in_tile = o.ok && inside, outside = o.ok && !inside;
     const uint32_t pix = (uint32_t)(o.iy * vw<MV>(vr) + o.ix);
     const int l = inside ? ly * c.tw + lx : 0;
-    if (PASS == PASS_DEPTH_FRAG && CR_TILE_REJECT) {
-        uint32_t seen = 0u;
-        if (in_tile) seen = atomicMax(reinterpret_cast<uint32_t *>(smem) + l, o.depth);
-        if (outside) red_max_u32(&vdepth<MV>(vr)[pix], o.depth);
-        o.doomed = o.nz < crd::uint_to_depth(seen) * a.keep_scale;
-    } else if (is_depth(PASS)) {
+    if (is_depth(PASS)) {
         if (in_tile) atomicMax(reinterpret_cast<uint32_t *>(smem) + l, o.depth);
         if (outside) red_max_u32(&vdepth<MV>(vr)[pix], o.depth);
     } else if (is_color(PASS)) {
@@ -531,7 +477,7 @@ __shared__ uint32_t s_frag_count;
 // one shared-memory atomic per warp, lanes placed by ballot rank.
 __device__ __forceinline__ void emit_fragment(const RasterArgs &a, uint32_t fbase,
                                               const PointOut &o) {
-    const bool keep = o.ok && !o.doomed;
+    const bool keep = o.ok;
     const uint32_t ballot = __ballot_sync(kFull, keep);
     const int lane = threadIdx.x & 31;
     uint32_t base = 0;
@@ -555,9 +501,7 @@ struct Frag {
     float z;
     uint32_t col;
 };
-#ifndef CR_FRAG_BATCH
-#define CR_FRAG_BATCH 2
-#endif
+constexpr int kFragBatch = 2;
 
 // Appends N fragments per lane: one ballot per fragment, one atomic per warp.
 template <int N>
@@ -597,7 +541,6 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
     o.pointIndex = c.first + local;
     o.color = color;
     o.ok = valid;
-    o.doomed = false;
     if (!all_keep) o.ok = o.ok && keep_point(a, c, o.pointIndex, lvl);
     // The depth passes keep nearly every point, so a warp vote to skip the
     // projection or the emission would cost more than it saves (the
@@ -613,7 +556,7 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
         emit_direct<PASS, MV>(a, vr, o);
     if (PASS == PASS_DEPTH_FRAG && emit) {
         if (fo) {
-            fo->keep = o.ok && !o.doomed;
+            fo->keep = o.ok;
             fo->xy = (uint32_t)o.ix | ((uint32_t)o.iy << 16);
             fo->z = o.nz;
             fo->col = o.color;
@@ -630,7 +573,6 @@ __device__ __forceinline__ void do_fragment(const RasterArgs &a, const ViewRegsT
                                             uint32_t xy, float nz, uint32_t color) {
     PointOut o;
     o.ok = valid;
-    o.doomed = false;
     o.ix = (int)(xy & 0xffffu);
     o.iy = (int)(xy >> 16);
     o.nz = nz;
@@ -711,15 +653,7 @@ __device__ __forceinline__ void tile_init(const RasterArgs &a, const ChunkRec &c
                                           unsigned char *smem) {
     const int n = c.tw * c.th;
     for (int l = threadIdx.x; l < n; l += kThreads) {
-        if (PASS == PASS_DEPTH_FRAG && CR_TILE_REJECT) {
-            // Running maximum and seed: the plane's current value (a lower
-            // bound of the final depth; any earlier value of this frame is one).
-            constexpr int kPx = TileCfg<PASS_DEPTH_FRAG>::kPx;
-            const int gx = c.x0 + l % c.tw, gy = c.y0 + l / c.tw;
-            const uint32_t d = view_depth<MV>(a)[gy * view_w<MV>(a) + gx];
-            reinterpret_cast<uint32_t *>(smem)[l] = d;
-            reinterpret_cast<uint32_t *>(smem)[kPx + l] = d;
-        } else if (is_depth(PASS)) {
+        if (is_depth(PASS)) {
             reinterpret_cast<uint32_t *>(smem)[l] = 0u;
         } else if (is_color(PASS)) {
             constexpr int kPx = TileCfg<PASS_COLOR>::kPx;
@@ -741,12 +675,7 @@ __device__ __forceinline__ void tile_flush(const RasterArgs &a, const ViewRegsT<
     const int n = c.tw * c.th;
     for (int l = threadIdx.x; l < n; l += kThreads) {
         const uint32_t pix = (uint32_t)((c.y0 + l / c.tw) * vw<MV>(vr) + c.x0 + l % c.tw);
-        if (PASS == PASS_DEPTH_FRAG && CR_TILE_REJECT) {
-            constexpr int kPx = TileCfg<PASS_DEPTH_FRAG>::kPx;
-            const uint32_t v = reinterpret_cast<const uint32_t *>(smem)[l];
-            if (v > reinterpret_cast<const uint32_t *>(smem)[kPx + l])
-                red_max_u32(&vdepth<MV>(vr)[pix], v);
-        } else if (is_depth(PASS)) {
+        if (is_depth(PASS)) {
             const uint32_t v = reinterpret_cast<const uint32_t *>(smem)[l];
             if (v) red_max_u32(&vdepth<MV>(vr)[pix], v);
         } else if (is_color(PASS)) {
@@ -778,34 +707,6 @@ __device__ __forceinline__ void cp_async_commit() {
 }
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Bulk staging of a chunk's level bytes, coarse words and colours into shared
-// memory (cp.async.bulk completing on an mbarrier; this GPU's memory only,
-// no multicast).  A chunk is staged when its first point is 16-byte aligned
-// in the level array and it has at most kStagePoints points.
-constexpr uint32_t kStagePoints = 2048;
-constexpr uint32_t kStageBytes = kStagePoints * (1 + 4 + 4);
-constexpr uint32_t kStageWaitLimit = 1u << 16;  // polls of an mbarrier before giving up
-__device__ __forceinline__ bool stage_ok(uint32_t first, uint32_t count) {
-    return (first & 15u) == 0u && count <= kStagePoints && count > 0u;
-}
-using crb::bulk_g2s;
-using crb::mbar_expect_tx;
-using crb::mbar_init;
-using crb::mbar_wait;
-// Thread 0: the bulk copies of one chunk's level bytes, coarse words and
-// colours into a stage buffer, completing on `bar`.
-__device__ __forceinline__ void stage_issue(unsigned char *stage, uint64_t *bar,
-                                            const uint8_t *levels, const uint32_t *low,
-                                            const uint32_t *colors, uint32_t first,
-                                            uint32_t count) {
-    const uint32_t nl = (count + 15u) & ~15u, nw = ((count + 3u) & ~3u) * 4u;
-    crb::fence_proxy_async_smem();
-    mbar_expect_tx(bar, nl + 2u * nw);
-    bulk_g2s(stage, levels + first, nl, bar);
-    bulk_g2s(stage + kStagePoints, low + first, nw, bar);
-    bulk_g2s(stage + 5 * kStagePoints, colors + first, nw, bar);
 }
 
 // Largest view v with begin[v] <= k (views without chunks share their
@@ -892,10 +793,6 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
     // and record and prefetches the record while the CTA draws the current
     // one.
     __shared__ uint32_t s_k[2], s_kview[2], s_kslot[2];  // per record buffer
-    constexpr bool kStage = CR_BULK_STAGE && PASS == PASS_DEPTH_FRAG && !MV;
-    __shared__ __align__(8) uint64_t s_mbar[2];
-    unsigned char *stage_base = smem + TileCfg<PASS_DEPTH_FRAG>::kTileBytes;
-    uint32_t stage_phase = 0u;  // per buffer: the parity of its next completion
     auto finish = [&]() {
         if (threadIdx.x == 0) {
             __threadfence();
@@ -929,18 +826,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                        reinterpret_cast<const uint4 *>(a.chunks + slot) + q);
         if (PASS == PASS_COLOR_FRAG) cp_async4(&rec_frags[b][0], a.frag_count + slot);
         if (MV && kFrag) cp_async4(&rec_frags[b][1], a.chunk_poff + slot);
-        if (kStage) {
-            const uint32_t f = __ldg(&a.chunks[slot].first), n = __ldg(&a.chunks[slot].count);
-            if (stage_ok(f, n))
-                stage_issue(stage_base + b * kStageBytes, &s_mbar[b], a.levels, a.low, a.colors,
-                            f, n);
-        }
     };
-    if (kStage && threadIdx.x == 0) {
-        mbar_init(&s_mbar[0], 1u);
-        mbar_init(&s_mbar[1], 1u);
-        crb::mbar_init_fence();
-    }
     if (threadIdx.x == 0) {
         claim(0);
         sb.file = 0xffffffffu;
@@ -967,7 +853,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         const uint32_t work = PASS == PASS_COLOR_FRAG ? nfrag : c.count;
         const bool tiled = a.use_tiles && a.radius_zero && c.tw > 0 &&
                            c.tw * c.th <= TileCfg<PASS>::kPx &&
-                           c.tw * c.th <= CR_TILE_PX_PER_POINT * (int)work &&
+                           c.tw * c.th <= (int)work &&
                            (!is_color(PASS) || c.count < 4096u);
         if (new_file || tiled) {
             __syncthreads();  // everyone has read sb.file (and the view state)
@@ -1046,18 +932,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 }
             }
         } else if ((c.first & 3u) == 0u) {
-            // Four points per thread, 16-byte loads (from the bulk-staged
-            // copy in shared memory when the chunk was staged).
-            bool staged = false;
-            const unsigned char *stg = stage_base + buf * kStageBytes;
-            if (kStage && stage_ok(c.first, c.count)) {
-                staged = mbar_wait(&s_mbar[buf], (stage_phase >> buf) & 1u, kStageWaitLimit);
-                if (!staged) {  // give up: record it, wait once more, read global memory
-                    if (a.status) *(volatile uint32_t *)a.status = kErrStageWait;
-                    mbar_wait(&s_mbar[buf], (stage_phase >> buf) & 1u, kStageWaitLimit);
-                }
-                stage_phase ^= 1u << buf;
-            }
+            // Four points per thread, 16-byte loads.
             const uint32_t nquads = (c.count + 3u) >> 2;
             for (uint32_t q0 = 0; q0 < nquads; q0 += kThreads) {
                 const uint32_t q = q0 + threadIdx.x;
@@ -1065,13 +940,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 const uint32_t base = c.first + 4u * q;
                 uint32_t lv4 = 0;
                 uint4 lo4 = make_uint4(0, 0, 0, 0), me4 = lo4, hi4 = lo4, co4 = lo4;
-                if (qv && staged) {
-                    lv4 = reinterpret_cast<const uint32_t *>(stg)[q];
-                    lo4 = reinterpret_cast<const uint4 *>(stg + kStagePoints)[q];
-                    co4 = reinterpret_cast<const uint4 *>(stg + 5 * kStagePoints)[q];
-                    if (need_med) me4 = __ldg(reinterpret_cast<const uint4 *>(a.med + base));
-                    if (need_high) hi4 = __ldg(reinterpret_cast<const uint4 *>(a.high + base));
-                } else if (qv) {
+                if (qv) {
                     lv4 = __ldg(reinterpret_cast<const uint32_t *>(a.levels + base));
                     lo4 = __ldg(reinterpret_cast<const uint4 *>(a.low + base));
                     if (need_med) me4 = __ldg(reinterpret_cast<const uint4 *>(a.med + base));
@@ -1080,11 +949,11 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                         co4 = __ldg(reinterpret_cast<const uint4 *>(a.colors + base));
                 }
                 const uint32_t l0 = 4u * q;
-                if (CR_FRAG_BATCH > 1 && PASS == PASS_DEPTH_FRAG && !MV && emit) {
-                    // The fragments of CR_FRAG_BATCH points per atomic (one
+                if (PASS == PASS_DEPTH_FRAG && !MV && emit) {
+                    // The fragments of kFragBatch points per atomic (one
                     // view: the batched-view kernel has no registers to
                     // spare for them).
-                    constexpr int kB = CR_FRAG_BATCH > 1 ? CR_FRAG_BATCH : 1;
+                    constexpr int kB = kFragBatch;
                     Frag f[kB];
                     const uint32_t lvs[4] = {lv4 & 0xffu, (lv4 >> 8) & 0xffu, (lv4 >> 16) & 0xffu,
                                              lv4 >> 24};
@@ -1165,46 +1034,25 @@ __device__ __forceinline__ uint32_t hash_slot(uint32_t xy) {
     return ((xy & 0xffffu) + 37u * (xy >> 16)) & (kHashSlots - 1u);
 }
 
-#ifndef CR_HASH3
-#define CR_HASH3 0
-#endif
-// Packed table rows: R | count << 20, G, B — exact while the chunk has fewer
-// than 4096 fragments (a count below 2^12, a red sum below 255 * 4096 < 2^20).
-__device__ __forceinline__ bool hash_packed(uint32_t nfrag) { return CR_HASH3 && nfrag < 4096u; }
-
 template <bool MV>
-__device__ __forceinline__ void hash_add_sums(uint32_t *hkey, uint32_t *hsum, const RasterArgs &a,
-                                              const ViewRegsT<MV> &vr, uint32_t pix, uint32_t xy,
-                                              uint32_t r, uint32_t g, uint32_t b, uint32_t n,
-                                              bool p3 = false) {
+__device__ __forceinline__ void hash_add(uint32_t *hkey, uint32_t *hsum, const RasterArgs &a,
+                                         const ViewRegsT<MV> &vr, uint32_t pix, uint32_t xy,
+                                         uint32_t col) {
+    const uint32_t r = col & 0xffu, g = (col >> 8) & 0xffu, b = (col >> 16) & 0xffu;
     uint32_t h = hash_slot(xy);
     for (int probe = 0; probe < kHashProbes; ++probe) {
         uint32_t cur = hkey[h];
         if (cur == kHashEmpty) cur = atomicCAS(hkey + h, kHashEmpty, pix);
         if (cur == kHashEmpty || cur == pix) {
-            if (p3) {
-                atomicAdd(hsum + h, r | (n << 20));
-                atomicAdd(hsum + kHashSlots + h, g);
-                atomicAdd(hsum + 2 * kHashSlots + h, b);
-            } else {
-                atomicAdd(hsum + h, r);
-                atomicAdd(hsum + kHashSlots + h, g);
-                atomicAdd(hsum + 2 * kHashSlots + h, b);
-                atomicAdd(hsum + 3 * kHashSlots + h, n);
-            }
+            atomicAdd(hsum + h, r);
+            atomicAdd(hsum + kHashSlots + h, g);
+            atomicAdd(hsum + 2 * kHashSlots + h, b);
+            atomicAdd(hsum + 3 * kHashSlots + h, 1u);
             return;
         }
         h = (h + 1u) & (kHashSlots - 1u);
     }
-    color_global<MV>(a, vr, pix, r, g, b, n);
-}
-
-template <bool MV>
-__device__ __forceinline__ void hash_add(uint32_t *hkey, uint32_t *hsum, const RasterArgs &a,
-                                         const ViewRegsT<MV> &vr, uint32_t pix, uint32_t xy,
-                                         uint32_t col, bool p3) {
-    hash_add_sums<MV>(hkey, hsum, a, vr, pix, xy, col & 0xffu, (col >> 8) & 0xffu,
-                      (col >> 16) & 0xffu, 1u, p3);
+    color_global<MV>(a, vr, pix, r, g, b, 1u);
 }
 
 // Clears the table (at kernel start).
@@ -1221,7 +1069,6 @@ template <bool MV>
 __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<MV> &vr,
                                            uint32_t *hkey, uint32_t *hsum, uint32_t n,
                                            uint32_t base, int W, const uint32_t *depth) {
-    const bool p3 = hash_packed(n);
     if ((base & 3u) == 0u) {
         for (uint32_t f = 4u * threadIdx.x; f < n; f += 4u * kThreads) {
             const uint4 xy = __ldcs(reinterpret_cast<const uint4 *>(a.frag_xy + base + f));
@@ -1240,7 +1087,7 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (cl[q] != 0u && zs[q] >= crd::uint_to_depth(cl[q]) * a.keep_scale)
-                    hash_add<MV>(hkey, hsum, a, vr, pix[q], xs[q], cs[q], p3);
+                    hash_add<MV>(hkey, hsum, a, vr, pix[q], xs[q], cs[q]);
         }
     } else {
         for (uint32_t f = threadIdx.x; f < n; f += kThreads) {
@@ -1249,7 +1096,7 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
             const uint32_t cl = __ldg(depth + pix);
             const uint2 zc = a.frag_zc[base + f];
             if (cl != 0u && __uint_as_float(zc.x) >= crd::uint_to_depth(cl) * a.keep_scale)
-                hash_add<MV>(hkey, hsum, a, vr, pix, xy, zc.y, p3);
+                hash_add<MV>(hkey, hsum, a, vr, pix, xy, zc.y);
         }
     }
 }
@@ -1260,16 +1107,15 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
 // completes the sums (and after every thread has read the current claim).
 template <bool MV>
 __device__ __forceinline__ void hash_flush(const RasterArgs &a, const ViewRegsT<MV> &vr,
-                                           uint32_t *hkey, uint32_t *hsum, bool p3,
+                                           uint32_t *hkey, uint32_t *hsum,
                                            uint32_t *cursor = nullptr, uint32_t *next = nullptr) {
     uint32_t claimed = 0u;
     if (cursor && threadIdx.x == 0) claimed = atomicAdd(cursor, 1u);
     for (uint32_t i = threadIdx.x; i < kHashSlots; i += kThreads) {
         const uint32_t pix = hkey[i];
         if (pix == kHashEmpty) continue;
-        const uint32_t w0 = hsum[i];
-        color_global<MV>(a, vr, pix, p3 ? (w0 & 0xfffffu) : w0, hsum[kHashSlots + i],
-                         hsum[2 * kHashSlots + i], p3 ? (w0 >> 20) : hsum[3 * kHashSlots + i]);
+        color_global<MV>(a, vr, pix, hsum[i], hsum[kHashSlots + i], hsum[2 * kHashSlots + i],
+                         hsum[3 * kHashSlots + i]);
         hkey[i] = kHashEmpty;
         hsum[i] = hsum[kHashSlots + i] = hsum[2 * kHashSlots + i] = hsum[3 * kHashSlots + i] = 0u;
     }
@@ -1285,7 +1131,7 @@ __device__ __forceinline__ void hash_chunk(const RasterArgs &a, const ViewRegsT<
     const uint32_t nfrag = __ldg(a.frag_count + k);
     hash_frags<false>(a, vr, hkey, hsum, nfrag, __ldg(&a.chunks[k].first), a.u.width, a.t.depth);
     __syncthreads();  // the chunk's sums are complete (and k has been read by all)
-    hash_flush<false>(a, vr, hkey, hsum, hash_packed(nfrag), cursor, next);
+    hash_flush<false>(a, vr, hkey, hsum, cursor, next);
 }
 
 // 1024 slots (about three times a chunk's typical distinct visible pixels)
@@ -1382,7 +1228,7 @@ __global__ void __launch_bounds__(kThreads, 6)
                          (uint32_t)(s_pbegin[view] + __ldg(a.chunk_poff + slot)), vd.width,
                          vd.depth);
         __syncthreads();  // the chunk's sums are complete (and k has been read by all)
-        hash_flush<true>(a, vr, hkey, hsum, hash_packed(nfrag), cursor, &s_k);
+        hash_flush<true>(a, vr, hkey, hsum, cursor, &s_k);
         __syncthreads();  // the next claim and the cleared table
     }
     if (threadIdx.x == 0) {
@@ -1455,11 +1301,8 @@ __global__ void __launch_bounds__(kThreads) raster_kernel(const __grid_constant_
 
 // The one-view depth passes fit 64 registers without spilling, so four CTAs
 // (and their 32 KB screen tiles) share an SM.
-#ifndef CR_DEPTH_MIN_BLOCKS
-#define CR_DEPTH_MIN_BLOCKS 4
-#endif
 template <int PASS>
-__global__ void __launch_bounds__(kThreads, CR_DEPTH_MIN_BLOCKS) depth_kernel(const __grid_constant__ RasterArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) depth_kernel(const __grid_constant__ RasterArgs a) {
     raster_body<PASS, false>(a);
 }
 
@@ -1574,7 +1417,6 @@ RasterArgs make_args(cr_cloud *cloud, const RasterUniforms &u, const RasterTarge
     a.fcolors = nullptr;
     a.dldimg = nullptr;
     a.fgrad = nullptr;
-    a.status = cloud->ctx->d_status;
     return a;
 }
 
