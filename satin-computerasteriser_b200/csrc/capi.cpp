@@ -289,9 +289,8 @@ cr_status validate_render(cr_context *ctx, cr_frame *frame, const cr_config *cfg
 cr_status nearest_index_pass(cr_context *ctx, cr_frame *f, cr_cloud *cloud, const cr_config *cfg,
                              const cr_camera *cam) {
     cudaStream_t s = ctx->stream;
-    const size_t npix = (size_t)f->width * f->height;
-    CR_CUDA(cudaMemsetAsync(f->d_nearest, 0, npix * sizeof(unsigned long long), s));
-    cr_status st = launch_cull(cloud, make_cull_uniforms(cfg, cam, f->width, f->height), s);
+    const FrameClear fc = nearest_clear_of(f);
+    cr_status st = launch_cull(cloud, make_cull_uniforms(cfg, cam, f->width, f->height), s, &fc);
     if (st) return st;
     RasterTargets t{f->d_depth, f->d_accum, f->d_nearest};
     return launch_raster(cloud, PASS_NEAREST, make_raster_uniforms(cfg, cam, f->width, f->height),
@@ -992,12 +991,17 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         if (stages & CR_STAGE_RESOLVE) {
             PassTimer pt(ctx, CR_PASS_RESOLVE);
             if ((st = frame_copy_fence(f, s))) return st;
+            // With single-pixel footprints a pixel holds at most a sample per
+            // resident point: up to kPackedMaxCount points no field can
+            // carry, and there is nothing to check or to run again (a launch
+            // of 3 us otherwise).
+            const bool check = packed && !(frags && max_samples <= kPackedMaxCount);
             if (coverage) {
                 if ((st = launch_resolve_coverage(f, ru, s))) return st;
-            } else if ((st = launch_resolve_hqs(f, ru, s, packed, nullptr))) {
+            } else if ((st = launch_resolve_hqs(f, ru, s, check, nullptr))) {
                 return st;
             }
-            if (packed) {
+            if (check) {
                 // Exact re-run, which returns at once unless the resolve set
                 // the redo flag: zero the accumulators, colour pass with one
                 // 32-bit add per field, resolve.
@@ -1027,12 +1031,11 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
             if (clouds[i]->resident > 0) first = clouds[i];
         if (first) {
             {
-                PassTimer pt(ctx, CR_PASS_CLEAR);
-                CR_CUDA(cudaMemsetAsync(f->d_nearest, 0, npix * sizeof(unsigned long long), s));
-            }
-            {
+                // The key plane is zeroed by extra CTAs of the cull's launch.
                 PassTimer pt(ctx, CR_PASS_CULL);
-                if ((st = launch_cull(first, make_cull_uniforms(cfg, cam, W, H), s))) return st;
+                const FrameClear fc = nearest_clear_of(f);
+                if ((st = launch_cull(first, make_cull_uniforms(cfg, cam, W, H), s, &fc)))
+                    return st;
             }
             {
                 PassTimer pt(ctx, CR_PASS_DEPTH);

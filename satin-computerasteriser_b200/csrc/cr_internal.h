@@ -341,6 +341,7 @@ struct FrameClear {
     size_t naccum;
 };
 FrameClear frame_clear_of(cr_frame *f);
+FrameClear nearest_clear_of(cr_frame *f);  // the nearest key plane instead
 
 // clear: also zero that frame in the same launch (CTAs after the cull's).
 cr_status launch_cull(cr_cloud *cloud, const CullUniforms &u, cudaStream_t s,

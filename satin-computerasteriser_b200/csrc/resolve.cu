@@ -55,24 +55,43 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// Four pixels per thread, a grid-stride apart: the four keys are read before
+// the winners' colours (a gather over the pool), and those before any pixel
+// is written, so a thread waits for two round trips per four pixels.
 __global__ void __launch_bounds__(kThreads)
     resolve_nearest(const unsigned long long *__restrict__ keys,
                     const uint32_t *__restrict__ colors, uint32_t *__restrict__ rgba,
                     float *__restrict__ depthf, uint32_t npix, ResolveUniforms u) {
-    const uint32_t p = blockIdx.x * kThreads + threadIdx.x;
-    if (p >= npix) return;
-    const unsigned long long k = keys[p];
-    const uint32_t d = (uint32_t)(k >> 32);
-    const uint32_t idx = ~(uint32_t)k;
-    if (d == 0u || idx == 0xffffffffu) {
-        rgba[p] = pack_rgba(u.background[0], u.background[1], u.background[2], 0.0f);
-        depthf[p] = 0.0f;
-        return;
+    crd::grid_wait();
+    crd::launch_dependents();
+    const uint32_t stride = gridDim.x * kThreads;
+    const uint32_t back = pack_rgba(u.background[0], u.background[1], u.background[2], 0.0f);
+    for (uint32_t p0 = blockIdx.x * kThreads + threadIdx.x; p0 < npix; p0 += 4u * stride) {
+        unsigned long long k[4];
+        uint32_t c[4];
+        bool hit[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t p = p0 + (uint32_t)j * stride;
+            k[j] = p < npix ? keys[p] : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t idx = ~(uint32_t)k[j];
+            hit[j] = (uint32_t)(k[j] >> 32) != 0u && idx != 0xffffffffu;
+            c[j] = hit[j] ? colors[idx] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t p = p0 + (uint32_t)j * stride;
+            if (p >= npix) break;
+            rgba[p] = hit[j] ? pack_rgba((float)(c[j] & 0xffu) / 255.0f,
+                                         (float)((c[j] >> 8) & 0xffu) / 255.0f,
+                                         (float)((c[j] >> 16) & 0xffu) / 255.0f, 1.0f)
+                             : back;
+            depthf[p] = hit[j] ? crd::uint_to_depth((uint32_t)(k[j] >> 32)) : 0.0f;
+        }
     }
-    const uint32_t c = colors[idx];
-    rgba[p] = pack_rgba((float)(c & 0xffu) / 255.0f, (float)((c >> 8) & 0xffu) / 255.0f,
-                        (float)((c >> 16) & 0xffu) / 255.0f, 1.0f);
-    depthf[p] = crd::uint_to_depth(d);
 }
 
 __device__ __forceinline__ float unorm_ch(uint32_t v, int ch) {
@@ -331,6 +350,13 @@ FrameClear frame_clear_of(cr_frame *f) {
                       (uint32_t)(npix - 4 * n4), f->d_accum, npix + 1};
 }
 
+FrameClear nearest_clear_of(cr_frame *f) {
+    // The key plane as 16-byte words; an odd number of keys leaves two words.
+    const size_t npix = (size_t)f->width * (size_t)f->height;
+    return FrameClear{nullptr, 0, reinterpret_cast<uint32_t *>(f->d_nearest + (npix & ~(size_t)1)),
+                      (uint32_t)(npix & 1) * 2u, reinterpret_cast<uint4 *>(f->d_nearest), npix / 2};
+}
+
 cr_status launch_frame_clear(cr_frame *f, cudaStream_t s) {
     const FrameClear c = frame_clear_of(f);
     frame_clear<<<f->ctx->sm_count * 8, kThreads, 0, s>>>(c.depth4, c.ndepth4, c.tail, c.ntail,
@@ -349,8 +375,11 @@ cr_status launch_accum_redo_clear(cr_frame *f, cudaStream_t s) {
 cr_status launch_resolve_nearest(cr_frame *f, const uint32_t *colors, const ResolveUniforms &u,
                                  cudaStream_t s) {
     const uint32_t npix = (uint32_t)f->width * (uint32_t)f->height;
-    resolve_nearest<<<(npix + kThreads - 1) / kThreads, kThreads, 0, s>>>(
-        f->d_nearest, colors, f->d_rgba[0], f->d_depthf, npix, u);
+    const uint32_t full = (npix + 4 * kThreads - 1) / (4 * kThreads);
+    CR_CUDA(launch_programmatic(resolve_nearest,
+                                dim3(std::min(full, (uint32_t)f->ctx->sm_count * 16)),
+                                dim3(kThreads), 0, s, (const unsigned long long *)f->d_nearest,
+                                colors, f->d_rgba[0], f->d_depthf, npix, u));
     CR_CUDA(cudaGetLastError());
     f->final_rgba = 0;
     return CR_OK;
