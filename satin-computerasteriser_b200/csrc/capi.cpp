@@ -950,7 +950,7 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
             const bool clear_in_cull = !resident.empty() && resident[0]->cap.maxResidentBatches > 0;
             if (!clear_in_cull) {
                 PassTimer pt(ctx, CR_PASS_CLEAR);
-                if ((st = launch_frame_clear(f, s))) return st;
+                if ((st = launch_frame_clear(frame_clear_of(f), ctx->sm_count, s))) return st;
             }
             const CullUniforms cu = make_cull_uniforms(cfg, cam, W, H);
             {
@@ -1235,21 +1235,22 @@ CR_API cr_status cr_hqs_forward_f32(cr_context *ctx, cr_frame *f, cr_cloud *clou
     const size_t npix = (size_t)f->width * f->height;
     if (!f->d_fsum) {
         if ((st = dalloc(&f->d_fsum, npix * sizeof(float4))) ||
-            (st = dalloc(&f->d_fcount, npix * 4)))
+            (st = dalloc(&f->d_fcount, (npix + 3) / 4 * 16)))
             return st;
     }
-    CR_CUDA(cudaMemsetAsync(f->d_depth, 0, npix * 4, s));
-    CR_CUDA(cudaMemsetAsync(f->d_fsum, 0, npix * sizeof(float4), s));
-    CR_CUDA(cudaMemsetAsync(f->d_fcount, 0, npix * 4, s));
+    // The planes are zeroed by extra CTAs of the cull's launch.
+    const FrameClear fc = f32_clear_of(f);
     if (cloud->resident > 0) {
         const RasterUniforms rau = make_raster_uniforms(cfg, cam, f->width, f->height);
         RasterTargets t{f->d_depth, f->d_accum, f->d_nearest};
         t.fsum = f->d_fsum;
         t.fcount = f->d_fcount;
-        if ((st = launch_cull(cloud, make_cull_uniforms(cfg, cam, f->width, f->height), s)) ||
-            (st = launch_raster(cloud, PASS_DEPTH, rau, t, s)) ||
+        if ((st = launch_cull(cloud, make_cull_uniforms(cfg, cam, f->width, f->height), s, &fc)) ||
+            (st = launch_raster_f32(cloud, PASS_DEPTH, rau, t, nullptr, nullptr, nullptr, s)) ||
             (st = launch_raster_f32(cloud, PASS_COLOR_F32, rau, t, colors, nullptr, nullptr, s)))
             return st;
+    } else if ((st = launch_frame_clear(fc, ctx->sm_count, s))) {
+        return st;
     }
     const float bg[3] = {cfg->backgroundColor[0], cfg->backgroundColor[1],
                          cfg->backgroundColor[2]};

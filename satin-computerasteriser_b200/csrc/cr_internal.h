@@ -193,6 +193,7 @@ struct cr_cloud {
     uint32_t *d_cull_cta = nullptr;          // per-CTA survivor and chunk counts
     ChunkRec *d_chunks = nullptr;            // chunk work records
     uint64_t chunk_cap = 0;                  // capacity of d_chunks
+    uint32_t cull_chunk_points = 0;          // most points of a record of the last cull
 
     // Fragments of the last depth pass, in pool point index space: a chunk
     // starting at point p keeps its n kept points compacted at [p, p + n).
@@ -223,7 +224,7 @@ struct cr_frame {
     uint32_t *d_rgba[2] = {nullptr, nullptr}; // RGBA8 ping-pong (resolve, hole fill)
     float *d_depthf = nullptr;              // resolve R32F depth
     float4 *d_fsum = nullptr;               // differentiable colours: FP32 R, G, B sums (lazy)
-    uint32_t *d_fcount = nullptr;           //   and their sample counts
+    uint32_t *d_fcount = nullptr;           //   and their sample counts (whole 16-byte groups)
     int final_rgba = 0;                     // which d_rgba holds the final image
     int last_mode = -1;                     // 0 HQS, 1 nearest, -1 none
     // Asynchronous read-back: `rendered` is recorded on the context stream
@@ -330,8 +331,9 @@ InlineFiles inline_files(const cr_cloud *c);
 // Copies frame_files to d_files if a camera update left it only on the host.
 cr_status ensure_device_files(cr_cloud *c);
 
-// Zeroing of an HQS frame's depth plane (whole 16-byte groups, then a tail
-// of up to three words) and accumulators with the redo word behind them.
+// Zeroing of a frame's planes: a plane of words (whole 16-byte groups, then a
+// tail of up to three words) and two of 16-byte groups.  An HQS frame: the
+// depth plane, and the accumulators with the redo word behind them.
 struct FrameClear {
     uint4 *depth4;
     size_t ndepth4;
@@ -339,9 +341,12 @@ struct FrameClear {
     uint32_t ntail;
     uint4 *accum;
     size_t naccum;
+    uint4 *more;
+    size_t nmore;
 };
 FrameClear frame_clear_of(cr_frame *f);
 FrameClear nearest_clear_of(cr_frame *f);  // the nearest key plane instead
+FrameClear f32_clear_of(cr_frame *f);      // depth plane, FP32 sums, sample counts
 
 // clear: also zero that frame in the same launch (CTAs after the cull's).
 cr_status launch_cull(cr_cloud *cloud, const CullUniforms &u, cudaStream_t s,
@@ -400,8 +405,9 @@ constexpr uint32_t kPackedMaxCount = 16843009u;
 
 cr_status launch_raster(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
                         const RasterTargets &t, cudaStream_t s);
-// PASS_COLOR_F32 (colors: 3 floats per pool point) or PASS_GRAD (dldimg: 3
-// floats per pixel, grad: 3 floats per pool point, added to) of one cloud.
+// The differentiable passes of one cloud: PASS_DEPTH, PASS_COLOR_F32 (colors: 3
+// floats per pool point) or PASS_GRAD (dldimg: 3 floats per pixel, grad: 3
+// floats per pool point, added to).
 cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
                             const RasterTargets &t, const float *colors, const float *dldimg,
                             float *grad, cudaStream_t s);
@@ -480,8 +486,9 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
                           const RasterUniforms &u, const RasterTargets &t,
                           const ResolveUniforms &ru, cudaStream_t s);
 uint32_t hqs_redo_max_clouds();
-// Zeroes the depth plane, the accumulators and the redo word of an HQS frame.
-cr_status launch_frame_clear(cr_frame *f, cudaStream_t s);
+// Zeroes a frame's planes in a launch of its own (launch_cull does it in the
+// cull's).
+cr_status launch_frame_clear(const FrameClear &c, int sm_count, cudaStream_t s);
 // Coverage resolve (weighted-blended accumulation) into d_rgba[0].
 cr_status launch_resolve_coverage(cr_frame *f, const ResolveUniforms &u, cudaStream_t s);
 

@@ -333,6 +333,7 @@ __global__ void __launch_bounds__(kCullThreads)
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
         for (size_t i = t0; i < clear.naccum; i += stride) clear.accum[i] = z;
         for (size_t i = t0; i < clear.ndepth4; i += stride) clear.depth4[i] = z;
+        for (size_t i = t0; i < clear.nmore; i += stride) clear.more[i] = z;
         if (t0 < clear.ntail) clear.tail[t0] = 0u;
         return;
     }
@@ -560,6 +561,7 @@ cr_status launch_cull(cr_cloud *cloud, const CullUniforms &u, cudaStream_t s,
     }
     const uint32_t cp = (uint32_t)std::max(cloud->ctx->chunk_points, kMinChunkPoints);
     const uint32_t ctas = (n + kCullThreads - 1) / kCullThreads;
+    cloud->cull_chunk_points = cp;
     CullArgs a{cloud->d_batches,  n,
                cloud->d_files,    (uint32_t)cloud->files.size(),
                cloud->d_cull_tmp, cloud->d_cull_cta,

@@ -40,6 +40,8 @@
 // predicated single instructions rather than branches around code.
 // Integer max and sum are associative and commutative: the planes are
 // bit-identical to a per-point atomic order either way.
+#include <algorithm>
+
 #include "cr_device.cuh"
 #include "cr_internal.h"
 #include "cr_resolve.cuh"
@@ -237,7 +239,7 @@ __device__ __forceinline__ bool keep_point(const RasterArgs &a, const ChunkRec &
 // decodePoint + projection + clip + pixel (DepthPass/Shaders.metal:188-211,
 // ColorPass/Shaders.metal:70-104, NearestDepth/Shaders.metal:68-85).
 template <int PASS, bool MV>
-__device__ __forceinline__ void project_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const BatchShared &sb,
+__device__ __forceinline__ void project_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const float *T,
                                               const ChunkRec &c, uint32_t lo, uint32_t me,
                                               uint32_t hi, PointOut &o) {
     // Split-precision decode: the coarse (low), medium and fine (high) 10-bit
@@ -263,7 +265,7 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
     o.px = (float)x * c.qx + c.minX;
     o.py = (float)y * c.qy + c.minY;
     o.pz = (float)z * c.qz + c.minZ;
-    const crd::f4 clip = crd::mulp(sb.T, o.px, o.py, o.pz);
+    const crd::f4 clip = crd::mulp(T, o.px, o.py, o.pz);
     bool ok = o.ok;
     if (clip.w <= 0.0f) ok = false;
     const float nx = clip.x / clip.w, ny = clip.y / clip.w, nz = clip.z / clip.w;
@@ -546,7 +548,7 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
     // projection or the emission would cost more than it saves (the
     // emission is correct for a warp with no kept point).
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
-    project_point<PASS, MV>(a, vr, sb, c, lo, me, hi, o);
+    project_point<PASS, MV>(a, vr, sb.T, c, lo, me, hi, o);
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
     if (!a.radius_zero)
         emit_footprint<PASS, MV>(a, vr, sb, o);
@@ -1299,6 +1301,50 @@ __global__ void __launch_bounds__(kThreads) raster_kernel(const __grid_constant_
     raster_body<PASS, MV>(a);
 }
 
+// The differentiable passes of one view with single-pixel footprints (depth
+// plane, FP32 colour sums, adjoint): a thread per point, 256 points of a
+// chunk record to a step, `steps` steps to a record; the grid strides over
+// all of them.  A training view holds a million points or so, of which the
+// four-points-a-thread passes make two rounds in the few hundred chunks that
+// there are: half of the SMs' warps had no work, and each waited for its
+// chain of loads (record, words, depth, colour) alone.  With a step to a CTA
+// the work spreads over every warp slot.  10M points, 512 x 512, a view:
+// depth 25 -> 13 us, colour 38 -> 16 us, adjoint 33 -> 17 us.
+constexpr int kStepPoints = kThreads;
+template <int PASS>
+__global__ void __launch_bounds__(kThreads, 6)
+    point_pass(const __grid_constant__ RasterArgs a, uint32_t steps) {
+    // The inline files' transforms; a larger table is read where it is.
+    __shared__ __align__(16) float sT[kInlineFiles][16];
+    for (uint32_t t = threadIdx.x; t < 16u * a.ifiles.n; t += kThreads)
+        sT[t >> 4][t & 15u] = a.ifiles.f[t >> 4].transform[t & 15u];
+    crd::grid_wait();
+    crd::launch_dependents();
+    __syncthreads();
+    const ViewRegsT<false> vr(a);
+    const uint32_t total = a.counters[CNT_CHUNKS] * steps;
+    for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
+        const uint32_t k = v / steps, local = (v - k * steps) * kStepPoints + threadIdx.x;
+        ChunkRec c;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            reinterpret_cast<uint4 *>(&c)[q] = __ldg(reinterpret_cast<const uint4 *>(a.chunks + k) + q);
+        if (local >= c.count) continue;
+        PointOut o;
+        o.pointIndex = c.first + local;
+        o.color = 0u;
+        o.ok = true;
+        const bool all_keep = (a.u.lodDither ? 1.0f : 0.5f) < (c.thr - 7.0f) + 0.5f;
+        const uint32_t lo = __ldg(a.low + o.pointIndex);
+        const uint32_t me = c.level <= 1 ? __ldg(a.med + o.pointIndex) : 0u;
+        const uint32_t hi = c.level == 0 ? __ldg(a.high + o.pointIndex) : 0u;
+        if (!all_keep) o.ok = keep_point(a, c, o.pointIndex, __ldg(a.levels + o.pointIndex));
+        project_point<PASS, false>(a, vr, a.ifiles.n ? sT[c.file] : a.files[c.file].transform, c,
+                                   lo, me, hi, o);
+        if (o.ok) emit_direct<PASS, false>(a, vr, o);
+    }
+}
+
 // The one-view depth passes fit 64 registers without spilling, so four CTAs
 // (and their 32 KB screen tiles) share an SM.
 template <int PASS>
@@ -1340,6 +1386,15 @@ constexpr auto kernel_for() {
         return depth_views_kernel<PASS>;
     else
         return raster_kernel<PASS, MV>;
+}
+
+template <int PASS>
+int point_pass_blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, point_pass<PASS>, kThreads, 0) !=
+        cudaSuccess)
+        n = 1;
+    return n < 1 ? 1 : n;
 }
 
 template <int PASS, bool MV>
@@ -1476,16 +1531,39 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
 
 uint32_t hqs_redo_max_clouds() { return kRedoMaxClouds; }
 
+// A step to a CTA while there are CTAs.  The chunk records are those of the
+// cloud's last cull, at the chunk size it was launched with.
+template <int PASS>
+cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, uint32_t chunk_points,
+                              cudaStream_t s) {
+    const uint32_t steps = (chunk_points + kStepPoints - 1) / kStepPoints;
+    return launch_programmatic(point_pass<PASS>,
+                               dim3(ctx->sm_count * point_pass_blocks_per_sm<PASS>()),
+                               dim3(kThreads), 0, s, a, steps);
+}
+
 cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
                             const RasterTargets &t, const float *colors, const float *dldimg,
                             float *grad, cudaStream_t s) {
-    if (pass != PASS_COLOR_F32 && pass != PASS_GRAD)
+    if (pass != PASS_DEPTH && pass != PASS_COLOR_F32 && pass != PASS_GRAD)
         return cri::fail(CR_ERR_INTERNAL, "launch_raster_f32: pass");
     RasterArgs a = make_args(cloud, u, t);
+    if (!a.ifiles.n) {
+        const cr_status st = ensure_device_files(cloud);
+        if (st) return st;
+    }
     a.fcolors = colors;
     a.dldimg = dldimg;
     a.fgrad = grad;
     cr_context *ctx = cloud->ctx;
+    if (a.radius_zero) {
+        const uint32_t cp = cloud->cull_chunk_points;
+        CR_CUDA(pass == PASS_DEPTH       ? launch_point_pass<PASS_DEPTH>(a, ctx, cp, s)
+                : pass == PASS_COLOR_F32 ? launch_point_pass<PASS_COLOR_F32>(a, ctx, cp, s)
+                                         : launch_point_pass<PASS_GRAD>(a, ctx, cp, s));
+        return CR_OK;
+    }
+    if (pass == PASS_DEPTH) return launch_raster(cloud, pass, u, t, s);
     if (ctx->blocks_per_sm[pass] == 0)
         ctx->blocks_per_sm[pass] = pass == PASS_COLOR_F32
                                        ? blocks_per_sm_for<PASS_COLOR_F32, false>()

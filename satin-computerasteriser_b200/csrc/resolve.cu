@@ -225,6 +225,8 @@ __global__ void __launch_bounds__(kThreads)
 __global__ void __launch_bounds__(kThreads)
     resolve_f32(const float4 *__restrict__ fsum, const uint32_t *__restrict__ fcount,
                 float *__restrict__ image, uint32_t npix, float bg0, float bg1, float bg2) {
+    crd::grid_wait();
+    crd::launch_dependents();
     for (uint32_t p = blockIdx.x * kThreads + threadIdx.x; p < npix; p += gridDim.x * kThreads) {
         const uint32_t n = fcount[p];
         float *o = image + 3 * (size_t)p;
@@ -247,6 +249,8 @@ __global__ void __launch_bounds__(kThreads)
 __global__ void __launch_bounds__(kThreads)
     l2_loss(const float *__restrict__ image, const float *__restrict__ target, uint64_t n,
             float scale, float *__restrict__ dldimg, double *loss) {
+    crd::grid_wait();
+    crd::launch_dependents();
     __shared__ double part[kThreads / 32];
     double acc = 0.0;
     for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
@@ -294,18 +298,15 @@ __global__ void __launch_bounds__(kThreads)
     depthf[p] = crd::uint_to_depth(depth[p]);
 }
 
-// Zeroes the depth plane and the accumulators (with the redo word behind
-// them) of an HQS frame in one launch of 16-byte stores.
-__global__ void __launch_bounds__(kThreads)
-    frame_clear(uint4 *depth4, size_t ndepth4, uint32_t *depth_tail, uint32_t ntail,
-                uint4 *accum, size_t naccum) {
+// Zeroes a frame's planes in one launch of 16-byte stores.
+__global__ void __launch_bounds__(kThreads) frame_clear(const FrameClear c) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < naccum; i += stride)
-        accum[i] = z;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < ndepth4; i += stride)
-        depth4[i] = z;
-    if (blockIdx.x == 0 && threadIdx.x < ntail) depth_tail[threadIdx.x] = 0u;
+    for (size_t i = t0; i < c.naccum; i += stride) c.accum[i] = z;
+    for (size_t i = t0; i < c.ndepth4; i += stride) c.depth4[i] = z;
+    for (size_t i = t0; i < c.nmore; i += stride) c.more[i] = z;
+    if (t0 < c.ntail) c.tail[t0] = 0u;
 }
 
 // Top bit of every depth word flipped: unsigned order <-> signed order.
@@ -347,20 +348,28 @@ FrameClear frame_clear_of(cr_frame *f) {
     const size_t npix = (size_t)f->width * (size_t)f->height;
     const size_t n4 = npix / 4;  // depth words in whole 16-byte groups (the plane is 256-byte aligned)
     return FrameClear{reinterpret_cast<uint4 *>(f->d_depth), n4, f->d_depth + 4 * n4,
-                      (uint32_t)(npix - 4 * n4), f->d_accum, npix + 1};
+                      (uint32_t)(npix - 4 * n4), f->d_accum, npix + 1, nullptr, 0};
+}
+
+FrameClear f32_clear_of(cr_frame *f) {
+    FrameClear c = frame_clear_of(f);
+    const size_t npix = (size_t)f->width * (size_t)f->height;
+    c.accum = reinterpret_cast<uint4 *>(f->d_fsum);
+    c.naccum = npix;
+    c.more = reinterpret_cast<uint4 *>(f->d_fcount);  // allocated in whole groups
+    c.nmore = (npix + 3) / 4;
+    return c;
 }
 
 FrameClear nearest_clear_of(cr_frame *f) {
     // The key plane as 16-byte words; an odd number of keys leaves two words.
     const size_t npix = (size_t)f->width * (size_t)f->height;
     return FrameClear{nullptr, 0, reinterpret_cast<uint32_t *>(f->d_nearest + (npix & ~(size_t)1)),
-                      (uint32_t)(npix & 1) * 2u, reinterpret_cast<uint4 *>(f->d_nearest), npix / 2};
+                      (uint32_t)(npix & 1) * 2u, reinterpret_cast<uint4 *>(f->d_nearest), npix / 2, nullptr, 0};
 }
 
-cr_status launch_frame_clear(cr_frame *f, cudaStream_t s) {
-    const FrameClear c = frame_clear_of(f);
-    frame_clear<<<f->ctx->sm_count * 8, kThreads, 0, s>>>(c.depth4, c.ndepth4, c.tail, c.ntail,
-                                                           c.accum, c.naccum);
+cr_status launch_frame_clear(const FrameClear &c, int sm_count, cudaStream_t s) {
+    frame_clear<<<sm_count * 8, kThreads, 0, s>>>(c);
     CR_CUDA(cudaGetLastError());
     return CR_OK;
 }
@@ -451,9 +460,10 @@ cr_status launch_hole_fill_views(const ViewDesc *views, uint32_t nviews, uint32_
 cr_status launch_resolve_f32(cr_frame *f, const float background[3], float *image,
                              cudaStream_t s) {
     const uint32_t npix = (uint32_t)f->width * (uint32_t)f->height;
-    resolve_f32<<<views_grid(npix, f->ctx->sm_count), kThreads, 0, s>>>(
-        f->d_fsum, f->d_fcount, image, npix, background[0], background[1], background[2]);
-    CR_CUDA(cudaGetLastError());
+    CR_CUDA(launch_programmatic(resolve_f32, dim3(views_grid(npix, f->ctx->sm_count)),
+                                dim3(kThreads), 0, s, (const float4 *)f->d_fsum,
+                                (const uint32_t *)f->d_fcount, image, npix, background[0],
+                                background[1], background[2]));
     return CR_OK;
 }
 
@@ -462,8 +472,8 @@ cr_status launch_l2_loss(const float *image, const float *target, uint64_t n, fl
     if (n == 0) return CR_OK;
     const uint64_t need = (n + kThreads - 1) / kThreads;
     const uint32_t grid = (uint32_t)std::min<uint64_t>(need, (uint64_t)sm_count * 8);
-    l2_loss<<<grid, kThreads, 0, s>>>(image, target, n, scale, dldimg, loss);
-    CR_CUDA(cudaGetLastError());
+    CR_CUDA(launch_programmatic(l2_loss, dim3(grid), dim3(kThreads), 0, s, image, target, n, scale,
+                                dldimg, loss));
     return CR_OK;
 }
 

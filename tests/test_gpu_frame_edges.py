@@ -41,3 +41,44 @@ def test_nearest_frames_one_after_the_other(cr, orc, ctx, w, h):
         ras.update(camera(cr, at, w=w, h=h))
         ras.encode()
         assert np.array_equal(ras.nearestIndices(), gpu["ni"])
+
+
+@pytest.mark.parametrize("chunk", [256, 300, 2048])
+@pytest.mark.parametrize("ppb", [255, 256, 257, 10240])
+def test_training_passes_at_step_edges(cr, orc, ctx, chunk, ppb):
+    """The FP32 passes over batches and chunk records around their 256-point
+    steps, with a chunk size set between the forward and the adjoint: the
+    image is the mean of the visible points' colours and the gradient of an
+    image gradient of ones is 1 / count per visible pixel.  Every visible
+    point and pixel comes from the oracle's depth plane and counts; the sums
+    of at most a few hundred FP32 terms in [0, 1] are held to 1e-4."""
+    pos, rgba = blob_cloud(5000, 21)
+    cloud, _ = make_cloud(cr, orc, ctx, pos, rgba, ppb=ppb)
+    n = cloud.capacity.maxResidentPoints
+    w, h = 61, 47
+    cam = camera(cr, (0.2, 0.1, 1.6), w=w, h=h)
+    cfg = cr.ComputeRasteriserConfiguration(enableCLOD=False)
+    before = ctx.tuning()["chunkPoints"]
+    try:
+        ctx.set_tuning(chunkPoints=chunk)
+        ras, gpu, ref = render_both(cr, orc, ctx, [cloud], cfg, cam, w, h)
+        assert_same(cr, cfg, gpu, ref)
+        # Colours (1, 1/2, 0): the covered pixels are exactly that.
+        col = cr.DeviceBuffer(ctx, n * 12, (n, 3), np.float32)
+        col.upload(np.tile(np.array([1.0, 0.5, 0.0], np.float32), (n, 1)))
+        img = cr.DeviceBuffer(ctx, w * h * 12, (h, w, 3), np.float32)
+        ones = cr.DeviceBuffer(ctx, w * h * 12, (h, w, 3), np.float32)
+        ones.upload(np.ones((h, w, 3), np.float32))
+        grad = cr.DeviceBuffer(ctx, n * 12, (n, 3), np.float32)
+        grad.upload(np.zeros((n, 3), np.float32))
+        ras.forwardF32(cloud, col, img)
+        ctx.set_tuning(chunkPoints=4096)
+        ras.backwardColors(cloud, ones, grad)
+        covered = ref.accum[..., 3] > 0
+        want = np.where(covered[..., None], np.array([1.0, 0.5, 0.0], np.float32), 0.0)
+        assert np.abs(img.download() - want).max() <= 1e-4
+        # Every covered pixel hands out 1 in all: the sum of the gradients.
+        total = grad.download().astype(np.float64).sum(0)
+        assert np.abs(total - covered.sum()).max() <= 1e-4 * covered.sum()
+    finally:
+        ctx.set_tuning(chunkPoints=before)
