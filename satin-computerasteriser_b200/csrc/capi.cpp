@@ -935,6 +935,11 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         // instead of decoding and projecting the points again.
         const bool frags =
             !variants && std::fmax(cfg->minimumPointSize, cfg->maximumPointSize) <= 1.0f;
+        // Larger footprints have passes of their own, whose colour pass also
+        // draws fragments; a colour stage on its own decodes the points,
+        // since the depth stage may have run with another configuration.
+        const bool splats = !variants && !frags && (stages & CR_STAGE_DEPTH) &&
+                            (stages & CR_STAGE_COLOR);
         // Packed colour adds while the frame holds fewer than 2^31 samples:
         // then a pixel's count field reads its true count plus at most 127
         // carries out of the blue sum, so a read count of at most
@@ -965,6 +970,7 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
                 PassTimer pt(ctx, CR_PASS_DEPTH);
                 for (cr_cloud *c : resident)
                     if ((st = variants ? launch_variant_pass(c, false, rau, *cfg, t, s)
+                              : splats ? launch_splats(c, false, rau, t, s)
                                        : launch_raster(c, frags ? PASS_DEPTH_FRAG : PASS_DEPTH,
                                                        rau, t, s)))
                         return st;
@@ -974,6 +980,7 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
             PassTimer pt(ctx, CR_PASS_COLOR);
             for (cr_cloud *c : resident)
                 if ((st = variants ? launch_variant_pass(c, true, rau, *cfg, t, s)
+                          : splats ? launch_splats(c, true, rau, t, s)
                                    : launch_raster(c, frags ? PASS_COLOR_FRAG : PASS_COLOR, rau,
                                                    t, s)))
                     return st;
@@ -991,11 +998,10 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         if (stages & CR_STAGE_RESOLVE) {
             PassTimer pt(ctx, CR_PASS_RESOLVE);
             if ((st = frame_copy_fence(f, s))) return st;
-            // With single-pixel footprints a pixel holds at most a sample per
-            // resident point: up to kPackedMaxCount points no field can
-            // carry, and there is nothing to check or to run again (a launch
-            // of 3 us otherwise).
-            const bool check = packed && !(frags && max_samples <= kPackedMaxCount);
+            // A pixel holds at most a sample per resident point: up to
+            // kPackedMaxCount points no field can carry, and there is nothing
+            // to check or to run again (a launch of 3 us otherwise).
+            const bool check = packed && max_samples > kPackedMaxCount;
             if (coverage) {
                 if ((st = launch_resolve_coverage(f, ru, s))) return st;
             } else if ((st = launch_resolve_hqs(f, ru, s, check, nullptr))) {
@@ -1008,10 +1014,10 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
                 RasterTargets tx = t;
                 tx.packed = 0;
                 tx.redo = f->d_redo;
-                if (frags && resident.size() <= hqs_redo_max_clouds()) {
+                if ((frags || splats) && resident.size() <= hqs_redo_max_clouds()) {
                     // From the fragments: all three steps in one launch.
-                    if ((st = launch_hqs_redo(f, resident.data(), (uint32_t)resident.size(), rau,
-                                              tx, ru, s)))
+                    if ((st = launch_hqs_redo(f, resident.data(), (uint32_t)resident.size(),
+                                              splats, rau, tx, ru, s)))
                         return st;
                 } else {
                     if ((st = launch_accum_redo_clear(f, s))) return st;

@@ -93,6 +93,7 @@ struct cr_context {
     int blocks_per_sm[7] = {};        // occupancy of the persistent point passes (per RasterPass)
     int blocks_per_sm_views[7] = {};  // the same, batched-view kernels
     int blocks_per_sm_hash_views = 0;  // the batched-view colour hash kernel
+    int blocks_per_sm_splat[2] = {};   // the splat depth and colour passes
     int chunk_points = 2048;           // points per chunk work record
     int view_group_pixels = 4194304;   // batched views: pixels per depth/colour group
     bool use_tiles = true;             // shared-memory screen tiles
@@ -405,6 +406,10 @@ constexpr uint32_t kPackedMaxCount = 16843009u;
 
 cr_status launch_raster(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
                         const RasterTargets &t, cudaStream_t s);
+// Depth or colour pass of one cloud and view with footprints of more than a
+// pixel.  The colour pass draws the fragments of the depth pass before it.
+cr_status launch_splats(cr_cloud *cloud, bool color, const RasterUniforms &u,
+                        const RasterTargets &t, cudaStream_t s);
 // The differentiable passes of one cloud: PASS_DEPTH, PASS_COLOR_F32 (colors: 3
 // floats per pool point) or PASS_GRAD (dldimg: 3 floats per pixel, grad: 3
 // floats per pool point, added to).
@@ -483,7 +488,7 @@ cr_status launch_accum_redo_clear(cr_frame *f, cudaStream_t s);
 // of every cloud with 32-bit adds (t.packed = 0), resolve into d_rgba[0].
 // At most hqs_redo_max_clouds() clouds.
 cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds,
-                          const RasterUniforms &u, const RasterTargets &t,
+                          bool splats, const RasterUniforms &u, const RasterTargets &t,
                           const ResolveUniforms &ru, cudaStream_t s);
 uint32_t hqs_redo_max_clouds();
 // Zeroes a frame's planes in a launch of its own (launch_cull does it in the

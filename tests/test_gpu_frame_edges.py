@@ -82,3 +82,66 @@ def test_training_passes_at_step_edges(cr, orc, ctx, chunk, ppb):
         assert np.abs(total - covered.sum()).max() <= 1e-4 * covered.sum()
     finally:
         ctx.set_tuning(chunkPoints=before)
+
+
+@pytest.mark.parametrize("ppb", [1, 333, 1024, 2050, 10240])
+@pytest.mark.parametrize("mode,scale,most", [(0, 6.0, 40.0), (1, 0.004, 3.0), (1, 0.02, 9.0),
+                                             (1, 0.3, 64.0)])
+def test_splats(cr, orc, ctx, ppb, mode, scale, most):
+    """Footprints from a pixel to the largest (radius 16), with batches that
+    start unaligned, at a frame edge, with and without tiles."""
+    pos, rgba = blob_cloud(300 if ppb == 1 else 5000, 33)
+    cloud, _ = make_cloud(cr, orc, ctx, pos, rgba, ppb=ppb)
+    cfg = cr.ComputeRasteriserConfiguration(pointSizeMode=mode, pointSizeScale=scale,
+                                            maximumPointSize=most, depthTolerance=0.02)
+    try:
+        for tiles in (True, False):
+            ctx.set_tuning(useTiles=tiles)
+            for w, h in ((211, 97), (19, 23)):
+                cam = camera(cr, (0.3, 0.1, 1.2), w=w, h=h)
+                _, gpu, ref = render_both(cr, orc, ctx, [cloud], cfg, cam, w, h)
+                assert_same(cr, cfg, gpu, ref)
+    finally:
+        ctx.set_tuning(useTiles=True)
+
+
+@pytest.mark.parametrize("chunk", [256, 1000, 1025, 5000])
+def test_splats_of_two_clouds_and_chunk_sizes(cr, orc, ctx, chunk):
+    a, _ = make_cloud(cr, orc, ctx, *blob_cloud(7000, 41), ppb=2051)
+    b, _ = make_cloud(cr, orc, ctx, *lattice_cloud(16, 42), ppb=1500)
+    cfg = cr.ComputeRasteriserConfiguration(pointSizeMode=1, pointSizeScale=0.01,
+                                            maximumPointSize=7.0, holeFillIterations=3,
+                                            colorizeChunks=chunk == 1000)
+    before = ctx.tuning()["chunkPoints"]
+    try:
+        ctx.set_tuning(chunkPoints=chunk)
+        w, h = 240, 130
+        _, gpu, ref = render_both(cr, orc, ctx, [a, b], cfg, camera(cr, (0.5, 0.2, 2.2), w=w, h=h),
+                                  w, h)
+        assert_same(cr, cfg, gpu, ref)
+    finally:
+        ctx.set_tuning(chunkPoints=before)
+
+
+def test_splats_past_the_packed_bound(cr, ctx):
+    """More samples in a splat's pixels than the packed adds can hold: the
+    frame is drawn again with 32-bit adds, every sum modulo 2^32."""
+    from test_gpu_accum_wrap import LIMIT, stacked_cloud
+    samples, w = LIMIT + 11, 16
+    cloud = stacked_cloud(cr, ctx, samples)
+    ras = cr.ComputeRasteriser(ctx)
+    ras.configuration = cr.ComputeRasteriserConfiguration(
+        enableCLOD=False, enableLODDither=False, pointSizeMode=0, pointSizeScale=9.0,
+        maximumPointSize=3.0)  # 9 / 3 units away: 3 pixels, radius 1
+    ras.addPointCloud(cloud)
+    ras.resize((w, w))
+    ras.update(camera(cr, (0.0, 0.0, 3.0), w=w, h=w))
+    ras.encode()
+    px = ras.pixels()
+    hit = np.argwhere(px["count"] != 0)
+    assert len(hit) == 9 and (hit.max(0) - hit.min(0)).tolist() == [2, 2]
+    s = (255 * samples) % (1 << 32)
+    for y, x in hit:
+        assert [int(px[y, x][k]) for k in ("red", "green", "blue", "count")] == [s, s, s, samples]
+    rgba = ras.outputRGBA8()
+    assert (rgba[hit[:, 0], hit[:, 1], 3] == 255).all()
