@@ -1253,8 +1253,14 @@ __global__ void __launch_bounds__(kThreads, 6)
 // sum uses), and the colour pass starts from those instead of decoding,
 // projecting and sizing the points again.  A step whose rectangle is larger
 // than the tile goes to the frame pixel by pixel.
-// 20M points with 0.5 m splats at 1080p: one global atomic (depth) and one
-// depth read and two global adds (colour) per splat pixel took 108 and 292 us.
+// 20M points with 0.5 m splats at 1080p: the frame 433 -> 280 us (one global
+// atomic (depth), and one depth read and two global adds (colour) per splat
+// pixel, with a second decode, took 108 and 292 us; these passes 72 and 119).
+// Bound by the scattered global adds of the steps that do not fit a tile:
+// without tiles 305 us; tiles of 4,096 pixels (three CTAs an SM) the same as
+// of 2,048, of 6,144 or steps of 512 or 2,048 points slower; larger
+// rectangles cut into bands of the tile's size 338 us, since their splats
+// overlap too little to pay for clearing and flushing the bands.
 // ---------------------------------------------------------------------------
 constexpr int kSplatEach = 4;  // points per thread and step
 constexpr uint32_t kSplatPoints = kSplatEach * kThreads;
