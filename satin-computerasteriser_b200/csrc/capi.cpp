@@ -946,8 +946,13 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         // kPackedMaxCount proves that no field carried.
         const bool packed = !variants && (stages & CR_STAGE_COLOR) && (stages & CR_STAGE_RESOLVE) &&
                             max_samples < (1ull << 31);
+        // The variants' passes without coverage do the same, but are not run
+        // again: they pack while no pixel can pass kPackedMaxCount at all.
+        const bool variants_packed =
+            variants && !coverage && (stages & CR_STAGE_COLOR) && (stages & CR_STAGE_RESOLVE) &&
+            max_samples <= kPackedMaxCount;
         RasterTargets t{f->d_depth, f->d_accum, f->d_nearest};
-        t.packed = packed ? 1 : 0;
+        t.packed = packed || variants_packed ? 1 : 0;
         if (stages & CR_STAGE_DEPTH) {
             // The frame's depth plane, accumulators and redo word are zeroed
             // by extra CTAs of the first cull launch (its CTAs are few and

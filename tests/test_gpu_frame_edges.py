@@ -145,3 +145,39 @@ def test_splats_past_the_packed_bound(cr, ctx):
         assert [int(px[y, x][k]) for k in ("red", "green", "blue", "count")] == [s, s, s, samples]
     rgba = ras.outputRGBA8()
     assert (rgba[hit[:, 0], hit[:, 1], 3] == 255).all()
+
+
+@pytest.mark.parametrize("ppb,files", [(255, 1), (257, 5), (10240, 4)])
+@pytest.mark.parametrize("most", [1.0, 5.0])
+def test_effects_at_step_edges(cr, orc, ctx, ppb, files, most):
+    """Displacement and tint over batches around the 256-point steps, with a
+    file table in the kernel parameters and one past them, and with single
+    pixels and splats.  With no displacement and a tint of weight zero the
+    frame is the plain one's; with a weight below zero nothing is coloured."""
+    from scenes import to_product_packed
+    pos, rgba = blob_cloud(4000, 61)
+    packed = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=ppb)
+    prod = to_product_packed(cr, packed)
+    prod.files = cr.identity_files(files)
+    prod.batches = prod.batches.copy()
+    prod.batches["fileIndex"] = np.arange(len(prod.batches)) % files
+    cloud = cr.ComputeRasteriserPointCloud(ctx, packed=prod)
+    w, h = 97, 61
+    cam = camera(cr, (0.2, 0.1, 1.4), w=w, h=h)
+    cfg = cr.ComputeRasteriserConfiguration(pointSizeMode=0, pointSizeScale=4.0,
+                                            maximumPointSize=most)
+    ras, gpu, ref = render_both(cr, orc, ctx, [cloud], cfg, cam, w, h)
+    assert_same(cr, cfg, gpu, ref)
+    cfg.applyDisplacement = cfg.applyTint = True
+    cloud.displacementBuffer()
+    tint = cloud.tintBuffer()
+    zero = np.zeros(tint.shape, np.float32)
+    for weight in (0.0, -1.0):
+        zero[:, 3] = weight
+        tint.upload(zero)
+        ras.update(cam)
+        ras.encode()
+        px = ras.pixels()
+        assert np.array_equal(px["depth"], ref.depth)
+        accum = np.stack([px["red"], px["green"], px["blue"], px["count"]], -1)
+        assert np.array_equal(accum, ref.accum if weight == 0.0 else 0 * ref.accum)
