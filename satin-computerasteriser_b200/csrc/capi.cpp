@@ -456,6 +456,8 @@ CR_API cr_status cr_context_create(int device, cr_context **out) {
         e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->d_status), ctx->h_status, 0);
     if (e != cudaSuccess) {
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->h_pick) cudaFreeHost(ctx->h_pick);
+    if (ctx->d_pick) cudaFree(ctx->d_pick);
         cudaStreamDestroy(ctx->stream);
         delete ctx->pack;
         delete ctx;
@@ -486,6 +488,8 @@ CR_API cr_status cr_context_destroy(cr_context *ctx) {
     }
     cudaStreamDestroy(ctx->stream);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->h_pick) cudaFreeHost(ctx->h_pick);
+    if (ctx->d_pick) cudaFree(ctx->d_pick);
     delete ctx;
     return CR_OK;
 }
@@ -1320,28 +1324,12 @@ CR_API cr_status cr_pick(cr_context *ctx, cr_frame *f, cr_cloud *cloud, const fl
     const int pyb = trunc_i((ndc[1] * 0.5f + 0.5f) * (float)H);
     const int py = std::min(std::max(H - 1 - pyb, 0), H - 1);
     if ((st = nearest_index_pass(ctx, f, cloud, cfg, cam))) return st;
-    const int r = std::max(0, search_radius);
-    const int row0 = std::max(0, py - r), row1 = std::min(H - 1, py + r);
-    std::vector<uint32_t> band((size_t)(row1 - row0 + 1) * W);
-    if ((st = read_nearest(f, nullptr, band.data(), row0, row1 - row0 + 1))) return st;
-    long best_d = -1;
-    uint32_t best = 0;
-    const long r2 = (long)r * r;
-    for (int y = row0; y <= row1; ++y) {
-        const long dy = y - py;
-        for (int x = std::max(0, px - r); x <= std::min(W - 1, px + r); ++x) {
-            const long dx = x - px;
-            const long d = dx * dx + dy * dy;
-            if (d > r2 || (best_d >= 0 && d >= best_d)) continue;
-            const uint32_t v = band[(size_t)(y - row0) * W + x];
-            if (v != CR_INVALID_INDEX) {
-                best_d = d;
-                best = v;
-            }
-        }
-    }
-    if (best_d >= 0) {
-        *index_out = best;
+    if ((st = launch_pick(f, px, py, search_radius, ctx->stream))) return st;
+    CR_CUDA(cudaStreamSynchronize(ctx->stream));
+    if ((st = device_status(ctx))) return st;
+    const volatile uint32_t *picked = ctx->h_pick;
+    if (picked[0]) {
+        *index_out = picked[1];
         *found_out = 1;
     }
     return CR_OK;

@@ -104,6 +104,12 @@ struct cr_context {
     // after the calls that synchronise with the context's stream.
     uint32_t *h_status = nullptr;
     uint32_t *d_status = nullptr;
+    // cr_pick (lazy): the search's running minimum and CTA count (device
+    // memory, reset by the search itself), and its answer, found and index
+    // (page-locked, mapped as the status word is).
+    unsigned long long *d_pick = nullptr;
+    uint32_t *h_pick = nullptr;
+    uint32_t *d_picked = nullptr;
     // Profiling: a ring of frames, each with a start/stop event per pass.
     static constexpr int kProfRing = 256;
     bool profiling = false;
@@ -526,6 +532,10 @@ cr_status launch_hole_fill_views(const ViewDesc *views, uint32_t nviews, uint32_
 cr_status launch_resolve_nearest(cr_frame *f, const uint32_t *colors, const ResolveUniforms &u,
                                  cudaStream_t s);
 cr_status launch_hole_fill(cr_frame *f, int iterations, cudaStream_t s);
+// The nearest key plane's covered pixel closest to (px, py) within `radius`
+// pixels, the first in row order among equals: {found, its point's index} to
+// ctx->d_picked.
+cr_status launch_pick(cr_frame *f, int px, int py, int radius, cudaStream_t s);
 // XOR 0x80000000 into every word of the frame's depth plane.
 cr_status launch_flip_depth_order(cr_frame *f, cudaStream_t s);
 cr_status launch_split_nearest(const unsigned long long *keys, uint32_t *depth_out,

@@ -258,6 +258,45 @@ __global__ void __launch_bounds__(kThreads)
     if (index) index[p] = ~(uint32_t)k;
 }
 
+// Pixels [x0, x1] x [y0, y1] of the nearest key plane around (px, py): the
+// covered pixel with the smallest squared distance, at most r2, and among
+// equals the first in row order.  A candidate is its distance (33 bits at
+// most) above its pixel (31 bits), so the search is one 64-bit minimum: per
+// CTA, then over the CTAs in `best`; the last CTA writes the answer and sets
+// both words back for the next search.  (The rows of the window copied to the
+// host and searched there took 60 us of a pick of 150.)
+__global__ void __launch_bounds__(kThreads)
+    pick_nearest(const unsigned long long *__restrict__ keys, int w, int px, int py, int x0, int x1,
+                 int y0, int y1, long long r2, unsigned long long *best, uint32_t *out) {
+    crd::grid_wait();
+    crd::launch_dependents();
+    __shared__ unsigned long long s_best;
+    constexpr unsigned long long kNone = ~0ull;
+    if (threadIdx.x == 0) s_best = kNone;
+    __syncthreads();
+    const uint32_t cols = (uint32_t)(x1 - x0 + 1), n = cols * (uint32_t)(y1 - y0 + 1);
+    unsigned long long mine = kNone;
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+        const int x = x0 + (int)(i % cols), y = y0 + (int)(i / cols);
+        const long long dx = x - px, dy = y - py, d = dx * dx + dy * dy;
+        const uint32_t pix = (uint32_t)y * (uint32_t)w + (uint32_t)x;
+        if (d > r2 || ~(uint32_t)keys[pix] == 0xffffffffu) continue;
+        const unsigned long long c = ((unsigned long long)d << 31) | pix;
+        mine = c < mine ? c : mine;
+    }
+    if (mine != kNone) atomicMin(&s_best, mine);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (s_best != kNone) atomicMin(best, s_best);
+    __threadfence();
+    if (atomicAdd(reinterpret_cast<uint32_t *>(best + 1), 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    const unsigned long long b = atomicExch(best, kNone);
+    best[1] = 0ull;
+    out[1] = b != kNone ? ~(uint32_t)keys[b & 0x7fffffffull] : 0u;
+    out[0] = b != kNone ? 1u : 0u;
+}
+
 // Differentiable colours: the pixel's mean FP32 colour (background where no
 // sample), row 0 = top, 3 floats per pixel.
 __global__ void __launch_bounds__(kThreads)
@@ -443,6 +482,36 @@ cr_status launch_hole_fill(cr_frame *f, int iterations, cudaStream_t s) {
         CR_CUDA(cudaGetLastError());
         f->final_rgba = dst;
     }
+    return CR_OK;
+}
+
+cr_status launch_pick(cr_frame *f, int px, int py, int radius, cudaStream_t s) {
+    cr_context *ctx = f->ctx;
+    if (!ctx->d_pick) {
+        unsigned long long *d = nullptr;
+        CR_CUDA(cudaMalloc((void **)&d, 2 * sizeof(*d)));
+        const unsigned long long init[2] = {~0ull, 0ull};
+        if (const cudaError_t e = cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, s)) {
+            cudaFree(d);
+            return cri::cuda_fail(e, "cudaMemcpyAsync (pick words)");
+        }
+        ctx->d_pick = d;
+    }
+    if (!ctx->h_pick) {
+        CR_CUDA(cudaHostAlloc((void **)&ctx->h_pick, 2 * sizeof(uint32_t), cudaHostAllocMapped));
+        CR_CUDA(cudaHostGetDevicePointer((void **)&ctx->d_picked, ctx->h_pick, 0));
+    }
+    const long long r = std::max(radius, 0);
+    const int x0 = (int)std::max<long long>(0, px - r);
+    const int x1 = (int)std::min<long long>(f->width - 1, px + r);
+    const int y0 = (int)std::max<long long>(0, py - r);
+    const int y1 = (int)std::min<long long>(f->height - 1, py + r);
+    const uint32_t n = (uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1);  // below 2^31
+    const uint32_t grid = std::min((n + 4 * kThreads - 1) / (4 * kThreads),
+                                   (uint32_t)ctx->sm_count * 8);
+    CR_CUDA(launch_programmatic(pick_nearest, dim3(grid), dim3(kThreads), 0, s,
+                                (const unsigned long long *)f->d_nearest, f->width, px, py, x0, x1,
+                                y0, y1, r * r, ctx->d_pick, ctx->d_picked));
     return CR_OK;
 }
 

@@ -181,3 +181,25 @@ def test_effects_at_step_edges(cr, orc, ctx, ppb, files, most):
         assert np.array_equal(px["depth"], ref.depth)
         accum = np.stack([px["red"], px["green"], px["blue"], px["count"]], -1)
         assert np.array_equal(accum, ref.accum if weight == 0.0 else 0 * ref.accum)
+
+
+@pytest.mark.parametrize("radius", [0, 1, 10, 63, 100000])
+def test_pick_window(cr, orc, ctx, radius):
+    """The pick is the covered pixel nearest to the cursor, the first in row
+    order among equals, at any radius and at the frame's edges: the same
+    search over the index plane read back."""
+    pos, rgba = blob_cloud(400, 71)
+    cloud, _ = make_cloud(cr, orc, ctx, pos, rgba)
+    w, h = 150, 83
+    cam = camera(cr, (0.2, 0.1, 1.9), w=w, h=h)
+    cfg = cr.ComputeRasteriserConfiguration(mode=cr.MODE_NEAREST)
+    ras, _, _ = render_both(cr, orc, ctx, [cloud], cfg, cam, w, h)
+    plane = ras.nearestIndices()
+    ys, xs = np.nonzero(plane != 0xffffffff)
+    for nx, ny in ((0.0, 0.0), (-1.0, 1.0), (1.0, -1.0), (0.31, -0.27), (-0.9, -0.4)):
+        px = min(max(int(np.float32(nx * 0.5 + 0.5) * w), 0), w - 1)
+        py = min(max(h - 1 - int(np.float32(ny * 0.5 + 0.5) * h), 0), h - 1)
+        d = (xs - px) ** 2 + (ys - py) ** 2
+        best = np.lexsort((xs, ys, d))[0]
+        want = int(plane[ys[best], xs[best]]) if d[best] <= radius * radius else None
+        assert ras.pickPointIndex((nx, ny), cloud, cam, searchRadius=radius) == want
