@@ -227,7 +227,7 @@ cr_status allocate_cloud(cr_cloud *c, cr_capacity cap, const cr_raster_file *fil
         return st;
     c->chunk_cap = chunk_capacity(cap, kMinChunkPoints);
     if ((st = dalloc(&c->d_chunks, c->chunk_cap * sizeof(ChunkRec))) ||
-        (st = dalloc(&c->d_frag_count, c->chunk_cap * sizeof(uint32_t))) ||
+        (st = dalloc(&c->d_frag_count, c->chunk_cap * kFragCounts * sizeof(uint32_t))) ||
         (st = dalloc(&c->d_frag_xy, pts * 4)) || (st = dalloc(&c->d_frag_zc, pts * 8)))
         return st;
     c->d_files_cap = (uint32_t)c->files.size();

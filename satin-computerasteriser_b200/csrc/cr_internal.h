@@ -80,6 +80,8 @@ static_assert(sizeof(CullRec) == 64, "CullRec is 64 bytes");
 static_assert(sizeof(ChunkRec) == 64, "ChunkRec is 64 bytes");
 
 constexpr int kMinChunkPoints = 256;
+// Fragment counts per chunk record: one for each warp of the depth pass's CTA.
+constexpr uint32_t kFragCounts = 8;
 
 struct cr_context {
     PackScratch *pack = nullptr;  // grow-only packer scratch
@@ -207,7 +209,7 @@ struct cr_cloud {
     // starting at point p keeps its n kept points compacted at [p, p + n).
     uint32_t *d_frag_xy = nullptr;     // pixel x | row << 16
     uint2 *d_frag_zc = nullptr;        // NDC z bits, RGBA8 (after the colorize options)
-    uint32_t *d_frag_count = nullptr;  // kept points per chunk record
+    uint32_t *d_frag_count = nullptr;  // kept points per chunk record and warp (kFragCounts)
     // Per-point float4 attributes of the colour variants, written by user
     // kernels (lazy, zeroed on allocation): displacement, the previous
     // frame's displacement (motion blur), tint.
@@ -456,8 +458,8 @@ static_assert(sizeof(ViewDesc) == 192, "ViewDesc is 192 bytes");
 
 // Fragment arena of one cloud's batched views: view v's fragments occupy
 // [prefix of the views' fragment spans, + its span); chunk record j of view
-// v has its count at count[v * chunk_stride + j] and its offset within the
-// view's span at poff[same].  cap entries; *overflow is set by the depth
+// v has its kFragCounts counts at count[(v * chunk_stride + j) * kFragCounts]
+// and its offset within the view's span at poff[v * chunk_stride + j].  cap entries; *overflow is set by the depth
 // pass when the spans exceed cap (the colour pass then decodes the points).
 struct ViewsFragments {
     uint32_t *xy;

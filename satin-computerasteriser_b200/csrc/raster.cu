@@ -75,8 +75,6 @@ struct TileCfg<PASS_DEPTH_FRAG> {
     static constexpr int kBytes = kPx * 4;
 };
 template <>
-struct TileCfg<PASS_COLOR_FRAG> : TileCfg<PASS_COLOR> {};
-template <>
 struct TileCfg<PASS_COLOR_F32> {  // no screen tiles
     static constexpr int kPx = 0;
     static constexpr int kBytes = 0;
@@ -85,7 +83,7 @@ template <>
 struct TileCfg<PASS_GRAD> : TileCfg<PASS_COLOR_F32> {};
 
 __host__ __device__ constexpr bool is_depth(int p) { return p == PASS_DEPTH || p == PASS_DEPTH_FRAG; }
-__host__ __device__ constexpr bool is_color(int p) { return p == PASS_COLOR || p == PASS_COLOR_FRAG; }
+__host__ __device__ constexpr bool is_color(int p) { return p == PASS_COLOR; }
 
 struct RasterArgs {
     const ChunkRec *chunks;
@@ -275,7 +273,7 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
     const int W = vw<MV>(vr), H = vh<MV>(vr);
     o.ix = (int)((nx * 0.5f + 0.5f) * (float)W);
     const int iy = (int)((ny * 0.5f + 0.5f) * (float)H);
-    if (o.ix < 0 || o.ix >= W || iy < 0 || iy >= H) ok = false;
+    if ((uint32_t)o.ix >= (uint32_t)W || (uint32_t)iy >= (uint32_t)H) ok = false;
     o.iy = H - 1 - iy;
     // depth_to_uint without its clamps: the saturating conversion already
     // maps z * 2^32 to 0 for z <= 0 or NaN and to 0xFFFFFFFF for z >= 1.
@@ -472,73 +470,43 @@ __device__ __forceinline__ void emit_footprint(const RasterArgs &a, const ViewRe
     if (PASS == PASS_GRAD) grad_store(a, o.pointIndex, g);
 }
 
-// Shared count of the fragments the current chunk has kept.
-__shared__ uint32_t s_frag_count;
+// A chunk's points are split over the CTA's warps in contiguous pieces of
+// whole 128-point rounds (warp_span points a warp, the same split in every
+// pass): each warp packs the fragments of its piece from the piece's own
+// start, counting them in a register, and leaves its count beside the other
+// warps' (kFragWarps per chunk record); the colour pass walks each piece with
+// the warp of the same number.  One count per chunk instead took a
+// shared-memory atomic and a shuffle per point (per two points in the
+// one-view kernel, at the price of eight registers).  100M points at 1080p: the
+// frame 358 -> 353 us; a 1M-point lattice at 720p 45.6 -> 41.0; 64 views of 50M
+// points 9.30 -> 9.12 ms.
+constexpr uint32_t kFragWarps = kThreads / 32;
+static_assert(kFragWarps == kFragCounts, "the count arrays have a word per warp");
+__device__ __forceinline__ uint32_t warp_span(uint32_t count) {
+    return 128u * ((count + 128u * kFragWarps - 1u) / (128u * kFragWarps));
+}
 
-// Appends the warp's kept points to the chunk's fragment range [fbase, fbase+n):
-// one shared-memory atomic per warp, lanes placed by ballot rank.
-__device__ __forceinline__ void emit_fragment(const RasterArgs &a, uint32_t fbase,
-                                              const PointOut &o) {
-    const bool keep = o.ok;
-    const uint32_t ballot = __ballot_sync(kFull, keep);
-    const int lane = threadIdx.x & 31;
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&s_frag_count, __popc(ballot));
-    base = __shfl_sync(kFull, base, 0);
-    if (keep) {
-        const uint32_t i = fbase + base + __popc(ballot & ((1u << lane) - 1u));
+// Appends the warp's kept points at fragment `at`, lanes placed by ballot
+// rank; returns how many were kept.
+__device__ __forceinline__ uint32_t emit_fragment(const RasterArgs &a, uint32_t at,
+                                                  const PointOut &o) {
+    const uint32_t ballot = __ballot_sync(kFull, o.ok);
+    if (o.ok) {
+        const uint32_t i = at + __popc(ballot & ((1u << (threadIdx.x & 31)) - 1u));
         a.frag_xy[i] = (uint32_t)o.ix | ((uint32_t)o.iy << 16);
         a.frag_zc[i] = make_uint2(__float_as_uint(o.nz), o.color);
     }
-}
-
-// A point's fragment, held back so that several points of a thread are
-// appended with one shared-memory atomic per warp.  Two points per atomic:
-// the one-view depth pass 212 -> 207 µs on the 100M-point 1080p frames;
-// four spill registers and were slower, and so does the batched-view kernel
-// with two.
-struct Frag {
-    bool keep;
-    uint32_t xy;
-    float z;
-    uint32_t col;
-};
-constexpr int kFragBatch = 2;
-
-// Appends N fragments per lane: one ballot per fragment, one atomic per warp.
-template <int N>
-__device__ __forceinline__ void emit_fragments(const RasterArgs &a, uint32_t fbase,
-                                               const Frag (&f)[N]) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t b[N], tot = 0;
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        b[k] = __ballot_sync(kFull, f[k].keep);
-        tot += __popc(b[k]);
-    }
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&s_frag_count, tot);
-    base = __shfl_sync(kFull, base, 0);
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        if (f[k].keep) {
-            const uint32_t i = fbase + base + __popc(b[k] & lt);
-            a.frag_xy[i] = f[k].xy;
-            a.frag_zc[i] = make_uint2(__float_as_uint(f[k].z), f[k].col);
-        }
-        base += __popc(b[k]);
-    }
+    return __popc(ballot);
 }
 
 // One point; every lane of the warp calls this (warp-uniform early outs).
-// With fo, the depth pass's fragment is returned there instead of appended.
+// frag_at: the depth pass's next fragment, advanced by the points it kept.
 template <int PASS, bool MV>
 __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const BatchShared &sb,
                                          unsigned char *smem, const ChunkRec &c, bool tiled,
                                          bool valid, uint32_t local, uint32_t lvl, uint32_t lo,
-                                         uint32_t me, uint32_t hi, uint32_t color, uint32_t fbase,
-                                         bool emit, bool all_keep, Frag *fo = nullptr) {
+                                         uint32_t me, uint32_t hi, uint32_t color,
+                                         uint32_t &frag_at, bool emit, bool all_keep) {
     PointOut o;
     o.pointIndex = c.first + local;
     o.color = color;
@@ -556,98 +524,7 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
         emit_tile<PASS, MV>(a, vr, c, smem, o);
     else
         emit_direct<PASS, MV>(a, vr, o);
-    if (PASS == PASS_DEPTH_FRAG && emit) {
-        if (fo) {
-            fo->keep = o.ok;
-            fo->xy = (uint32_t)o.ix | ((uint32_t)o.iy << 16);
-            fo->z = o.nz;
-            fo->col = o.color;
-        } else {
-            emit_fragment(a, fbase, o);
-        }
-    }
-}
-
-// One fragment of the colour pass (PASS_COLOR_FRAG); every lane calls this.
-template <bool MV>
-__device__ __forceinline__ void do_fragment(const RasterArgs &a, const ViewRegsT<MV> &vr, unsigned char *smem,
-                                            const ChunkRec &c, bool tiled, bool valid,
-                                            uint32_t xy, float nz, uint32_t color) {
-    PointOut o;
-    o.ok = valid;
-    o.ix = (int)(xy & 0xffffu);
-    o.iy = (int)(xy >> 16);
-    o.nz = nz;
-    o.color = color;
-    if (tiled)
-        emit_tile<PASS_COLOR_FRAG, MV>(a, vr, c, smem, o);
-    else
-        emit_direct<PASS_COLOR_FRAG, MV>(a, vr, o);
-}
-
-// Four fragments of one thread in the colour pass, the first `nvalid` of
-// them real.  The settled depths of all four pixels are read (read-only
-// path, or the tile's staged copy) before any accumulation, so the thread
-// waits for one L2 round trip per quad instead of one per fragment.
-template <bool MV>
-__device__ __forceinline__ void color_quad(const RasterArgs &a, const ViewRegsT<MV> &vr, unsigned char *smem,
-                                           const ChunkRec &c, bool tiled, uint32_t nvalid,
-                                           const uint4 &xy4, const float4 &z4, const uint4 &co4) {
-    constexpr int kPx = TileCfg<PASS_COLOR>::kPx;
-    uint32_t *acc = reinterpret_cast<uint32_t *>(smem);
-    const uint32_t *sdep = acc + 3 * kPx;
-    const uint32_t xy[4] = {xy4.x, xy4.y, xy4.z, xy4.w};
-    const float nz[4] = {z4.x, z4.y, z4.z, z4.w};
-    const uint32_t col[4] = {co4.x, co4.y, co4.z, co4.w};
-    uint32_t pix[4], closest[4];
-    int l[4];
-    bool in[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int ix = (int)(xy[i] & 0xffffu), iy = (int)(xy[i] >> 16);
-        pix[i] = (uint32_t)(iy * vw<MV>(vr) + ix);
-        const int lx = ix - c.x0, ly = iy - c.y0;
-        in[i] = tiled && (unsigned)lx < (unsigned)c.tw && (unsigned)ly < (unsigned)c.th;
-        l[i] = in[i] ? ly * c.tw + lx : 0;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        closest[i] = 0u;
-        if ((uint32_t)i < nvalid) closest[i] = in[i] ? sdep[l[i]] : __ldg(vdepth<MV>(vr) + pix[i]);
-    }
-    // Consecutive visible fragments of the quad on the same pixel (neighbour
-    // points of a Morton-ordered batch often share one) are summed in
-    // registers and added once: fewer adds to a contended address.
-    uint32_t rr = 0, gg = 0, bb = 0, nn = 0, cur = 0xffffffffu;
-    bool cin = false;
-    int cl = 0;
-    auto flush = [&]() {
-        if (nn == 0u) return;
-        if (cin) {
-            atomicAdd(acc + cl, rr | (nn << 20));
-            atomicAdd(acc + kPx + cl, gg);
-            atomicAdd(acc + 2 * kPx + cl, bb);
-        } else {
-            color_global<MV>(a, vr, cur, rr, gg, bb, nn);
-        }
-    };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const bool vis = closest[i] != 0u && nz[i] >= crd::uint_to_depth(closest[i]) * a.keep_scale;
-        if (!vis) continue;
-        if (pix[i] != cur) {
-            flush();
-            cur = pix[i];
-            cin = in[i];
-            cl = l[i];
-            rr = gg = bb = nn = 0u;
-        }
-        rr += col[i] & 0xffu;
-        gg += (col[i] >> 8) & 0xffu;
-        bb += (col[i] >> 16) & 0xffu;
-        nn += 1u;
-    }
-    flush();
+    if (PASS == PASS_DEPTH_FRAG && emit) frag_at += emit_fragment(a, frag_at, o);
 }
 
 template <int PASS, bool MV>
@@ -735,11 +612,11 @@ __device__ __forceinline__ uint32_t find_view(const uint32_t *begin, uint32_t nv
 // switches frame, camera and file table when the view changes.
 template <int PASS, bool MV>
 __device__ __forceinline__ void raster_body(const RasterArgs &a) {
-    constexpr bool kFrag = PASS == PASS_DEPTH_FRAG || PASS == PASS_COLOR_FRAG;
+    constexpr bool kFrag = PASS == PASS_DEPTH_FRAG;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ BatchShared sb;
     __shared__ __align__(16) ChunkRec rec[2];
-    __shared__ __align__(16) uint32_t rec_frags[2][4];  // frag count, span offset
+    __shared__ __align__(16) uint32_t rec_poff[2][4];  // offset in the view's fragment span
     __shared__ uint32_t s_vbegin[MV ? kMaxViews + 1 : 1];
     __shared__ unsigned long long s_pbegin[MV && kFrag ? kMaxViews + 1 : 1];
     __shared__ uint32_t s_wsum[kThreads / 32];
@@ -826,13 +703,11 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         for (int q = 0; q < 4; ++q)
             cp_async16(reinterpret_cast<uint4 *>(&rec[b]) + q,
                        reinterpret_cast<const uint4 *>(a.chunks + slot) + q);
-        if (PASS == PASS_COLOR_FRAG) cp_async4(&rec_frags[b][0], a.frag_count + slot);
-        if (MV && kFrag) cp_async4(&rec_frags[b][1], a.chunk_poff + slot);
+        if (MV && kFrag) cp_async4(&rec_poff[b][0], a.chunk_poff + slot);
     };
     if (threadIdx.x == 0) {
         claim(0);
         sb.file = 0xffffffffu;
-        s_frag_count = 0u;
     }
     cp_async_commit();
     uint32_t loaded_view = 0xffffffffu;
@@ -842,20 +717,18 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         if (s_k[buf] >= nchunks) break;
         const uint32_t cur_view = s_kview[buf], cur_slot = s_kslot[buf];
         const ChunkRec c = rec[buf];
-        const uint32_t nfrag = PASS == PASS_COLOR_FRAG ? rec_frags[buf][0] : 0u;
         const uint32_t fslot = cur_slot;
         // First fragment of the chunk: pool index space (one view), or the
         // view's fragment span in the arena (batched views).
         const uint32_t fbase =
-            MV ? (kFrag ? (uint32_t)(s_pbegin[cur_view] + rec_frags[buf][1]) : 0u) : c.first;
+            MV ? (kFrag ? (uint32_t)(s_pbegin[cur_view] + rec_poff[buf][0]) : 0u) : c.first;
         if (threadIdx.x == 0) claim(buf ^ 1);
         cp_async_commit();
         const uint32_t file_id = MV ? cur_view * a.nfiles + c.file : c.file;
         const bool new_file = file_id != sb.file;
-        const uint32_t work = PASS == PASS_COLOR_FRAG ? nfrag : c.count;
         const bool tiled = a.use_tiles && a.radius_zero && c.tw > 0 &&
                            c.tw * c.th <= TileCfg<PASS>::kPx &&
-                           c.tw * c.th <= (int)work &&
+                           c.tw * c.th <= (int)c.count &&
                            (!is_color(PASS) || c.count < 4096u);
         if (new_file || tiled) {
             __syncthreads();  // everyone has read sb.file (and the view state)
@@ -902,44 +775,20 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         // highest level (7) does with the largest dither (hash_unit reaches
         // 1.0f; 0.5f without dither): (thr - L) + 0.5f only grows as L falls.
         const bool all_keep = (a.u.lodDither ? 1.0f : 0.5f) < (c.thr - 7.0f) + 0.5f;
-        if (PASS == PASS_COLOR_FRAG) {
-            // The chunk's fragments, four per thread when 16-byte aligned.
-            if ((fbase & 3u) == 0u) {
-                const uint32_t nquads = (nfrag + 3u) >> 2;
-                for (uint32_t q0 = 0; q0 < nquads; q0 += kThreads) {
-                    const uint32_t q = q0 + threadIdx.x;
-                    const uint32_t base = fbase + 4u * q;
-                    uint4 xy4 = make_uint4(0, 0, 0, 0), co4 = xy4;
-                    float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (q < nquads) {
-                        xy4 = __ldcs(reinterpret_cast<const uint4 *>(a.frag_xy + base));
-                        const uint4 zc01 = __ldcs(reinterpret_cast<const uint4 *>(a.frag_zc + base));
-                        const uint4 zc23 =
-                            __ldcs(reinterpret_cast<const uint4 *>(a.frag_zc + base + 2));
-                        z4 = make_float4(__uint_as_float(zc01.x), __uint_as_float(zc01.z),
-                                         __uint_as_float(zc23.x), __uint_as_float(zc23.z));
-                        co4 = make_uint4(zc01.y, zc01.w, zc23.y, zc23.w);
-                    }
-                    const uint32_t nv = q < nquads ? min(4u, nfrag - 4u * q) : 0u;
-                    color_quad<MV>(a, vr, smem, c, tiled, nv, xy4, z4, co4);
-                }
-            } else {
-                for (uint32_t l0 = 0; l0 < nfrag; l0 += kThreads) {
-                    const uint32_t l = l0 + threadIdx.x;
-                    const bool v = l < nfrag;
-                    const uint32_t i = fbase + (v ? l : 0u);
-                    const uint2 zc = v ? a.frag_zc[i] : make_uint2(0u, 0u);
-                    do_fragment<MV>(a, vr, smem, c, tiled, v, v ? a.frag_xy[i] : 0u,
-                                    __uint_as_float(zc.x), zc.y);
-                }
-            }
-        } else if ((c.first & 3u) == 0u) {
+        // The warp's piece of the chunk and its fragments' place.
+        const uint32_t span = warp_span(c.count), piece = (threadIdx.x >> 5) * span;
+        // Passes without fragments take rounds of the whole CTA in turn.
+        constexpr bool kPieces = PASS == PASS_DEPTH_FRAG;
+        const uint32_t end = kPieces ? min(piece + span, c.count) : c.count;
+        const uint32_t frag0 = fbase + piece;
+        uint32_t frag_at = frag0;
+        if ((c.first & 3u) == 0u) {
             // Four points per thread, 16-byte loads.
-            const uint32_t nquads = (c.count + 3u) >> 2;
-            for (uint32_t q0 = 0; q0 < nquads; q0 += kThreads) {
-                const uint32_t q = q0 + threadIdx.x;
-                const bool qv = q < nquads;
-                const uint32_t base = c.first + 4u * q;
+            for (uint32_t p0 = kPieces ? piece : 4u * (threadIdx.x & ~31u); p0 < end;
+                 p0 += kPieces ? 128u : 4u * kThreads) {
+                const uint32_t l0 = p0 + 4u * (threadIdx.x & 31);
+                const bool qv = l0 < end;
+                const uint32_t base = c.first + l0;
                 uint32_t lv4 = 0;
                 uint4 lo4 = make_uint4(0, 0, 0, 0), me4 = lo4, hi4 = lo4, co4 = lo4;
                 if (qv) {
@@ -950,68 +799,43 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                     if (kNeedColor)
                         co4 = __ldg(reinterpret_cast<const uint4 *>(a.colors + base));
                 }
-                const uint32_t l0 = 4u * q;
-                if (PASS == PASS_DEPTH_FRAG && !MV && emit) {
-                    // The fragments of kFragBatch points per atomic (one
-                    // view: the batched-view kernel has no registers to
-                    // spare for them).
-                    constexpr int kB = kFragBatch;
-                    Frag f[kB];
-                    const uint32_t lvs[4] = {lv4 & 0xffu, (lv4 >> 8) & 0xffu, (lv4 >> 16) & 0xffu,
-                                             lv4 >> 24};
-                    const uint32_t los[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
-                    const uint32_t mes[4] = {me4.x, me4.y, me4.z, me4.w};
-                    const uint32_t his[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
-                    const uint32_t cos[4] = {co4.x, co4.y, co4.z, co4.w};
+                const uint32_t lvs[4] = {lv4 & 0xffu, (lv4 >> 8) & 0xffu, (lv4 >> 16) & 0xffu,
+                                         lv4 >> 24};
+                const uint32_t los[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
+                const uint32_t mes[4] = {me4.x, me4.y, me4.z, me4.w};
+                const uint32_t his[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
+                const uint32_t cos[4] = {co4.x, co4.y, co4.z, co4.w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        do_point<PASS, MV>(a, vr, sb, smem, c, tiled, qv && l0 + j < c.count,
-                                           l0 + j, lvs[j], los[j], mes[j], his[j], cos[j], fbase,
-                                           emit, all_keep, &f[j % kB]);
-                        if (j % kB == kB - 1) emit_fragments<kB>(a, fbase, f);
-                    }
-                } else {
-                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, qv && l0 + 0 < c.count, l0 + 0,
-                                       lv4 & 0xffu, lo4.x, me4.x, hi4.x, co4.x, fbase, emit,
-                                       all_keep);
-                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, qv && l0 + 1 < c.count, l0 + 1,
-                                       (lv4 >> 8) & 0xffu, lo4.y, me4.y, hi4.y, co4.y, fbase,
-                                       emit, all_keep);
-                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, qv && l0 + 2 < c.count, l0 + 2,
-                                       (lv4 >> 16) & 0xffu, lo4.z, me4.z, hi4.z, co4.z, fbase,
-                                       emit, all_keep);
-                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, qv && l0 + 3 < c.count, l0 + 3,
-                                       lv4 >> 24, lo4.w, me4.w, hi4.w, co4.w, fbase, emit,
-                                       all_keep);
-                }
+                for (int j = 0; j < 4; ++j)
+                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, l0 + j < end, l0 + j, lvs[j],
+                                       los[j], mes[j], his[j], cos[j], frag_at, emit, all_keep);
             }
         } else {
             // Unaligned start (pointsPerBatch not a multiple of 4): one point per thread.
-            for (uint32_t l0 = 0; l0 < c.count; l0 += kThreads) {
-                const uint32_t local = l0 + threadIdx.x;
-                const bool v = local < c.count;
+            for (uint32_t p0 = kPieces ? piece : (threadIdx.x & ~31u); p0 < end;
+                 p0 += kPieces ? 32u : kThreads) {
+                const uint32_t local = p0 + (threadIdx.x & 31);
+                const bool v = local < end;
                 const uint32_t i = c.first + (v ? local : 0u);
                 const uint32_t lv = v ? a.levels[i] : 0u;
                 const uint32_t lo = v ? a.low[i] : 0u;
                 const uint32_t me = (v && need_med) ? a.med[i] : 0u;
                 const uint32_t hi = (v && need_high) ? a.high[i] : 0u;
                 const uint32_t co = (v && kNeedColor) ? a.colors[i] : 0u;
-                do_point<PASS, MV>(a, vr, sb, smem, c, tiled, v, local, lv, lo, me, hi, co, fbase, emit, all_keep);
+                do_point<PASS, MV>(a, vr, sb, smem, c, tiled, v, local, lv, lo, me, hi, co,
+                                   frag_at, emit, all_keep);
             }
         }
-        if (tiled || PASS == PASS_DEPTH_FRAG) {
+        if (PASS == PASS_DEPTH_FRAG && (threadIdx.x & 31) == 0)
+            a.frag_count[fslot * kFragWarps + (threadIdx.x >> 5)] = frag_at - frag0;
+        if (tiled) {
             __syncthreads();
-            if (tiled) tile_flush<PASS, MV>(a, vr, c, smem);
-            if (PASS == PASS_DEPTH_FRAG && threadIdx.x == 0) {
-                a.frag_count[fslot] = s_frag_count;
-                s_frag_count = 0u;
-            }
+            tile_flush<PASS, MV>(a, vr, c, smem);
         }
     }
     cp_async_wait_all();
     finish();
 }
-
 
 // Colour pass over the depth pass's fragments for one view, one chunk per CTA
 // (claimed from the work cursor).  A chunk's points are one compact region of
@@ -1065,26 +889,42 @@ __device__ __forceinline__ void hash_clear(uint32_t *hkey, uint32_t *hsum) {
     }
 }
 
-// The colour pass over one chunk's n fragments starting at base, against
-// the frame of W columns whose depth plane is `depth`: sums into the table.
+// Streaming loads of two fragments' words (zero where there are none).
+__device__ __forceinline__ uint2 load2(const uint32_t *p, bool in) {
+    return in ? __ldcs(reinterpret_cast<const uint2 *>(p)) : make_uint2(0u, 0u);
+}
+__device__ __forceinline__ uint4 load4(const uint2 *p, bool in) {
+    return in ? __ldcs(reinterpret_cast<const uint4 *>(p)) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The colour pass over the fragments of chunk record `slot`, whose range
+// starts at base, against the frame of W columns whose depth plane is `depth`:
+// sums into the table.  Each warp walks its piece of the range.
 template <bool MV>
 __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<MV> &vr,
-                                           uint32_t *hkey, uint32_t *hsum, uint32_t n,
+                                           uint32_t *hkey, uint32_t *hsum, size_t slot,
                                            uint32_t base, int W, const uint32_t *depth) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t n = __ldg(a.frag_count + slot * kFragWarps + warp);
+    base += warp * warp_span(__ldg(&a.chunks[slot].count));
     if ((base & 3u) == 0u) {
-        for (uint32_t f = 4u * threadIdx.x; f < n; f += 4u * kThreads) {
-            const uint4 xy = __ldcs(reinterpret_cast<const uint4 *>(a.frag_xy + base + f));
-            const uint4 zc01 = __ldcs(reinterpret_cast<const uint4 *>(a.frag_zc + base + f));
-            const uint4 zc23 = __ldcs(reinterpret_cast<const uint4 *>(a.frag_zc + base + f + 2));
-            const uint32_t xs[4] = {xy.x, xy.y, xy.z, xy.w},
-                           cs[4] = {zc01.y, zc01.w, zc23.y, zc23.w};
-            const float zs[4] = {__uint_as_float(zc01.x), __uint_as_float(zc01.z),
-                                 __uint_as_float(zc23.x), __uint_as_float(zc23.z)};
+        // Two neighbouring fragments per lane and half round: a piece's last
+        // round then fills whole half warps before it leaves lanes idle.
+        for (uint32_t f0 = 2u * lane; f0 - 2u * lane < n; f0 += 128u) {
+            const uint32_t f1 = f0 + 64u;
+            const uint2 x0 = load2(a.frag_xy + base + f0, f0 < n);
+            const uint2 x1 = load2(a.frag_xy + base + f1, f1 < n);
+            const uint4 z0 = load4(a.frag_zc + base + f0, f0 < n);
+            const uint4 z1 = load4(a.frag_zc + base + f1, f1 < n);
+            const uint32_t fs[4] = {f0, f0 + 1u, f1, f1 + 1u};
+            const uint32_t xs[4] = {x0.x, x0.y, x1.x, x1.y}, cs[4] = {z0.y, z0.w, z1.y, z1.w};
+            const float zs[4] = {__uint_as_float(z0.x), __uint_as_float(z0.z),
+                                 __uint_as_float(z1.x), __uint_as_float(z1.z)};
             uint32_t pix[4], cl[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 pix[q] = (xs[q] >> 16) * (uint32_t)W + (xs[q] & 0xffffu);
-                cl[q] = f + q < n ? __ldg(depth + pix[q]) : 0u;
+                cl[q] = fs[q] < n ? __ldg(depth + pix[q]) : 0u;
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -1092,7 +932,7 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
                     hash_add<MV>(hkey, hsum, a, vr, pix[q], xs[q], cs[q]);
         }
     } else {
-        for (uint32_t f = threadIdx.x; f < n; f += kThreads) {
+        for (uint32_t f = lane; f < n; f += 32u) {
             const uint32_t xy = a.frag_xy[base + f];
             const uint32_t pix = (xy >> 16) * (uint32_t)W + (xy & 0xffffu);
             const uint32_t cl = __ldg(depth + pix);
@@ -1130,8 +970,7 @@ __device__ __forceinline__ void hash_flush(const RasterArgs &a, const ViewRegsT<
 __device__ __forceinline__ void hash_chunk(const RasterArgs &a, const ViewRegsT<false> &vr,
                                            uint32_t *hkey, uint32_t *hsum, uint32_t k,
                                            uint32_t *cursor = nullptr, uint32_t *next = nullptr) {
-    const uint32_t nfrag = __ldg(a.frag_count + k);
-    hash_frags<false>(a, vr, hkey, hsum, nfrag, __ldg(&a.chunks[k].first), a.u.width, a.t.depth);
+    hash_frags<false>(a, vr, hkey, hsum, k, __ldg(&a.chunks[k].first), a.u.width, a.t.depth);
     __syncthreads();  // the chunk's sums are complete (and k has been read by all)
     hash_flush<false>(a, vr, hkey, hsum, cursor, next);
 }
@@ -1225,8 +1064,7 @@ __global__ void __launch_bounds__(kThreads, 6)
         const uint32_t slot = view * a.chunk_stride + (k - s_vbegin[view]);
         const ViewDesc &vd = a.views[view];
         const ViewRegsT<true> vr{vd.width, vd.height, vd.depth, vd.accum, vd.nearest};
-        const uint32_t nfrag = __ldg(a.frag_count + slot);
-        hash_frags<true>(a, vr, hkey, hsum, nfrag,
+        hash_frags<true>(a, vr, hkey, hsum, slot,
                          (uint32_t)(s_pbegin[view] + __ldg(a.chunk_poff + slot)), vd.width,
                          vd.depth);
         __syncthreads();  // the chunk's sums are complete (and k has been read by all)

@@ -68,7 +68,7 @@ struct ViewsCloud {
     ChunkRec *chunks = nullptr;           // nviews * chunk_stride
     uint32_t *counters = nullptr;         // nviews * CNT_COUNT
     uint32_t *chunk_poff = nullptr;       // nviews * chunk_stride
-    uint32_t *frag_count = nullptr;       // nviews * chunk_stride
+    uint32_t *frag_count = nullptr;       // nviews * chunk_stride * kFragCounts
     uint32_t *frag_xy = nullptr;  // frag_cap each
     uint2 *frag_zc = nullptr;
     uint32_t *frag_overflow = nullptr;
@@ -287,7 +287,8 @@ cr_status views_alloc(cr_context *ctx, ViewsState *s, cr_frame *const *frames, u
             const unsigned long long budget = free_b / 8 / std::max(nclouds, 1u) / 12;
             vc.frag_cap = std::min<unsigned long long>({need, budget, 0xfffffff0ull});
             const size_t slots = (size_t)nviews * vc.chunk_stride;
-            if ((st = dalloc(&vc.chunk_poff, slots * 4)) || (st = dalloc(&vc.frag_count, slots * 4)) ||
+            if ((st = dalloc(&vc.chunk_poff, slots * 4)) ||
+                (st = dalloc(&vc.frag_count, slots * kFragCounts * 4)) ||
                 (st = dalloc(&vc.frag_xy, vc.frag_cap * 4)) ||
                 (st = dalloc(&vc.frag_zc, vc.frag_cap * 8)) ||
                 (st = dalloc(&vc.frag_overflow, 16)))
@@ -336,7 +337,7 @@ cr_status views_enqueue(cr_context *ctx, ViewsState *s, int b, cr_cloud *const *
             const size_t slot0 = (size_t)v0 * vc.chunk_stride;
             const ViewsFragments fr{vc.frag_xy,
                                     vc.frag_zc,
-                                    vc.frag_count ? vc.frag_count + slot0 : nullptr,
+                                    vc.frag_count ? vc.frag_count + slot0 * kFragCounts : nullptr,
                                     vc.chunk_poff ? vc.chunk_poff + slot0 : nullptr,
                                     vc.frag_cap,
                                     vc.frag_overflow};
