@@ -1478,15 +1478,18 @@ __global__ void __launch_bounds__(kThreads) raster_kernel(const __grid_constant_
 }
 
 // The differentiable passes of one view with single-pixel footprints (depth
-// plane, FP32 colour sums, adjoint): a thread per point, 256 points of a
-// chunk record to a step, `steps` steps to a record; the grid strides over
-// all of them.  A training view holds a million points or so, of which the
+// plane, FP32 colour sums, adjoint): 512 points of a chunk record to a step,
+// two to a thread, `steps` steps to a record; the grid strides over all of
+// them.  A training view holds a million points or so, of which the
 // four-points-a-thread passes make two rounds in the few hundred chunks that
 // there are: half of the SMs' warps had no work, and each waited for its
-// chain of loads (record, words, depth, colour) alone.  With a step to a CTA
-// the work spreads over every warp slot.  10M points, 512 x 512, a view:
-// depth 25 -> 13 us, colour 38 -> 16 us, adjoint 33 -> 17 us.
-constexpr int kStepPoints = kThreads;
+// chain of loads (record, words, depth, colour) alone.  Steps spread the work
+// over every warp slot, and a thread's two points wait together.  10M points,
+// 512 x 512, 16 views: the step 1.80 ms with the four-point passes, 1.17 with a
+// point a thread (six CTAs an SM; 1.14 with eight), 1.12 with two (1.14 with
+// five CTAs), 1.19 with four.
+constexpr int kStepEach = 2;  // points per thread and step
+constexpr int kStepPoints = kStepEach * kThreads;
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 6)
     point_pass(const __grid_constant__ RasterArgs a, uint32_t steps) {
@@ -1498,26 +1501,57 @@ __global__ void __launch_bounds__(kThreads, 6)
     crd::launch_dependents();
     __syncthreads();
     const ViewRegsT<false> vr(a);
+    const int W = a.u.width;
     const uint32_t total = a.counters[CNT_CHUNKS] * steps;
     for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
-        const uint32_t k = v / steps, local = (v - k * steps) * kStepPoints + threadIdx.x;
+        const uint32_t k = v / steps, local0 = (v - k * steps) * kStepPoints + threadIdx.x;
         ChunkRec c;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             reinterpret_cast<uint4 *>(&c)[q] = __ldg(reinterpret_cast<const uint4 *>(a.chunks + k) + q);
-        if (local >= c.count) continue;
-        PointOut o;
-        o.pointIndex = c.first + local;
-        o.color = 0u;
-        o.ok = true;
+        if (local0 >= c.count) continue;
+        const float *T = a.ifiles.n ? sT[c.file] : a.files[c.file].transform;
         const bool all_keep = (a.u.lodDither ? 1.0f : 0.5f) < (c.thr - 7.0f) + 0.5f;
-        const uint32_t lo = __ldg(a.low + o.pointIndex);
-        const uint32_t me = c.level <= 1 ? __ldg(a.med + o.pointIndex) : 0u;
-        const uint32_t hi = c.level == 0 ? __ldg(a.high + o.pointIndex) : 0u;
-        if (!all_keep) o.ok = keep_point(a, c, o.pointIndex, __ldg(a.levels + o.pointIndex));
-        project_point<PASS, false>(a, vr, a.ifiles.n ? sT[c.file] : a.files[c.file].transform, c,
-                                   lo, me, hi, o);
-        if (o.ok) emit_direct<PASS, false>(a, vr, o);
+        uint32_t lo[kStepEach], me[kStepEach], hi[kStepEach], lv[kStepEach];
+#pragma unroll
+        for (int j = 0; j < kStepEach; ++j) {
+            const uint32_t i = c.first + local0 + j * kThreads;
+            const bool in = local0 + j * kThreads < c.count;
+            lo[j] = in ? __ldg(a.low + i) : 0u;
+            me[j] = in && c.level <= 1 ? __ldg(a.med + i) : 0u;
+            hi[j] = in && c.level == 0 ? __ldg(a.high + i) : 0u;
+            lv[j] = in && !all_keep ? __ldg(a.levels + i) : 0u;
+        }
+        PointOut o[kStepEach];
+        uint32_t pix[kStepEach], closest[kStepEach];
+#pragma unroll
+        for (int j = 0; j < kStepEach; ++j) {
+            o[j].pointIndex = c.first + local0 + j * kThreads;
+            o[j].color = 0u;
+            o[j].ok = local0 + j * kThreads < c.count;
+            if (!all_keep) o[j].ok = o[j].ok && keep_point(a, c, o[j].pointIndex, lv[j]);
+            project_point<PASS, false>(a, vr, T, c, lo[j], me[j], hi[j], o[j]);
+            pix[j] = (uint32_t)(o[j].iy * W + o[j].ix);
+            if (PASS == PASS_DEPTH) {
+                if (o[j].ok) red_max_u32(a.t.depth + pix[j], o[j].depth);
+            } else {
+                closest[j] = o[j].ok ? __ldg(a.t.depth + pix[j]) : 0u;
+            }
+        }
+        if (PASS == PASS_DEPTH) continue;
+#pragma unroll
+        for (int j = 0; j < kStepEach; ++j) {
+            if (closest[j] == 0u ||
+                !(o[j].nz >= crd::uint_to_depth(closest[j]) * a.keep_scale))
+                continue;
+            if (PASS == PASS_COLOR_F32) {
+                color_f32_sample(a, pix[j], o[j].pointIndex);
+            } else {
+                float g[3] = {0.0f, 0.0f, 0.0f};
+                grad_sample(a, pix[j], g);
+                grad_store(a, o[j].pointIndex, g);
+            }
+        }
     }
 }
 

@@ -44,7 +44,7 @@ def test_nearest_frames_one_after_the_other(cr, orc, ctx, w, h):
 
 
 @pytest.mark.parametrize("chunk", [256, 300, 2048])
-@pytest.mark.parametrize("ppb", [255, 256, 257, 10240])
+@pytest.mark.parametrize("ppb", [255, 257, 511, 512, 513, 10240])
 def test_training_passes_at_step_edges(cr, orc, ctx, chunk, ppb):
     """The FP32 passes over batches and chunk records around their 256-point
     steps, with a chunk size set between the forward and the adjoint: the
