@@ -68,6 +68,7 @@ struct PackScratch {
     float4 *sorted = nullptr;               // positions in Morton order
     uint8_t *lv_morton = nullptr;           // levels in Morton order
     uint32_t *grid = nullptr;               // dense LOD occupancy grids
+    bool grid_empty = false;                // every voxel of all cap_grid is empty
     PackSeg *segs = nullptr;                // the segments of a run
     RadixSeg *rsegs = nullptr;              //   and what the sort needs of them
     RadixScratch radix;                     // the sort's look-back words and histograms

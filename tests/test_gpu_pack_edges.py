@@ -66,3 +66,22 @@ def test_refused_chunk_is_still_refused(cr, ctx):
     with pytest.raises(cr.CRError):
         cloud.addRawChunksGPU(cr.GPUPacker(ctx), [(pos, rgba), (bad, rgba)])
     assert cloud.residentBatchCount == 0
+
+
+def test_voxel_grids_between_runs(cr, orc):
+    """The LOD grids are cleared by the runs themselves: packs of one level, of
+    a single voxel, of coarse and fine grids and of chunks, one after the other
+    in one context, each as the CPU packs it."""
+    ctx = cr.Context(0)
+    runs = [(700, 1, 64, 1.0), (1, 2, 1, 1.0), (900, 2, 1, 1.0), (5000, 4, 9, 1.0),
+            (5000, 4, 64, 7.0), (300, 8, 2, 0.3), (5000, 3, 33, 2.0), (64, 4, 64, 1.0)]
+    for n, lod, divs, scale in runs + runs[::-1]:
+        pos, rgba = blob_cloud(n, n + lod + divs, scale=scale)
+        ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=512, lodLevels=lod,
+                       coarseVoxelDivisions=divs)
+        cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, ppb=512, lod=lod, divs=divs)
+        check_region(cloud, ref, 0, 512, src)
+        two = cr.ComputeRasteriserPointCloud(ctx, cr.ComputeRasteriserCapacity(30, 512))
+        packer = cr.GPUPacker(ctx, lodLevels=lod, coarseVoxelDivisions=divs)
+        for first in two.addRawChunksGPU(packer, [(pos, rgba), (pos, rgba)]):
+            check_region(two, ref, first, 512)
