@@ -34,6 +34,8 @@ struct RadixScratch {
     uint32_t *hist = nullptr;   // [segment][kRadixMaxPasses][256], filled by the caller
     uint32_t *bases = nullptr;  // the same shape
     uint32_t *runs = nullptr;   // per segment: bit p set = pass p runs
+    uint32_t *ties = nullptr;   // per segment: low key bits that no pass sorted
+    unsigned long long *sample = nullptr;  // radix_sample's tables and counts
     uint32_t *tiles = nullptr;
     uint32_t epoch = 0;
 };
@@ -45,12 +47,16 @@ uint32_t radix_tiles(uint32_t n);
 cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStream_t s);
 // Stable sort of every segment's keys by their low key_bits bits (the bits
 // above them are zero), with the keys' places in the segment as values.
-// segs is device memory.  A bounded wait that gives up stores kErrSortWait
-// into *status.
+// segs is device memory; n0: the keys of the first.  ties_ok: the passes over
+// the lowest digits of a single large segment of 64-bit keys may be left out;
+// keys that agree above the segment's tie bits (RadixScratch::ties) are then in
+// input order, and the caller orders them.  A bounded wait that gives up
+// stores kErrSortWait into *status.
+constexpr uint32_t kSampleMinKeys = 1u << 19;
 template <typename K>
 cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
-                     uint64_t ntiles, int key_bits, RadixScratch &rs, uint32_t *status,
-                     cudaStream_t s);
+                     uint64_t ntiles, uint32_t n0, int key_bits, bool ties_ok, RadixScratch &rs,
+                     uint32_t *status, cudaStream_t s);
 
 struct PackSeg;
 

@@ -303,12 +303,16 @@ __device__ __forceinline__ uint32_t lod_cell(const float4 &p, const LodArgs &a) 
 // and the assignment of level L also claims level L + 1 for the points it
 // leaves unassigned (each level has its own grid), so the points are read
 // once per level instead of twice.
+// MOVED: ties were put in order, so a lane's index may be below that of a lane
+// before it.
+template <bool MOVED>
 __device__ __forceinline__ void lod_claim_one(bool part, const float4 &p, uint32_t i,
                                               const LodArgs &a) {
     const unsigned act = __ballot_sync(0xffffffffu, part);
     if (!part) return;
     const uint32_t cell = lod_cell(p, a);
     const unsigned same = __match_any_sync(act, cell);
+    if (MOVED) i = __reduce_min_sync(same, i);
     if ((int)(__ffs(same) - 1) == (int)(threadIdx.x & 31u)) atomicMin(&a.grid[cell], i);
 }
 
@@ -328,40 +332,101 @@ __device__ __forceinline__ const uint32_t *sorted_index(const uint32_t *vals0,
 constexpr int kEach = 4;
 constexpr uint32_t kPointsPerCta = kEach * kThreads;
 
+// What the sort left in order (RadixBuffers, RadixScratch).  Where it left out
+// low digits (ties), the gather orders the keys that agree above them, and the
+// other values buffer holds the final indices.
+struct Sorted {
+    uint32_t *vals[2];
+    const unsigned long long *keys[2];  // 64-bit keys, else unused
+    const uint32_t *runs, *ties;
+    int want_index;  // the final indices are read (source indices asked for)
+};
+__device__ __forceinline__ const uint32_t *final_index(const Sorted &so, uint32_t si,
+                                                       uint64_t begin) {
+    const uint32_t set = so.runs[si];
+    if (so.ties[si] != 0u) return ((__popc(set) & 1) ? so.vals[0] : so.vals[1]) + begin;
+    return sorted_index(so.vals[0], so.vals[1], set, begin);
+}
+
+// Places of a CTA's keys among the keys that agree with them above `low` bits:
+// a key moves back by the keys before it with larger low bits and on by the
+// keys after it with smaller ones (equal keys keep their order).  The CTA's
+// keys are staged in shared memory; a run that leaves it is read on in place.
+__device__ __forceinline__ void tie_places(const unsigned long long *__restrict__ keys, uint32_t n,
+                                           uint64_t first, uint32_t low, unsigned long long *skey,
+                                           uint32_t (&place)[kEach]) {
+    const uint32_t count = (uint32_t)min((uint64_t)n - first, (uint64_t)kPointsPerCta);
+#pragma unroll
+    for (int k = 0; k < kEach; ++k) {
+        const uint32_t t = threadIdx.x + k * kThreads;
+        if (t < count) skey[t] = __ldg(keys + first + t);
+    }
+    __syncthreads();
+    auto key_at = [&](uint32_t i) {
+        const uint32_t t = i - (uint32_t)first;  // wraps below the CTA's keys
+        return t < count ? skey[t] : __ldg(keys + i);
+    };
+    const unsigned long long mask = (1ull << low) - 1ull;
+#pragma unroll
+    for (int k = 0; k < kEach; ++k) {
+        const uint32_t i = (uint32_t)first + threadIdx.x + k * kThreads;
+        place[k] = i;
+        if (threadIdx.x + k * kThreads >= count) continue;
+        const unsigned long long mine = skey[threadIdx.x + k * kThreads];
+        uint32_t at = i;
+        for (uint32_t j = i; j > 0u; --j) {
+            const unsigned long long other = key_at(j - 1u);
+            if ((other ^ mine) & ~mask) break;
+            at -= (other & mask) > (mine & mask) ? 1u : 0u;
+        }
+        for (uint32_t j = i + 1u; j < n; ++j) {
+            const unsigned long long other = key_at(j);
+            if ((other ^ mine) & ~mask) break;
+            at += (other & mask) < (mine & mask) ? 1u : 0u;
+        }
+        place[k] = at;
+    }
+}
+
 // Stage 4: gather into Morton order, all levels at max_level (packLODInit),
 // and the coarsest level's claims when there is more than one level.
 template <bool ONE>
 __global__ void __launch_bounds__(kThreads)
-    pack_gather_claim(const __grid_constant__ Segs segs, const uint32_t *__restrict__ vals0,
-                      const uint32_t *__restrict__ vals1, const uint32_t *__restrict__ runs,
+    pack_gather_claim(const __grid_constant__ Segs segs, const __grid_constant__ Sorted so,
                       float4 *__restrict__ sorted, uint8_t *__restrict__ lv, uint32_t max_level) {
+    __shared__ unsigned long long skey[ONE ? kPointsPerCta : 1];
     const uint32_t si = seg_of<ONE, &PackSeg::block0>(segs, blockIdx.x);
     const PackSeg &sg = seg_at<ONE>(segs, si);
     const uint64_t i0 = (uint64_t)(blockIdx.x - sg.block0) * kPointsPerCta + threadIdx.x;
-    const uint32_t *idx = sorted_index(vals0, vals1, runs[si], sg.begin);
+    const uint32_t set = so.runs[si];
+    const uint32_t *idx = sorted_index(so.vals[0], so.vals[1], set, sg.begin);
     const float4 *pos = sg.pos;
-    uint32_t from[kEach];
+    uint32_t from[kEach], place[kEach];
     float4 p[kEach];
 #pragma unroll
     for (int k = 0; k < kEach; ++k) {
         const uint64_t i = i0 + k * kThreads;
+        place[k] = (uint32_t)i;
         from[k] = i < sg.n && idx ? __ldg(idx + i) : (uint32_t)i;
     }
 #pragma unroll
     for (int k = 0; k < kEach; ++k)
         p[k] = i0 + k * kThreads < sg.n ? __ldg(pos + from[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t low = ONE ? so.ties[0] : 0u;  // only a single segment has any
+    if (ONE && low != 0u)
+        tie_places(so.keys[__popc(set) & 1], sg.n, i0 - threadIdx.x, low, skey, place);
 #pragma unroll
-    for (int k = 0; k < kEach; ++k) {
-        const uint64_t i = i0 + k * kThreads;
-        if (i < sg.n) {
-            sorted[sg.begin + i] = p[k];
-            lv[sg.begin + i] = (uint8_t)max_level;
+    for (int k = 0; k < kEach; ++k)
+        if (i0 + k * kThreads < sg.n) {
+            sorted[sg.begin + place[k]] = p[k];
+            lv[sg.begin + place[k]] = (uint8_t)max_level;
+            if (ONE && low != 0u && so.want_index)
+                ((__popc(set) & 1) ? so.vals[0] : so.vals[1])[place[k]] = from[k];
         }
-    }
     if (max_level > 0u)
 #pragma unroll
         for (int k = 0; k < kEach; ++k)
-            lod_claim_one(i0 + k * kThreads < sg.n, p[k], (uint32_t)(i0 + k * kThreads), sg.lod[0]);
+            lod_claim_one<ONE>(i0 + k * kThreads < sg.n, p[k], place[k], sg.lod[0]);
 }
 
 // The holder of a voxel sets it back to "empty" when it takes its level (every
@@ -403,7 +468,7 @@ __global__ void __launch_bounds__(kThreads)
     }
 #pragma unroll
     for (int k = 0; k < kEach; ++k)
-        lod_claim_one(left[k], p[k], (uint32_t)(i0 + k * kThreads), sg.lod[level + 1]);
+        lod_claim_one<false>(left[k], p[k], (uint32_t)(i0 + k * kThreads), sg.lod[level + 1]);
 }
 
 // Stages 6 and 7: per batch AABB, RasterBatch and stable level bucketing
@@ -428,8 +493,7 @@ template <int NL, bool ONE>
 __global__ void __launch_bounds__(kBatchThreads)
     pack_batches(const __grid_constant__ Segs segs, const float4 *__restrict__ sorted,
                  uint8_t *__restrict__ lv, uint32_t max_level, uint32_t ppb,
-                 const uint32_t *__restrict__ vals0, const uint32_t *__restrict__ vals1,
-                 const uint32_t *__restrict__ runs, cr_raster_batch *__restrict__ batches,
+                 const __grid_constant__ Sorted so, cr_raster_batch *__restrict__ batches,
                  uint32_t *__restrict__ low, uint32_t *__restrict__ med,
                  uint32_t *__restrict__ high, uint32_t *__restrict__ colors,
                  uint8_t *__restrict__ levels, uint32_t *__restrict__ src_out) {
@@ -559,7 +623,7 @@ __global__ void __launch_bounds__(kBatchThreads)
     }
     // 3. Stable bucketing of the warp's segment, each point quantised into
     // its final place.
-    const uint32_t *idx = src_out ? sorted_index(vals0, vals1, runs[si], sg.begin) : nullptr;
+    const uint32_t *idx = src_out ? final_index(so, si, sg.begin) : nullptr;
     for (uint32_t r0 = s0; r0 < s1; r0 += 32u * kBatchRounds) {
         float4 p[kBatchRounds];
         uint32_t raw[kBatchRounds];
@@ -880,25 +944,32 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
                                   {sc.idx[0], sc.idx[1]}};
         PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
                     (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
-        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, 63, sc.radix, ctx->d_status, s);
+        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, segs[0].n, 63, true, sc.radix,
+                           ctx->d_status, s);
     } else {
         using K = uint32_t;
         const RadixBuffers<K> buf{{static_cast<K *>(sc.keys[0]), static_cast<K *>(sc.keys[1])},
                                   {sc.idx[0], sc.idx[1]}};
         PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
                     (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
-        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, 30, sc.radix, ctx->d_status, s);
+        st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, segs[0].n, 30, false, sc.radix,
+                           ctx->d_status, s);
     }
     if (st) return st;
 
     // Stages 4-5: gather, LOD levels (each level its own dense grid).
+    const Sorted so{{sc.idx[0], sc.idx[1]},
+                    {static_cast<const unsigned long long *>(sc.keys[0]),
+                     static_cast<const unsigned long long *>(sc.keys[1])},
+                    sc.radix.runs,
+                    sc.radix.ties,
+                    src_idx_host ? 1 : 0};
     // The grids are empty but for a run that did not come to its end.
     if (!sc.grid_empty && cell_sum) CR_CUDA(cudaMemsetAsync(sc.grid, 0xff, sc.cap_grid * 4, s));
     const bool empty_after = sc.grid_empty || cell_sum > 0;
     sc.grid_empty = false;
     PACK_LAUNCH(nseg, (unsigned)blocks, kThreads, s, pack_gather_claim<true>,
-                pack_gather_claim<false>, arg, sc.idx[0], sc.idx[1], sc.radix.runs, sc.sorted,
-                sc.lv_morton, max_level);
+                pack_gather_claim<false>, arg, so, sc.sorted, sc.lv_morton, max_level);
     for (uint32_t level = 0; level + 1 < max_level; ++level)
         PACK_LAUNCH(nseg, (unsigned)blocks, kThreads, s, pack_lod_assign<true>,
                     pack_lod_assign<false>, arg, sc.sorted, sc.lv_morton, level, max_level);
@@ -908,13 +979,13 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
     uint32_t *src = src_idx_host ? sc.src_idx : nullptr;
     if (L <= 4)
         PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<4, true>),
-                    (pack_batches<4, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, sc.idx[0],
-                    sc.idx[1], sc.radix.runs, cloud->d_batches, cloud->d_low, cloud->d_med,
+                    (pack_batches<4, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, so,
+                    cloud->d_batches, cloud->d_low, cloud->d_med,
                     cloud->d_high, cloud->d_colors, cloud->d_levels, src);
     else
         PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<8, true>),
-                    (pack_batches<8, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, sc.idx[0],
-                    sc.idx[1], sc.radix.runs, cloud->d_batches, cloud->d_low, cloud->d_med,
+                    (pack_batches<8, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, so,
+                    cloud->d_batches, cloud->d_low, cloud->d_med,
                     cloud->d_high, cloud->d_colors, cloud->d_levels, src);
     sc.grid_empty = empty_after;
     if (src)

@@ -21,6 +21,13 @@
 //                     in shared memory and writes one coalesced run per
 //                     digit.  Equal keys keep their input order (stable), as
 //                     the CPU's stable sort does.
+// Low digits of a large sort (radix_sample).  The keys of a large cloud differ
+// mostly in their high digits, so the passes over the lowest digits only order
+// the few keys that agree in all others.  A sample of the keys estimates how
+// many agree, and when they are few those passes are left out: the segment's
+// tie word then says how many low bits were not sorted, and the reader of the
+// sorted keys orders each run of keys that agree above them (its cost grows
+// with the runs' lengths, which the sample bounds).
 // Nothing is read back: which of the two buffers a segment's pass reads
 // follows from the segment's set of digits (bit p: pass p runs), and so does
 // where its sorted keys and indices end up.
@@ -82,11 +89,58 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
     return x;
 }
 
-// A segment's digit bases and the set of its passes: one CTA per segment, a
-// thread per digit.
+// How many pairs of kSamples keys, drawn with replacement from all n, agree
+// above their low 24 (and 32) bits: a hash table of 39-bit (31-bit) values per
+// choice, each slot a value and the samples that had it.  n times the chance
+// that two keys agree is the mean length of the run that a key is in.
+constexpr uint32_t kSamples = 1u << 16;
+constexpr int kSampleSlotBits = 18;
+constexpr int kSampleChoices = 2;
+__global__ void __launch_bounds__(kThreads)
+    radix_sample(const unsigned long long *__restrict__ keys, uint32_t n,
+                 unsigned long long *__restrict__ table, unsigned long long *__restrict__ pairs) {
+    constexpr uint32_t kMask = (1u << kSampleSlotBits) - 1u;
+    const uint32_t s = blockIdx.x * kThreads + threadIdx.x;
+    uint32_t h = s * 0x9e3779b9u + 0x7f4a7c15u;  // a spread of the sample's number
+    h ^= h >> 16;
+    h *= 0x85ebca6bu;
+    h ^= h >> 13;
+    const unsigned long long key = keys[((unsigned long long)h * n) >> 32];
+#pragma unroll
+    for (int v = 0; v < kSampleChoices; ++v) {
+        const unsigned long long top = key >> (24 + 8 * v);  // 39 bits at most
+        unsigned long long *t = table + ((size_t)v << kSampleSlotBits);
+        uint32_t slot = (uint32_t)((top * 0x9e3779b97f4a7c15ull) >> 40);
+        uint32_t agree = 0;
+        for (int probe = 0; probe < 64; ++probe, ++slot) {
+            unsigned long long *w = t + (slot & kMask);
+            const unsigned long long old = atomicCAS(w, 0ull, (top << 20) | 1ull);
+            if (old == 0ull) break;
+            if (old >> 20 != top) continue;
+            agree = (uint32_t)(atomicAdd(w, 1ull) & 0xfffffull);
+            break;
+        }
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, agree);
+        if ((threadIdx.x & 31) == 0 && sum) atomicAdd(pairs + v, (unsigned long long)sum);
+    }
+}
+
+// Low passes to leave out given the sample: those whose bits separate runs of
+// at most kMaxMeanRun keys in the mean.
+constexpr unsigned long long kMaxMeanRun = 6;
+__device__ __forceinline__ uint32_t passes_left_out(const unsigned long long *pairs, uint32_t n) {
+    for (int v = kSampleChoices - 1; v >= 0; --v)
+        if (2ull * pairs[v] * n <= kMaxMeanRun * ((unsigned long long)kSamples * kSamples))
+            return 3u + (uint32_t)v;
+    return 0u;
+}
+
+// A segment's digit bases, the set of its passes and its tie word: one CTA per
+// segment, a thread per digit.  pairs: the sample (null: none was taken).
 __global__ void __launch_bounds__(kThreads)
     radix_bases(const uint32_t *__restrict__ hist, const RadixSeg *__restrict__ segs, int passes,
-                uint32_t *__restrict__ bases, uint32_t *__restrict__ runs) {
+                const unsigned long long *__restrict__ pairs, uint32_t *__restrict__ bases,
+                uint32_t *__restrict__ runs, uint32_t *__restrict__ ties) {
     __shared__ uint32_t sums[kRadixMaxPasses][kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n = segs[blockIdx.x].n;
@@ -111,7 +165,11 @@ __global__ void __launch_bounds__(kThreads)
             if (w < warp) base += sums[p][w];
         if (p < passes) bases[row + p * 256 + threadIdx.x] = base;
     }
-    if (threadIdx.x == 0) runs[blockIdx.x] = set;
+    if (threadIdx.x == 0) {
+        const uint32_t out = pairs ? passes_left_out(pairs, n) : 0u;
+        runs[blockIdx.x] = set & ~((1u << out) - 1u);
+        ties[blockIdx.x] = 8u * out;
+    }
 }
 
 template <typename K>
@@ -396,7 +454,7 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
 }  // namespace
 
 void radix_scratch_free(RadixScratch &r) {
-    void *ptrs[] = {r.lookback, r.hist, r.bases, r.runs, r.tiles};
+    void *ptrs[] = {r.lookback, r.hist, r.bases, r.runs, r.ties, r.tiles, r.sample};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     r = RadixScratch{};
@@ -416,6 +474,7 @@ cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStre
         CR_CUDA(cudaMalloc((void **)&rs.hist, rows * sizeof(uint32_t)));
         CR_CUDA(cudaMalloc((void **)&rs.bases, rows * sizeof(uint32_t)));
         CR_CUDA(cudaMalloc((void **)&rs.runs, segs * sizeof(uint32_t)));
+        CR_CUDA(cudaMalloc((void **)&rs.ties, segs * sizeof(uint32_t)));
         CR_CUDA(cudaMalloc((void **)&rs.tiles, kRadixMaxPasses * sizeof(uint32_t)));
         CR_CUDA(cudaMemsetAsync(rs.lookback, 0, tiles * 256 * sizeof(unsigned long long), s));
         rs.cap_tiles = tiles;
@@ -429,12 +488,27 @@ cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStre
 
 template <typename K>
 cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
-                     uint64_t ntiles, int key_bits, RadixScratch &rs, uint32_t *status,
-                     cudaStream_t s) {
+                     uint64_t ntiles, uint32_t n0, int key_bits, bool ties_ok, RadixScratch &rs,
+                     uint32_t *status, cudaStream_t s) {
     const int passes = (key_bits + 7) / 8;
     if (nseg == 0 || passes > kRadixMaxPasses || ntiles > rs.cap_tiles || nseg > rs.cap_segs)
         return cri::fail(CR_ERR_INTERNAL, "radix_sort: arguments");
-    radix_bases<<<nseg, kThreads, 0, s>>>(rs.hist, segs, passes, rs.bases, rs.runs);
+    // A sample is taken of one large segment of 64-bit keys: the passes left
+    // out then save more than the sample costs (15 us; at half a million keys
+    // two passes take that long).
+    const unsigned long long *pairs = nullptr;
+    if constexpr (sizeof(K) == 8) {
+        if (ties_ok && nseg == 1 && n0 >= kSampleMinKeys) {
+            const size_t words = ((size_t)kSampleChoices << kSampleSlotBits) + kSampleChoices;
+            if (!rs.sample) CR_CUDA(cudaMalloc((void **)&rs.sample, words * 8));
+            CR_CUDA(cudaMemsetAsync(rs.sample, 0, words * 8, s));
+            unsigned long long *found = rs.sample + ((size_t)kSampleChoices << kSampleSlotBits);
+            radix_sample<<<kSamples / kThreads, kThreads, 0, s>>>(buf.keys[0], n0, rs.sample, found);
+            CR_CUDA(cudaGetLastError());
+            pairs = found;
+        }
+    }
+    radix_bases<<<nseg, kThreads, 0, s>>>(rs.hist, segs, passes, pairs, rs.bases, rs.runs, rs.ties);
     CR_CUDA(cudaGetLastError());
     const size_t smem = onesweep_smem_bytes<K>();
     CR_CUDA(cudaFuncSetAttribute(radix_onesweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -455,7 +529,9 @@ cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t 
 }
 
 template cr_status radix_sort<uint32_t>(const RadixBuffers<uint32_t> &, const RadixSeg *, uint32_t,
-                                        uint64_t, int, RadixScratch &, uint32_t *, cudaStream_t);
+                                        uint64_t, uint32_t, int, bool, RadixScratch &, uint32_t *,
+                                        cudaStream_t);
 template cr_status radix_sort<unsigned long long>(const RadixBuffers<unsigned long long> &,
-                                                  const RadixSeg *, uint32_t, uint64_t, int,
-                                                  RadixScratch &, uint32_t *, cudaStream_t);
+                                                  const RadixSeg *, uint32_t, uint64_t, uint32_t,
+                                                  int, bool, RadixScratch &, uint32_t *,
+                                                  cudaStream_t);

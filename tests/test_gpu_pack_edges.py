@@ -1,5 +1,6 @@
 """The packer's kernels at the edges of their tiles, bit for bit against the
 CPU oracle's pack: whole numbers and bytes, so nothing is allowed for."""
+import numpy as np
 import pytest
 
 from scenes import blob_cloud
@@ -85,3 +86,28 @@ def test_voxel_grids_between_runs(cr, orc):
         packer = cr.GPUPacker(ctx, lodLevels=lod, coarseVoxelDivisions=divs)
         for first in two.addRawChunksGPU(packer, [(pos, rgba), (pos, rgba)]):
             check_region(two, ref, first, 512)
+
+
+@pytest.mark.parametrize("kind", ["spread", "ties", "crowded", "outlier"])
+@pytest.mark.parametrize("n", [(1 << 19) - 1, (1 << 19) + 4099])
+def test_low_digits_left_out(cr, orc, ctx, kind, n):
+    """63-bit keys around the size from which the sort samples them: spread
+    points (few agree above the low digits), points with runs that do (some
+    coincide, some differ in the last bits only, across the gather's CTAs),
+    points crowded into a few cells and a cloud shrunk by one far point (the
+    sample keeps every pass): the CPU pack's order each time."""
+    rng = np.random.default_rng(n + len(kind))
+    pos = rng.uniform(-1.0, 1.0, (n, 3)).astype(np.float32)
+    if kind == "ties":
+        pos[1000:1700] = pos[999]
+        pos[5000:9000:2] = pos[5001:9001:2]
+        pos[20000:26000] = pos[20000] + rng.uniform(-3e-5, 3e-5, (6000, 3)).astype(np.float32)
+    elif kind == "crowded":
+        pos = (pos[rng.integers(0, 50, n)] +
+               rng.uniform(-1e-4, 1e-4, (n, 3))).astype(np.float32)
+    elif kind == "outlier":
+        pos[7] = 5000.0
+    rgba = rng.integers(0, 1 << 32, n, dtype=np.uint32)
+    ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=10240, morton_bits=21, threads=8)
+    cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, bits=21)
+    check_region(cloud, ref, 0, 10240, src)
