@@ -570,11 +570,15 @@ cr_status launch_cull(cr_cloud *cloud, const CullUniforms &u, cudaStream_t s,
                cloud->d_visible,  cloud->d_chunks,
                cloud->d_counters, nullptr,
                (uint32_t)std::max(cloud->ctx->cull_spin_limit, 0), cloud->ctx->d_status};
-    // Half as many clear CTAs as SMs: the cull's few latency-bound CTAs then
-    // keep SMs of their own (with twice the SM count the cull took 33 µs
-    // instead of 26.5 µs on the 100M-point 1080p frames; a quarter is as
-    // fast, an eighth leaves the clear the longer part).
-    const uint32_t clear_ctas = clear ? std::max(1u, (uint32_t)cloud->ctx->sm_count / 2u) : 0u;
+    // A clear CTA for every SM without a cull CTA while those are few: the clear
+    // is then the longer part (10M points, 4 cull CTAs: 133 us a frame with half
+    // as many clear CTAs as SMs, 127 so; 1M points at 720p: 40.3 and 38.7; 20M
+    // points, 8 CTAs: 115.6 and 115.3).  Otherwise half as many as SMs, so that
+    // the latency-bound cull CTAs keep SMs of their own (100M points, 39 CTAs:
+    // 348.1 and 349.0 us).
+    const uint32_t sms = (uint32_t)cloud->ctx->sm_count;
+    const uint32_t clear_ctas =
+        !clear ? 0u : ctas <= sms / 16u ? sms - ctas : std::max(1u, sms / 2u);
     const InlineFiles ifl = inline_files(cloud);
     if (!ifl.n) {
         const cr_status st = ensure_device_files(cloud);
