@@ -519,7 +519,8 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
     project_point<PASS, MV>(a, vr, sb.T, c, lo, me, hi, o);
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
-    if (!a.radius_zero)
+    // Fragments are of single pixels (larger footprints take splat_depth).
+    if (PASS != PASS_DEPTH_FRAG && !a.radius_zero)
         emit_footprint<PASS, MV>(a, vr, sb, o);
     else if (tiled)
         emit_tile<PASS, MV>(a, vr, c, smem, o);
