@@ -86,6 +86,32 @@ struct TileCfg<PASS_GRAD> : TileCfg<PASS_COLOR_F32> {};
 __host__ __device__ constexpr bool is_depth(int p) { return p == PASS_DEPTH || p == PASS_DEPTH_FRAG; }
 __host__ __device__ constexpr bool is_color(int p) { return p == PASS_COLOR; }
 
+// Two floats in one 64-bit register pair.  Products and sums are fused
+// multiply-adds with an addend of -0 or a factor of 1, each rounded once, and
+// the two constants come from the kernel's parameters: as literals they are
+// folded away and the products and sums contracted, which rounds otherwise.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void split2(F2 a, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+struct F2Consts {
+    F2 one, minus_zero;
+    __device__ __forceinline__ F2 mul(F2 a, F2 b) const { return fma2(a, b, minus_zero); }
+    __device__ __forceinline__ F2 add(F2 a, F2 b) const { return fma2(a, one, b); }
+};
+
 struct RasterArgs {
     const ChunkRec *chunks;
     const cr_raster_file *files;
@@ -96,6 +122,7 @@ struct RasterArgs {
     RasterTargets t;
     RasterUniforms u;
     float keep_scale;  // 1 - depthTolerance
+    F2Consts two;      // 1 and -0, twice each
     int radius_zero;   // every footprint is a single pixel
     int use_tiles;
     uint32_t *frag_xy;  // pixel x | row << 16
@@ -213,6 +240,7 @@ __device__ __forceinline__ ViewRegsT<true> view_regs_mv() {
 
 struct BatchShared {
     float T[16];      // file.transform
+    F2 T2[16];        // its entries twice (two points at a time)
     float world[16];  // file.world (footprint only)
     uint32_t file;    // file cached in T / world
 };
@@ -235,17 +263,13 @@ __device__ __forceinline__ bool keep_point(const RasterArgs &a, const ChunkRec &
     return !(dither >= (c.thr - pointLevel) + 0.5f);
 }
 
-// decodePoint + projection + clip + pixel (DepthPass/Shaders.metal:188-211,
-// ColorPass/Shaders.metal:70-104, NearestDepth/Shaders.metal:68-85).
-template <int PASS, bool MV>
-__device__ __forceinline__ void project_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const float *T,
-                                              const ChunkRec &c, uint32_t lo, uint32_t me,
-                                              uint32_t hi, PointOut &o) {
-    // Split-precision decode: the coarse (low), medium and fine (high) 10-bit
-    // chunks for level >= 2 (10 bits), level 1 (20 bits) or level 0 (30
-    // bits).  A word the chunk's level does not use was never loaded and is
-    // zero; the level is the same for the whole chunk, so the branch is
-    // uniform and each level does only its own shifts.
+// Split-precision decode: the coarse (low), medium and fine (high) 10-bit
+// chunks for level >= 2 (10 bits), level 1 (20 bits) or level 0 (30 bits).  A
+// word the chunk's level does not use was never loaded and is zero; the level
+// is the same for the whole chunk, so the branch is uniform and each level
+// does only its own shifts.
+__device__ __forceinline__ void decode_words(const ChunkRec &c, uint32_t lo, uint32_t me,
+                                             uint32_t hi, float &fx, float &fy, float &fz) {
     uint32_t x, y, z;
     if (c.level >= 2) {
         x = lo & 1023u;
@@ -261,10 +285,16 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
         y = (((lo >> 10) & 1023u) << sl) | (((me >> 10) & 1023u) << sm) | ((hi >> 10) & 1023u);
         z = (((lo >> 20) & 1023u) << sl) | (((me >> 20) & 1023u) << sm) | ((hi >> 20) & 1023u);
     }
-    o.px = (float)x * c.qx + c.minX;
-    o.py = (float)y * c.qy + c.minY;
-    o.pz = (float)z * c.qz + c.minZ;
-    const crd::f4 clip = crd::mulp(T, o.px, o.py, o.pz);
+    fx = (float)x;
+    fy = (float)y;
+    fz = (float)z;
+}
+
+// Clip tests and pixel of a projected point (ColorPass/Shaders.metal:70-104,
+// NearestDepth/Shaders.metal:68-85).
+template <int PASS, bool MV>
+__device__ __forceinline__ void place_point(const RasterArgs &a, const ViewRegsT<MV> &vr,
+                                            const ChunkRec &c, const crd::f4 &clip, PointOut &o) {
     bool ok = o.ok;
     if (clip.w <= 0.0f) ok = false;
     const float nx = clip.x / clip.w, ny = clip.y / clip.w, nz = clip.z / clip.w;
@@ -287,6 +317,49 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
         else if (a.u.colorizeOverdraw)
             o.color = 0x00010101u;
     }
+}
+
+// decodePoint + projection + clip + pixel (DepthPass/Shaders.metal:188-211).
+template <int PASS, bool MV>
+__device__ __forceinline__ void project_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const float *T,
+                                              const ChunkRec &c, uint32_t lo, uint32_t me,
+                                              uint32_t hi, PointOut &o) {
+    float x, y, z;
+    decode_words(c, lo, me, hi, x, y, z);
+    o.px = x * c.qx + c.minX;
+    o.py = y * c.qy + c.minY;
+    o.pz = z * c.qz + c.minZ;
+    place_point<PASS, MV>(a, vr, c, crd::mulp(T, o.px, o.py, o.pz), o);
+}
+
+// project_point of two points.  T2: the transform with every entry twice.  The
+// decode's and the transform's 60 products and sums are 30 instructions, of
+// which the passes, bound by instruction issue, have one in seven fewer: 100M
+// points at 1080p 335 -> 328 us a frame, 64 views 8.45 -> 8.24 ms.
+template <int PASS, bool MV>
+__device__ __forceinline__ void project_pair(const RasterArgs &a, const ViewRegsT<MV> &vr,
+                                             const F2 *T2, const ChunkRec &c, const uint32_t *lo,
+                                             const uint32_t *me, const uint32_t *hi, PointOut &o0,
+                                             PointOut &o1) {
+    float x0, y0, z0, x1, y1, z1;
+    decode_words(c, lo[0], me[0], hi[0], x0, y0, z0);
+    decode_words(c, lo[1], me[1], hi[1], x1, y1, z1);
+    const F2Consts &k = a.two;
+    const F2 x = k.add(k.mul(f2(x0, x1), f2(c.qx, c.qx)), f2(c.minX, c.minX));
+    const F2 y = k.add(k.mul(f2(y0, y1), f2(c.qy, c.qy)), f2(c.minY, c.minY));
+    const F2 z = k.add(k.mul(f2(z0, z1), f2(c.qz, c.qz)), f2(c.minZ, c.minZ));
+    auto row = [&](int r, float &v0, float &v1) {
+        split2(k.add(k.add(k.add(k.mul(T2[r], x), k.mul(T2[4 + r], y)), k.mul(T2[8 + r], z)),
+                     T2[12 + r]),
+               v0, v1);
+    };
+    crd::f4 p0, p1;
+    row(0, p0.x, p1.x);
+    row(1, p0.y, p1.y);
+    row(2, p0.z, p1.z);
+    row(3, p0.w, p1.w);
+    place_point<PASS, MV>(a, vr, c, p0, o0);
+    place_point<PASS, MV>(a, vr, c, p1, o1);
 }
 
 __device__ __forceinline__ unsigned long long nearest_key(uint32_t depth, uint32_t index) {
@@ -502,7 +575,7 @@ __device__ __forceinline__ uint32_t emit_fragment(const RasterArgs &a, uint32_t 
 
 // One point; every lane of the warp calls this (warp-uniform early outs).
 // frag_at: the depth pass's next fragment, advanced by the points it kept.
-template <int PASS, bool MV>
+template <int PASS, bool MV, bool FP>
 __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV> &vr, const BatchShared &sb,
                                          unsigned char *smem, const ChunkRec &c, bool tiled,
                                          bool valid, uint32_t local, uint32_t lvl, uint32_t lo,
@@ -519,8 +592,7 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
     project_point<PASS, MV>(a, vr, sb.T, c, lo, me, hi, o);
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
-    // Fragments are of single pixels (larger footprints take splat_depth).
-    if (PASS != PASS_DEPTH_FRAG && !a.radius_zero)
+    if (FP && !a.radius_zero)
         emit_footprint<PASS, MV>(a, vr, sb, o);
     else if (tiled)
         emit_tile<PASS, MV>(a, vr, c, smem, o);
@@ -612,7 +684,10 @@ __device__ __forceinline__ uint32_t find_view(const uint32_t *begin, uint32_t nv
 // all views form one index space, view after view; each CTA scans the
 // per-view chunk counts once, finds a chunk's view by binary search and
 // switches frame, camera and file table when the view changes.
-template <int PASS, bool MV>
+// FP: footprints may be larger than a pixel.  Without them (fragments are of
+// single pixels; the nearest pass when its points are) the generic footprint
+// code stays out, and two points are projected at a time.
+template <int PASS, bool MV, bool FP>
 __device__ __forceinline__ void raster_body(const RasterArgs &a) {
     constexpr bool kFrag = PASS == PASS_DEPTH_FRAG;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -741,7 +816,11 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 // parameter, so the inline table is read in place.
                 const cr_raster_file *file = &(a.ifiles.n ? a.ifiles.f : a.files)[file_id];
                 if (threadIdx.x < 16)
-                    sb.T[threadIdx.x] = file->transform[threadIdx.x];
+                {
+                    const float t = file->transform[threadIdx.x];
+                    sb.T[threadIdx.x] = t;
+                    sb.T2[threadIdx.x] = f2(t, t);
+                }
                 else if (threadIdx.x < 32)
                     sb.world[threadIdx.x - 16] = file->world[threadIdx.x - 16];
                 if (threadIdx.x == 0) sb.file = file_id;
@@ -788,9 +867,6 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         uint32_t frag_at = frag0;
         if ((c.first & 3u) == 0u) {
             // Four points per thread, 16-byte loads.
-            // (Counted in quads without pieces: the nearest pass then takes 48
-            // registers instead of 60, five CTAs an SM instead of four, and 208
-            // instead of 219 us for 100M points at 1080p.)
             const uint32_t nquads = (c.count + 3u) >> 2;
             for (uint32_t p0 = kPieces ? piece : 0u; kPieces ? p0 < end : p0 < nquads;
                  p0 += kPieces ? 128u : kThreads) {
@@ -813,10 +889,37 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 const uint32_t mes[4] = {me4.x, me4.y, me4.z, me4.w};
                 const uint32_t his[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
                 const uint32_t cos[4] = {co4.x, co4.y, co4.z, co4.w};
+                if constexpr (!FP) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    do_point<PASS, MV>(a, vr, sb, smem, c, tiled, l0 + j < end, l0 + j, lvs[j],
-                                       los[j], mes[j], his[j], cos[j], frag_at, emit, all_keep);
+                    for (int j = 0; j < 4; j += 2) {
+                        PointOut o[2];
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            o[q].pointIndex = c.first + l0 + j + q;
+                            o[q].color = cos[j + q];
+                            o[q].ok = l0 + j + q < end;
+                            if (!all_keep)
+                                o[q].ok = o[q].ok && keep_point(a, c, o[q].pointIndex, lvs[j + q]);
+                        }
+                        project_pair<PASS, MV>(a, vr, sb.T2, c, los + j, mes + j, his + j, o[0],
+                                               o[1]);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            if (tiled)
+                                emit_tile<PASS, MV>(a, vr, c, smem, o[q]);
+                            else
+                                emit_direct<PASS, MV>(a, vr, o[q]);
+                            if (PASS == PASS_DEPTH_FRAG && emit)
+                                frag_at += emit_fragment(a, frag_at, o[q]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        do_point<PASS, MV, FP>(a, vr, sb, smem, c, tiled, l0 + j < end, l0 + j, lvs[j],
+                                           los[j], mes[j], his[j], cos[j], frag_at, emit,
+                                           all_keep);
+                }
             }
         } else {
             // Unaligned start (pointsPerBatch not a multiple of 4): one point per thread.
@@ -830,7 +933,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 const uint32_t me = (v && need_med) ? a.med[i] : 0u;
                 const uint32_t hi = (v && need_high) ? a.high[i] : 0u;
                 const uint32_t co = (v && kNeedColor) ? a.colors[i] : 0u;
-                do_point<PASS, MV>(a, vr, sb, smem, c, tiled, v, local, lv, lo, me, hi, co,
+                do_point<PASS, MV, FP>(a, vr, sb, smem, c, tiled, v, local, lv, lo, me, hi, co,
                                    frag_at, emit, all_keep);
             }
         }
@@ -1475,7 +1578,15 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
 
 template <int PASS, bool MV>
 __global__ void __launch_bounds__(kThreads) raster_kernel(const __grid_constant__ RasterArgs a) {
-    raster_body<PASS, MV>(a);
+    raster_body<PASS, MV, true>(a);
+}
+
+// The nearest pass of single-pixel points, at five CTAs per SM (48 registers, a
+// few spilled): 100M points at 1080p 207 us with the generic footprint code,
+// 195 so, 204 at four; 206 at five with one point at a time.
+__global__ void __launch_bounds__(kThreads, 5)
+    nearest_kernel(const __grid_constant__ RasterArgs a) {
+    raster_body<PASS_NEAREST, false, false>(a);
 }
 
 // The differentiable passes of one view with single-pixel footprints (depth
@@ -1560,7 +1671,7 @@ __global__ void __launch_bounds__(kThreads, 6)
 // (and their 32 KB screen tiles) share an SM.
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 4) depth_kernel(const __grid_constant__ RasterArgs a) {
-    raster_body<PASS, false>(a);
+    raster_body<PASS, false, PASS != PASS_DEPTH_FRAG>(a);
 }
 
 // The batched-view depth passes at five CTAs per SM (48 registers, a dozen
@@ -1569,7 +1680,7 @@ __global__ void __launch_bounds__(kThreads, 4) depth_kernel(const __grid_constan
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 5)
     depth_views_kernel(const __grid_constant__ RasterArgs a) {
-    raster_body<PASS, true>(a);
+    raster_body<PASS, true, PASS != PASS_DEPTH_FRAG>(a);
 }
 
 // The colour pass that decodes the points holds a 64 KB screen tile, so at
@@ -1577,13 +1688,13 @@ __global__ void __launch_bounds__(kThreads, 5)
 // compiler use up to 85 registers per thread instead of spilling.
 template <bool MV>
 __global__ void __launch_bounds__(kThreads, 3) raster_kernel_color(const __grid_constant__ RasterArgs a) {
-    raster_body<PASS_COLOR, MV>(a);
+    raster_body<PASS_COLOR, MV, true>(a);
 }
 
 // Colour pass of batched views whose fragments overflowed the arena: the
 // decode-and-project pass (color_hash_views_kernel draws the others).
 __global__ void __launch_bounds__(kThreads, 3) color_views_kernel(const __grid_constant__ RasterArgs a) {
-    if (*a.frag_overflow) raster_body<PASS_COLOR, true>(a);
+    if (*a.frag_overflow) raster_body<PASS_COLOR, true, true>(a);
 }
 
 // The kernel a pass launches.
@@ -1674,6 +1785,7 @@ RasterArgs make_args(cr_cloud *cloud, const RasterUniforms &u, const RasterTarge
     a.t = t;
     a.u = u;
     a.keep_scale = 1.0f - u.depthTolerance;
+    a.two = F2Consts{F2{0x3f8000003f800000ull}, F2{0x8000000080000000ull}};
     // pointFootprintRadius clamps the size to [lo, hi] with lo >= 1; when the
     // upper bound is 1 every radius is 0 whatever the distance.
     a.radius_zero = fmaxf(u.minimumPointSize, u.maximumPointSize) <= 1.0f ? 1 : 0;
@@ -1728,7 +1840,18 @@ cr_status launch_raster(cr_cloud *cloud, RasterPass pass, const RasterUniforms &
     case PASS_COLOR_FRAG:
         CR_CUDA(launch_programmatic(color_hash_kernel, dim3(grid), dim3(kThreads), 0, s, a));
         break;
-    default: launch_pass<PASS_NEAREST, false>(a, grid, s); break;
+    default:
+        if (a.radius_zero) {
+            constexpr int kBytes = TileCfg<PASS_NEAREST>::kBytes;
+            if (ctx->blocks_per_sm_nearest == 0)
+                ctx->blocks_per_sm_nearest = resident_blocks(nearest_kernel, kBytes);
+            CR_CUDA(launch_programmatic(nearest_kernel,
+                                        dim3(ctx->sm_count * ctx->blocks_per_sm_nearest),
+                                        dim3(kThreads), (size_t)kBytes, s, a));
+        } else {
+            launch_pass<PASS_NEAREST, false>(a, grid, s);
+        }
+        break;
     }
     CR_CUDA(cudaGetLastError());
     return CR_OK;
