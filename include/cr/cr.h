@@ -550,8 +550,8 @@ CR_API cr_status cr_context_pass_times(cr_context *ctx, int32_t nframes, float *
 /* ------------------------------------------------------------------------ */
 /* Launch tuning of the point passes                                         */
 /* ------------------------------------------------------------------------ */
-/* chunkPoints: survivor points per work record of the depth / colour /
- * nearest passes (>= 256); useTiles: accumulate compact batches in
+/* chunkPoints: most survivor points per work record of the depth / colour /
+ * nearest passes (>= 256; a small cloud's records have fewer); useTiles: accumulate compact batches in
  * shared-memory screen tiles.  Results do not depend on either value. */
 typedef struct cr_tuning {
     int32_t chunkPoints;     /* default 2048 */

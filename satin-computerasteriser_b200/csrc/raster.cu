@@ -1297,7 +1297,7 @@ __device__ __forceinline__ void splat_finish(const RasterArgs &a) {
 }
 
 __global__ void __launch_bounds__(kThreads, 4)
-    splat_depth(const __grid_constant__ RasterArgs a, uint32_t steps) {
+    splat_depth(const __grid_constant__ RasterArgs a, uint32_t steps, uint32_t most) {
     __shared__ uint32_t tile[kSplatPx];
     __shared__ SplatShared ss;
     __shared__ __align__(16) float sfile[kInlineFiles][32];  // transform, world
@@ -1312,7 +1312,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     const crd::PointSize ps{a.u.pointSizeMode, a.u.minimumPointSize, a.u.maximumPointSize,
                             a.u.pointSizeScale};
     const int lane = threadIdx.x & 31;
-    const uint32_t total = a.counters[CNT_CHUNKS] * steps;
+    const uint32_t total = min(a.counters[CNT_CHUNKS] * steps, most);
     uint32_t *cursor = a.counters + CNT_WORK_DEPTH;
     if (threadIdx.x == 0) {
         ss.next = atomicAdd(cursor, 1u);
@@ -1419,7 +1419,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 // keep every field below its width) and the pixels' visibility thresholds.
 constexpr int kSplatColorBytes = kSplatPx * 16;
 __global__ void __launch_bounds__(kThreads, 5)
-    splat_color(const __grid_constant__ RasterArgs a, uint32_t steps) {
+    splat_color(const __grid_constant__ RasterArgs a, uint32_t steps, uint32_t most) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t *acc = reinterpret_cast<uint32_t *>(smem);
     float *thr = reinterpret_cast<float *>(acc + 3 * kSplatPx);
@@ -1428,7 +1428,7 @@ __global__ void __launch_bounds__(kThreads, 5)
     crd::launch_dependents();
     const ViewRegsT<false> vr(a);
     const int W = a.u.width, H = a.u.height;
-    const uint32_t total = a.counters[CNT_CHUNKS] * steps;
+    const uint32_t total = min(a.counters[CNT_CHUNKS] * steps, most);
     uint32_t *cursor = a.counters + CNT_WORK_DEPTH;
     if (threadIdx.x == 0) {
         ss.next = atomicAdd(cursor, 1u);
@@ -1534,6 +1534,7 @@ struct RedoArgs {
     uint32_t npix;
     ResolveUniforms ru;
     uint32_t splat_steps[kRedoMaxClouds];  // splats: steps per chunk record; 0: single pixels
+    uint32_t splat_most[kRedoMaxClouds];   // and their bound
 };
 
 __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
@@ -1555,7 +1556,8 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
         const uint32_t nchunks = r.clouds[ci].counters[CNT_CHUNKS];
         const uint32_t steps = r.splat_steps[ci];
         if (steps) {
-            for (uint32_t v = 0; v < nchunks * steps; ++v) {
+            const uint32_t total = min(nchunks * steps, r.splat_most[ci]);
+            for (uint32_t v = 0; v < total; ++v) {
                 const uint32_t k = v / steps;
                 const uint32_t base = a.chunks[k].first + (v - k * steps) * kSplatPoints;
                 for (uint32_t f = threadIdx.x; f < a.frag_count[v]; f += kThreads)
@@ -1813,6 +1815,11 @@ uint32_t splat_steps(const cr_cloud *cloud) {
     const uint32_t most = std::min(cloud->cull_chunk_points, cloud->cap.pointsPerBatch);
     return (most + kSplatPoints - 1) / kSplatPoints;
 }
+// The room itself, for the records of a replayed capture whose cull had another
+// chunk size than the cloud's last one.
+uint32_t splat_most(const cr_cloud *cloud) {
+    return (uint32_t)std::min<uint64_t>(cloud->chunk_cap * kFragCounts, 0xffffffffu);
+}
 
 // One-view passes start while the previous kernel drains (programmatic
 // dependent launch); batched views, captured in a graph, launch plainly.
@@ -1864,18 +1871,18 @@ cr_status launch_splats(cr_cloud *cloud, bool color, const RasterUniforms &u,
         const cr_status st = ensure_device_files(cloud);
         if (st) return st;
     }
-    const uint32_t steps = splat_steps(cloud);
+    const uint32_t steps = splat_steps(cloud), most = splat_most(cloud);
     cr_context *ctx = cloud->ctx;
     if (color) {
         if (ctx->blocks_per_sm_splat[1] == 0)
             ctx->blocks_per_sm_splat[1] = resident_blocks(splat_color, kSplatColorBytes);
         CR_CUDA(launch_programmatic(splat_color, dim3(ctx->sm_count * ctx->blocks_per_sm_splat[1]),
-                                    dim3(kThreads), (size_t)kSplatColorBytes, s, a, steps));
+                                    dim3(kThreads), (size_t)kSplatColorBytes, s, a, steps, most));
     } else {
         if (ctx->blocks_per_sm_splat[0] == 0)
             ctx->blocks_per_sm_splat[0] = resident_blocks(splat_depth, 0);
         CR_CUDA(launch_programmatic(splat_depth, dim3(ctx->sm_count * ctx->blocks_per_sm_splat[0]),
-                                    dim3(kThreads), 0, s, a, steps));
+                                    dim3(kThreads), 0, s, a, steps, most));
     }
     return CR_OK;
 }
@@ -1892,6 +1899,7 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
         r.clouds[i] = RedoCloud{clouds[i]->d_chunks,   clouds[i]->d_counters, clouds[i]->d_frag_count,
                                 clouds[i]->d_frag_xy, clouds[i]->d_frag_zc};
         r.splat_steps[i] = splats ? splat_steps(clouds[i]) : 0u;
+        r.splat_most[i] = splat_most(clouds[i]);
     }
     r.nclouds = nclouds;
     r.redo = t.redo;
@@ -1906,8 +1914,8 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
 
 uint32_t hqs_redo_max_clouds() { return kRedoMaxClouds; }
 
-// A step to a CTA while there are CTAs.  The chunk records are those of the
-// cloud's last cull, at the chunk size it was launched with.
+// A step to a CTA while there are CTAs.  No chunk record of the cloud's last
+// cull has more than chunk_points points.
 template <int PASS>
 cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, uint32_t chunk_points,
                               cudaStream_t s) {

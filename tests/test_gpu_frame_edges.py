@@ -46,7 +46,7 @@ def test_nearest_frames_one_after_the_other(cr, orc, ctx, w, h):
 @pytest.mark.parametrize("chunk", [256, 300, 2048])
 @pytest.mark.parametrize("ppb", [255, 257, 511, 512, 513, 10240])
 def test_training_passes_at_step_edges(cr, orc, ctx, chunk, ppb):
-    """The FP32 passes over batches and chunk records around their 256-point
+    """The FP32 passes over batches and chunk records around their 512-point
     steps, with a chunk size set between the forward and the adjoint: the
     image is the mean of the visible points' colours and the gradient of an
     image gradient of ones is 1 / count per visible pixel.  Every visible
@@ -203,3 +203,26 @@ def test_pick_window(cr, orc, ctx, radius):
         best = np.lexsort((xs, ys, d))[0]
         want = int(plane[ys[best], xs[best]]) if d[best] <= radius * radius else None
         assert ras.pickPointIndex((nx, ny), cloud, cam, searchRadius=radius) == want
+
+
+@pytest.mark.parametrize("chunk", [512, 2048, 4096])
+@pytest.mark.parametrize("batches", [147, 148, 149])
+def test_record_size_of_small_clouds(cr, orc, ctx, chunk, batches):
+    """Frames of both modes, of single pixels and of footprints, on either side
+    of the pool size at which the cull's records change theirs (148 batches of
+    10,240 points on 148 SMs), next to a cloud of small batches."""
+    small, _ = make_cloud(cr, orc, ctx, *blob_cloud(900, 5), ppb=40)
+    cloud, _ = make_cloud(cr, orc, ctx, *blob_cloud(batches * 10240, 6))
+    assert cloud.residentBatchCount == batches
+    w, h = 97, 61
+    cam = camera(cr, (0.2, 0.1, 1.6), w=w, h=h)
+    before = ctx.tuning()["chunkPoints"]
+    try:
+        ctx.set_tuning(chunkPoints=chunk)
+        for mode, most in ((cr.MODE_HQS, 1.0), (cr.MODE_HQS, 3.0), (cr.MODE_NEAREST, 1.0)):
+            cfg = cr.ComputeRasteriserConfiguration(mode=mode, enableCLOD=False,
+                                                    maximumPointSize=most)
+            _, gpu, ref = render_both(cr, orc, ctx, [small, cloud], cfg, cam, w, h)
+            assert_same(cr, cfg, gpu, ref)
+    finally:
+        ctx.set_tuning(chunkPoints=before)
