@@ -332,13 +332,19 @@ __device__ __forceinline__ void project_point(const RasterArgs &a, const ViewReg
     place_point<PASS, MV>(a, vr, c, crd::mulp(T, o.px, o.py, o.pz), o);
 }
 
+// A transform's entries, each twice.
+struct Twice {
+    const float *T;
+    __device__ __forceinline__ F2 operator[](int i) const { return f2(T[i], T[i]); }
+};
+
 // project_point of two points.  T2: the transform with every entry twice.  The
 // decode's and the transform's 60 products and sums are 30 instructions, of
 // which the passes, bound by instruction issue, have one in seven fewer: 100M
 // points at 1080p 335 -> 328 us a frame, 64 views 8.45 -> 8.24 ms.
-template <int PASS, bool MV>
+template <int PASS, bool MV, class M>
 __device__ __forceinline__ void project_pair(const RasterArgs &a, const ViewRegsT<MV> &vr,
-                                             const F2 *T2, const ChunkRec &c, const uint32_t *lo,
+                                             const M T2, const ChunkRec &c, const uint32_t *lo,
                                              const uint32_t *me, const uint32_t *hi, PointOut &o0,
                                              PointOut &o1) {
     float x0, y0, z0, x1, y1, z1;
@@ -901,8 +907,8 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                             if (!all_keep)
                                 o[q].ok = o[q].ok && keep_point(a, c, o[q].pointIndex, lvs[j + q]);
                         }
-                        project_pair<PASS, MV>(a, vr, sb.T2, c, los + j, mes + j, his + j, o[0],
-                                               o[1]);
+                        project_pair<PASS, MV, const F2 *>(a, vr, sb.T2, c, los + j, mes + j,
+                                                           his + j, o[0], o[1]);
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             if (tiled)
@@ -1601,8 +1607,9 @@ __global__ void __launch_bounds__(kThreads, 5)
 // over every warp slot, and a thread's two points wait together.  10M points,
 // 512 x 512, 16 views: the step 1.80 ms with the four-point passes, 1.17 with a
 // point a thread (six CTAs an SM; 1.14 with eight), 1.12 with two (1.14 with
-// five CTAs), 1.19 with four.
+// five CTAs), 1.19 with four; 1.10 with the two in the same instructions.
 constexpr int kStepEach = 2;  // points per thread and step
+static_assert(kStepEach % 2 == 0, "points are projected in pairs");
 constexpr int kStepPoints = kStepEach * kThreads;
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 6)
@@ -1644,7 +1651,12 @@ __global__ void __launch_bounds__(kThreads, 6)
             o[j].color = 0u;
             o[j].ok = local0 + j * kThreads < c.count;
             if (!all_keep) o[j].ok = o[j].ok && keep_point(a, c, o[j].pointIndex, lv[j]);
-            project_point<PASS, false>(a, vr, T, c, lo[j], me[j], hi[j], o[j]);
+            if (j & 1)
+                project_pair<PASS, false>(a, vr, Twice{T}, c, lo + j - 1, me + j - 1, hi + j - 1,
+                                          o[j - 1], o[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kStepEach; ++j) {
             pix[j] = (uint32_t)(o[j].iy * W + o[j].ix);
             if (PASS == PASS_DEPTH) {
                 if (o[j].ok) red_max_u32(a.t.depth + pix[j], o[j].depth);
