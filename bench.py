@@ -619,11 +619,13 @@ def run_ours(args, dist):
            "config": config_dict(args), "e2e": e2e, "roofline": roofline, "clocks": clocks,
            # HQS: the cull (whose trailing CTAs clear the frame), depth,
            # colour, resolve, and the exact re-run, which returns at once
-           # unless a pixel passed 16,843,009 samples.  A frame split by
-           # points has no re-run (its colour adds are unpacked) but two
-           # depth-order flips.  Nearest: cull, nearest pass, resolve.
+           # unless a pixel passed 16,843,009 samples (a cloud of no more points
+           # has none launched).  A frame split by points has no re-run (its
+           # colour adds are unpacked) but two depth-order flips.  Nearest:
+           # cull, nearest pass, resolve.
            "gpu_launches": int(args.steps * (
-               (6 if args.shard == "points" else 5) if args.mode == "hqs" else 3)),
+               3 if args.mode != "hqs" else 6 if args.shard == "points"
+               else 5 if -(-args.points // 10240) * 10240 > 16_843_009 else 4)),
            "pass_ms": {n: round(float(v), 4) for n, v in zip(PASS_NAMES, avg)},
            "survivor_points_per_frame": int(active.mean()),
            "survivors_by_pose": {int(p): int(pose_bytes[p][2]) for p in sorted(pose_bytes)},
@@ -1019,7 +1021,9 @@ def run_packer(args, cr, ctx, torch, dist):
     cloud.close()
     ctx.trim()
     bit_exact = pack_parity(args, cr, ctx) if args.pack_check_points > 0 else None
-    # Algorithmic bytes per point (63-bit keys, 4 LOD levels): 8 radix passes
+    # Bytes per point of a pack that sorts every digit (63-bit keys, 4 LOD
+    # levels; a yardstick: the packer leaves out digits that all keys share
+    # and low ones that few keys need, and moves fewer): 8 radix passes
     # moving a 64-bit key and a 32-bit index in and out (192 B), the gather
     # (16 B in, 12 B of sorted position out), 3 LOD levels (12 B each), the
     # quantisation (12 B in, 12 B out) and the colour (4 B): 284 B.
@@ -1029,6 +1033,7 @@ def run_packer(args, cr, ctx, torch, dist):
     return {"points": n, "morton_bits": 63, "batches": int(len(res)),
             "pack_ms": round(ms, 2), "gpts_per_s": round(n / (ms / 1e3) / 1e9, 3),
             "roofline": {"bound": "hbm", "bytes_per_point": bpp,
+                         "bytes_model": "a pack that sorts all eight digits",
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "peak_source": peak_kind},
             "checks": checks, "bit_exact": bit_exact,
