@@ -6,11 +6,11 @@
 // reference appends survivors with an atomic counter, so its list order is
 // unspecified; here the list is in ascending slot order (deterministic and
 // comparable to the CPU oracle):
-//   1. cull_classify: one thread per slot; each 256-slot CTA compacts its
+//   1. classify: one thread per slot; each 256-slot CTA compacts its
 //      survivors in order with warp ballots, adds the per-batch values the
 //      point passes need (decode steps, screen rectangle), and writes its
 //      survivor and chunk counts.
-//   2. cull_compact: each CTA sums the counts of the CTAs before it, copies
+//   2. compact: each CTA sums the counts of the CTAs before it, copies
 //      its survivors to that offset and writes one chunk record per
 //      `chunkPoints` survivor points; the last CTA publishes the totals (the
 //      CUDA counterpart of the indirect argument buffer).
@@ -519,9 +519,6 @@ __global__ void __launch_bounds__(kCullThreads)
         }
     }
 }
-
-__global__ void __launch_bounds__(kCullThreads) cull_classify(CullArgs a) { classify_body(a); }
-__global__ void __launch_bounds__(kCullThreads) cull_compact(CullArgs a) { compact_body(a); }
 
 // Batched views: blockIdx.y selects the view's arguments (its uniforms, file
 // table and output ranges); the slots and the point pool are shared.

@@ -1664,18 +1664,19 @@ __global__ void __launch_bounds__(kThreads, 6)
                 closest[j] = o[j].ok ? __ldg(a.t.depth + pix[j]) : 0u;
             }
         }
-        if (PASS == PASS_DEPTH) continue;
+        if constexpr (PASS != PASS_DEPTH) {
 #pragma unroll
-        for (int j = 0; j < kStepEach; ++j) {
-            if (closest[j] == 0u ||
-                !(o[j].nz >= crd::uint_to_depth(closest[j]) * a.keep_scale))
-                continue;
-            if (PASS == PASS_COLOR_F32) {
-                color_f32_sample(a, pix[j], o[j].pointIndex);
-            } else {
-                float g[3] = {0.0f, 0.0f, 0.0f};
-                grad_sample(a, pix[j], g);
-                grad_store(a, o[j].pointIndex, g);
+            for (int j = 0; j < kStepEach; ++j) {
+                if (closest[j] == 0u ||
+                    !(o[j].nz >= crd::uint_to_depth(closest[j]) * a.keep_scale))
+                    continue;
+                if (PASS == PASS_COLOR_F32) {
+                    color_f32_sample(a, pix[j], o[j].pointIndex);
+                } else {
+                    float g[3] = {0.0f, 0.0f, 0.0f};
+                    grad_sample(a, pix[j], g);
+                    grad_store(a, o[j].pointIndex, g);
+                }
             }
         }
     }
