@@ -26,6 +26,9 @@ cr_status fail(cr_status st, const std::string &detail) {
 
 cr_status cuda_fail(cudaError_t e, const char *what) {
     g_detail = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
+    // Reported here: a failed allocation must not be found again by the check
+    // after the next launch (errors of the context itself stay).
+    cudaGetLastError();
     if (e == cudaErrorMemoryAllocation) return CR_ERR_OUT_OF_MEMORY;
     if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver ||
         e == cudaErrorInvalidDevice)
@@ -888,8 +891,7 @@ CR_API cr_status cr_frame_destroy(cr_frame *f) {
     dfree(f->d_rgba[0]);
     dfree(f->d_rgba[1]);
     dfree(f->d_depthf);
-    dfree(f->d_fsum);
-    dfree(f->d_fcount);
+    dfree(f->d_fsum);  // and the counts behind the sums
     delete f;
     return CR_OK;
 }
@@ -1249,9 +1251,12 @@ CR_API cr_status cr_hqs_forward_f32(cr_context *ctx, cr_frame *f, cr_cloud *clou
     cudaStream_t s = ctx->stream;
     const size_t npix = (size_t)f->width * f->height;
     if (!f->d_fsum) {
-        if ((st = dalloc(&f->d_fsum, npix * sizeof(float4))) ||
-            (st = dalloc(&f->d_fcount, (npix + 3) / 4 * 16)))
-            return st;
+        // One allocation, so that a frame has both planes or neither: the sums,
+        // then the counts.
+        float4 *planes = nullptr;
+        if ((st = dalloc(&planes, npix * sizeof(float4) + (npix + 3) / 4 * 16))) return st;
+        f->d_fsum = planes;
+        f->d_fcount = reinterpret_cast<uint32_t *>(planes + npix);
     }
     // The planes are zeroed by extra CTAs of the cull's launch.
     const FrameClear fc = f32_clear_of(f);

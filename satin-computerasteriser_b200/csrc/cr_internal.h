@@ -235,7 +235,8 @@ struct cr_frame {
     uint32_t *d_rgba[2] = {nullptr, nullptr}; // RGBA8 ping-pong (resolve, hole fill)
     float *d_depthf = nullptr;              // resolve R32F depth
     float4 *d_fsum = nullptr;               // differentiable colours: FP32 R, G, B sums (lazy)
-    uint32_t *d_fcount = nullptr;           //   and their sample counts (whole 16-byte groups)
+    uint32_t *d_fcount = nullptr;           //   and, behind them, their sample counts (whole
+                                            //   16-byte groups)
     int final_rgba = 0;                     // which d_rgba holds the final image
     int last_mode = -1;                     // 0 HQS, 1 nearest, -1 none
     // Asynchronous read-back: `rendered` is recorded on the context stream
