@@ -498,8 +498,14 @@ cr_status launch_pick(cr_frame *f, int px, int py, int radius, cudaStream_t s) {
         ctx->d_pick = d;
     }
     if (!ctx->h_pick) {
-        CR_CUDA(cudaHostAlloc((void **)&ctx->h_pick, 2 * sizeof(uint32_t), cudaHostAllocMapped));
-        CR_CUDA(cudaHostGetDevicePointer((void **)&ctx->d_picked, ctx->h_pick, 0));
+        // Kept only with its device address: the kernel writes there.
+        uint32_t *h = nullptr;
+        CR_CUDA(cudaHostAlloc((void **)&h, 2 * sizeof(uint32_t), cudaHostAllocMapped));
+        if (const cudaError_t e = cudaHostGetDevicePointer((void **)&ctx->d_picked, h, 0)) {
+            cudaFreeHost(h);
+            return cri::cuda_fail(e, "cudaHostGetDevicePointer (pick words)");
+        }
+        ctx->h_pick = h;
     }
     const long long r = std::max(radius, 0);
     const int x0 = (int)std::max<long long>(0, px - r);
