@@ -102,6 +102,7 @@ struct cr_context {
     int view_group_pixels = 4194304;   // batched views: pixels per depth/colour group
     bool use_tiles = true;             // shared-memory screen tiles
     int cull_spin_limit = 1 << 20;     // polls of a predecessor before a cull CTA gives up
+    uint32_t sort_wait_limit = 1u << 22;  // the same, a tile of the packer's sort
     // Device-side status word (page-locked, mapped into the device's address
     // space): kernels store an error code into it, and the host reads it
     // after the calls that synchronise with the context's stream.

@@ -50,13 +50,15 @@ cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStre
 // segs is device memory; n0: the keys of the first.  ties_ok: the passes over
 // the lowest digits of a single large segment of 64-bit keys may be left out;
 // keys that agree above the segment's tie bits (RadixScratch::ties) are then in
-// input order, and the caller orders them.  A bounded wait that gives up
-// stores kErrSortWait into *status.
+// input order, and the caller orders them.  A tile's wait for those before it
+// that gives up after wait_limit polls (0: every tile after a segment's first
+// gives up at once) stores kErrSortWait into *status; the values may then be
+// anything.
 constexpr uint32_t kSampleMinKeys = 1u << 19;
 template <typename K>
 cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
                      uint64_t ntiles, uint32_t n0, int key_bits, bool ties_ok, RadixScratch &rs,
-                     uint32_t *status, cudaStream_t s);
+                     uint32_t wait_limit, uint32_t *status, cudaStream_t s);
 
 struct PackSeg;
 

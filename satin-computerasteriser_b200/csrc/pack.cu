@@ -407,7 +407,8 @@ __global__ void __launch_bounds__(kThreads)
     for (int k = 0; k < kEach; ++k) {
         const uint64_t i = i0 + k * kThreads;
         place[k] = (uint32_t)i;
-        from[k] = i < sg.n && idx ? __ldg(idx + i) : (uint32_t)i;
+        // Bounded, since a sort that gave up waiting leaves any value.
+        from[k] = i < sg.n && idx ? min(__ldg(idx + i), sg.n - 1u) : (uint32_t)i;
     }
 #pragma unroll
     for (int k = 0; k < kEach; ++k)
@@ -945,7 +946,7 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
         PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
                     (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
         st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, segs[0].n, 63, true, sc.radix,
-                           ctx->d_status, s);
+                           ctx->sort_wait_limit, ctx->d_status, s);
     } else {
         using K = uint32_t;
         const RadixBuffers<K> buf{{static_cast<K *>(sc.keys[0]), static_cast<K *>(sc.keys[1])},
@@ -953,7 +954,7 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
         PACK_LAUNCH(nseg, dim3(rows(nseg), nseg), kThreads, s, (pack_morton<K, true>),
                     (pack_morton<K, false>), arg, buf.keys[0], sc.radix.hist);
         st = radix_sort<K>(buf, sc.rsegs, nseg, tiles, segs[0].n, 30, false, sc.radix,
-                           ctx->d_status, s);
+                           ctx->sort_wait_limit, ctx->d_status, s);
     }
     if (st) return st;
 

@@ -33,9 +33,11 @@
 // where its sorted keys and indices end up.
 // A tile waits only for tiles with smaller tickets, which started before it,
 // so the waits end whatever the GPU schedules; each wait is nevertheless
-// bounded (kLookbackLimit polls), after which the tile counts the missing
+// bounded (wait_limit polls), after which the tile counts the missing
 // predecessor as empty and stores kErrSortWait into the status word, which
-// the host reports as CR_ERR_TIMEOUT.
+// the host reports as CR_ERR_TIMEOUT.  The order is then no permutation: places
+// of the values' buffers keep what was there before, so their readers bound
+// them.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -49,7 +51,6 @@ constexpr int kThreads = 256;  // one thread per digit in the per-digit phases
 constexpr int kWarps = kThreads / 32;
 constexpr int kKeysPerLane = 16;
 constexpr int kTileKeys = kThreads * kKeysPerLane;  // 4096
-constexpr uint32_t kLookbackLimit = 1u << 22;
 
 // Look-back word of one (tile, digit): epoch (16 bits) | flag (2 bits) |
 // count (46 bits).  Flag 1: the tile's own count; flag 2: the inclusive count
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
     radix_onesweep(RadixBuffers<K> buf, const RadixSeg *__restrict__ segs, uint32_t nseg, int pass,
                    const uint32_t *__restrict__ bases, const uint32_t *__restrict__ runs,
                    unsigned long long *__restrict__ lookback, uint32_t epoch,
-                   uint32_t *__restrict__ tile_counter, uint32_t *status) {
+                   uint32_t *__restrict__ tile_counter, uint32_t wait_limit, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char smem[];
     K *skey = reinterpret_cast<K *>(smem);
     uint32_t *sval = reinterpret_cast<uint32_t *>(skey + kTileKeys);
@@ -394,9 +395,9 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
         // round (independent loads), newest first: add counts until a tile's
         // inclusive prefix; a word not yet published is polled (bounded).
         constexpr unsigned long long kCountMask = (1ull << 46) - 1ull;
-        bool gave_up = false;
+        bool gave_up = wait_limit == 0u;
         int64_t t = (int64_t)tile - 1;
-        while (t >= 0) {
+        while (t >= 0 && !gave_up) {
             const int nb = t + 1 < kLookbackBatch ? (int)(t + 1) : kLookbackBatch;
             unsigned long long v[kLookbackBatch];
 #pragma unroll
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
             const unsigned long long *w = lookback + (size_t)(t - nr) * 256 + dd;
             uint32_t polls = 0;
             unsigned long long x = ld_relaxed64(w);
-            while (!lookback_ready(x, epoch) && ++polls < kLookbackLimit) {
+            while (!lookback_ready(x, epoch) && ++polls < wait_limit) {
                 __nanosleep(32);
                 x = ld_relaxed64(w);
             }
@@ -489,7 +490,7 @@ cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStre
 template <typename K>
 cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,
                      uint64_t ntiles, uint32_t n0, int key_bits, bool ties_ok, RadixScratch &rs,
-                     uint32_t *status, cudaStream_t s) {
+                     uint32_t wait_limit, uint32_t *status, cudaStream_t s) {
     const int passes = (key_bits + 7) / 8;
     if (nseg == 0 || passes > kRadixMaxPasses || ntiles > rs.cap_tiles || nseg > rs.cap_segs)
         return cri::fail(CR_ERR_INTERNAL, "radix_sort: arguments");
@@ -522,16 +523,17 @@ cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t 
             rs.epoch = 1;
         }
         radix_onesweep<K><<<(unsigned)ntiles, kThreads, smem, s>>>(
-            buf, segs, nseg, p, rs.bases, rs.runs, rs.lookback, rs.epoch, rs.tiles + p, status);
+            buf, segs, nseg, p, rs.bases, rs.runs, rs.lookback, rs.epoch, rs.tiles + p,
+            wait_limit, status);
         CR_CUDA(cudaGetLastError());
     }
     return CR_OK;
 }
 
 template cr_status radix_sort<uint32_t>(const RadixBuffers<uint32_t> &, const RadixSeg *, uint32_t,
-                                        uint64_t, uint32_t, int, bool, RadixScratch &, uint32_t *,
-                                        cudaStream_t);
+                                        uint64_t, uint32_t, int, bool, RadixScratch &, uint32_t,
+                                        uint32_t *, cudaStream_t);
 template cr_status radix_sort<unsigned long long>(const RadixBuffers<unsigned long long> &,
                                                   const RadixSeg *, uint32_t, uint64_t, uint32_t,
-                                                  int, bool, RadixScratch &, uint32_t *,
+                                                  int, bool, RadixScratch &, uint32_t, uint32_t *,
                                                   cudaStream_t);
