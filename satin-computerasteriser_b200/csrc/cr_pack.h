@@ -52,8 +52,8 @@ cr_status radix_begin(RadixScratch &rs, uint32_t nseg, uint64_t ntiles, cudaStre
 // keys that agree above the segment's tie bits (RadixScratch::ties) are then in
 // input order, and the caller orders them.  A tile's wait for those before it
 // that gives up after wait_limit polls (0: every tile after a segment's first
-// gives up at once) stores kErrSortWait into *status; the values may then be
-// anything.
+// gives up at once) stores kErrSortWait into *status; the segment's keys and
+// values may then be anything, and its tie bits are 0.
 constexpr uint32_t kSampleMinKeys = 1u << 19;
 template <typename K>
 cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t nseg,

@@ -36,8 +36,8 @@
 // bounded (wait_limit polls), after which the tile counts the missing
 // predecessor as empty and stores kErrSortWait into the status word, which
 // the host reports as CR_ERR_TIMEOUT.  The order is then no permutation: places
-// of the values' buffers keep what was there before, so their readers bound
-// them.
+// of the buffers keep what was there before.  The values' readers bound them,
+// and the segment has no ties any more: nobody walks along runs of such keys.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -299,7 +299,8 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
     radix_onesweep(RadixBuffers<K> buf, const RadixSeg *__restrict__ segs, uint32_t nseg, int pass,
                    const uint32_t *__restrict__ bases, const uint32_t *__restrict__ runs,
                    unsigned long long *__restrict__ lookback, uint32_t epoch,
-                   uint32_t *__restrict__ tile_counter, uint32_t wait_limit, uint32_t *status) {
+                   uint32_t *__restrict__ tile_counter, uint32_t wait_limit,
+                   uint32_t *__restrict__ ties, uint32_t *status) {
     extern __shared__ __align__(16) unsigned char smem[];
     K *skey = reinterpret_cast<K *>(smem);
     uint32_t *sval = reinterpret_cast<uint32_t *>(skey + kTileKeys);
@@ -440,7 +441,10 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
             if (((x >> 46) & 3ull) == kFlagPrefix) break;
             t -= nr + 1;
         }
-        if (gave_up && status) *(volatile uint32_t *)status = kErrSortWait;
+        if (gave_up) {
+            ties[si] = 0u;
+            if (status) *(volatile uint32_t *)status = kErrSortWait;
+        }
         st_relaxed64(my, lookback_word(epoch, kFlagPrefix, excl + total));
     }
     gbase[dd] = digit_base[dd] + (uint32_t)excl - tbase;
@@ -524,7 +528,7 @@ cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t 
         }
         radix_onesweep<K><<<(unsigned)ntiles, kThreads, smem, s>>>(
             buf, segs, nseg, p, rs.bases, rs.runs, rs.lookback, rs.epoch, rs.tiles + p,
-            wait_limit, status);
+            wait_limit, rs.ties, status);
         CR_CUDA(cudaGetLastError());
     }
     return CR_OK;

@@ -51,3 +51,27 @@ def test_pack_after_a_sort_that_gave_up(cr, orc, inside, bits):
         pack_without_waiting(cr, ctx, inside, pos, rgba, bits)
     cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, bits=bits)
     check_region(cloud, ref, 0, 10240, src)
+
+
+def test_packs_after_a_sort_with_ties_gave_up(cr, orc, inside):
+    """63-bit keys of a cloud large enough to leave out low digits: with the
+    order wrong, no run of keys is walked along, and every voxel of the LOD
+    grids that was claimed is set free again, so later packs of the context
+    (of the same grids, and of smaller ones in the same memory) have the
+    CPU's levels."""
+    ctx = cr.Context(0)
+    rng = np.random.default_rng(9)
+    n = (1 << 19) + 4099
+    pos = rng.uniform(-1.0, 1.0, (n, 3)).astype(np.float32)
+    rgba = rng.integers(0, 1 << 32, n, dtype=np.uint32)
+    ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=10240, morton_bits=21, threads=8)
+    few, few_rgba = blob_cloud(30000, 4)
+    few_ref = orc.pack(few, colors_rgba8=few_rgba, pointsPerBatch=10240)
+    cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, bits=21)
+    check_region(cloud, ref, 0, 10240, src)
+    for _ in range(2):
+        pack_without_waiting(cr, ctx, inside, pos, rgba, 21)
+        cloud, src = gpu_pack(cr, ctx, few, rgba=few_rgba)
+        check_region(cloud, few_ref, 0, 10240, src)
+        cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, bits=21)
+        check_region(cloud, ref, 0, 10240, src)
