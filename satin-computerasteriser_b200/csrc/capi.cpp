@@ -126,7 +126,13 @@ cr_status flush_mirror(cr_cloud *c) {
     CR_CUDA(cudaMemcpyAsync(c->d_batches + lo, c->mirror.data() + lo,
                             (size_t)(hi - lo + 1) * sizeof(cr_raster_batch),
                             cudaMemcpyHostToDevice, c->ctx->stream));
+    c->unflushed_removals = 0;
     return CR_OK;
+}
+
+uint64_t drawn_points_bound(const cr_cloud *c) {
+    return ((uint64_t)c->cap.maxResidentBatches - c->free_slots.size() + c->unflushed_removals) *
+           c->cap.pointsPerBatch;
 }
 
 namespace {
@@ -211,6 +217,7 @@ cr_status allocate_cloud(cr_cloud *c, cr_capacity cap, const cr_raster_file *fil
         c->free_slots.push_back((int32_t)s);
     c->resident = 0;
     c->points = 0;
+    c->unflushed_removals = 0;
     c->dirty_lo = INT64_MAX;
     c->dirty_hi = -1;
 
@@ -678,6 +685,7 @@ CR_API cr_status cr_cloud_remove_batches(cr_cloud *c, const int32_t *slots, uint
         b.numPoints = 0;
         mark_dirty(c, slots[i], slots[i]);
         c->free_slots.push_back(slots[i]);
+        c->unflushed_removals += 1;
     }
     if (commit) {
         DeviceGuard g(c->ctx->device);
@@ -923,11 +931,16 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
     if (cfg->mode == CR_MODE_HIGH_QUALITY_AVERAGE) {
         // encodeHighQualityAverage (ComputeRasteriser.swift:322-456).
         std::vector<cr_cloud *> resident;
-        uint64_t max_samples = 0;  // upper bound on the frame's colour samples
+        // Upper bounds on the frame's colour samples: as the device's records are
+        // now, and whatever they become (a captured frame that is replayed after
+        // batches were added).
+        uint64_t max_samples = 0, pool_samples = 0;
         for (uint32_t i = 0; i < nclouds; ++i)
             if (clouds[i]->resident > 0) {
                 resident.push_back(clouds[i]);
-                max_samples += (uint64_t)clouds[i]->resident * clouds[i]->cap.pointsPerBatch;
+                max_samples += drawn_points_bound(clouds[i]);
+                pool_samples += (uint64_t)clouds[i]->cap.maxResidentBatches *
+                                clouds[i]->cap.pointsPerBatch;
             }
         const RasterUniforms rau = make_raster_uniforms(cfg, cam, W, H);
         // Colour variants (ComputeRasteriser.swift:229-253): their own depth
@@ -956,7 +969,7 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         // again: they pack while no pixel can pass kPackedMaxCount at all.
         const bool variants_packed =
             variants && !coverage && (stages & CR_STAGE_COLOR) && (stages & CR_STAGE_RESOLVE) &&
-            max_samples <= kPackedMaxCount;
+            pool_samples <= kPackedMaxCount;
         RasterTargets t{f->d_depth, f->d_accum, f->d_nearest};
         t.packed = packed || variants_packed ? 1 : 0;
         if (stages & CR_STAGE_DEPTH) {
@@ -1009,10 +1022,10 @@ static cr_status render_impl(cr_context *ctx, cr_frame *f, cr_cloud *const *clou
         if (stages & CR_STAGE_RESOLVE) {
             PassTimer pt(ctx, CR_PASS_RESOLVE);
             if ((st = frame_copy_fence(f, s))) return st;
-            // A pixel holds at most a sample per resident point: up to
+            // A pixel holds at most a sample per point: in pools of up to
             // kPackedMaxCount points no field can carry, and there is nothing
             // to check or to run again (a launch of 3 us otherwise).
-            const bool check = packed && max_samples > kPackedMaxCount;
+            const bool check = packed && pool_samples > kPackedMaxCount;
             if (coverage) {
                 if ((st = launch_resolve_coverage(f, ru, s))) return st;
             } else if ((st = launch_resolve_hqs(f, ru, s, check, nullptr))) {

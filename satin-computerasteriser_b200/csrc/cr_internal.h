@@ -188,6 +188,8 @@ struct cr_cloud {
     bool files_dirty = false;
     std::vector<cr_raster_batch> mirror;      // host mirror of every slot
     std::vector<int32_t> free_slots;          // LIFO, back() is handed out first
+    uint64_t unflushed_removals = 0;          // slots freed since the mirror was last flushed:
+                                              // the device still draws them
     int64_t dirty_lo = INT64_MAX, dirty_hi = -1;
     uint32_t resident = 0;
     uint64_t points = 0;
@@ -262,6 +264,9 @@ bool uploads_cancel(cr_cloud *c, int32_t slot);
 bool upload_slot_busy(const cr_cloud *c, uint32_t slot);
 void mark_dirty(cr_cloud *c, int64_t lo, int64_t hi);
 cr_status flush_mirror(cr_cloud *c);
+// No fewer points than the device's batch records hold: every slot that is not
+// free, and those whose removal has not reached the device.
+uint64_t drawn_points_bound(const cr_cloud *c);
 
 // Makes later work on `s` wait (on the device) for the frame's enqueued
 // asynchronous read-backs; call before the first write of the RGBA8 planes.

@@ -512,7 +512,7 @@ CR_API cr_status cr_render_multiview(cr_context *ctx, cr_frame *const *frames,
     for (uint32_t i = 0; i < nclouds; ++i) {
         if (clouds[i]->resident == 0) continue;
         resident.push_back(clouds[i]);
-        max_samples += (uint64_t)clouds[i]->resident * clouds[i]->cap.pointsPerBatch;
+        max_samples += drawn_points_bound(clouds[i]);
         for (int j = 0; j < 16; ++j)
             rmodels.push_back(models ? models[16 * i + j] : (j % 5 == 0 ? 1.0f : 0.0f));
     }
