@@ -43,6 +43,7 @@ enum CounterSlot : int {
     CNT_CULL_EPOCH = 10,  // one-pass cull: launches completed (its CTAs' publish flags are epoch + 1)
     CNT_CULL_DONE = 11,   // one-pass cull: CTAs finished (the last one advances the epoch)
     CNT_CULL_TICKET = 12, // one-pass cull: next CTA ticket (wraps to 0 after the launch's last)
+    CNT_CHUNK_POINTS = 13, // most points of a chunk record of the last cull
     CNT_COUNT = 32
 };
 
@@ -207,7 +208,6 @@ struct cr_cloud {
     uint32_t *d_cull_cta = nullptr;          // per-CTA survivor and chunk counts
     ChunkRec *d_chunks = nullptr;            // chunk work records
     uint64_t chunk_cap = 0;                  // capacity of d_chunks
-    uint32_t cull_chunk_points = 0;          // most points of a record of the last cull
 
     // Fragments of the last depth pass, in pool point index space: a chunk
     // starting at point p keeps its n kept points compacted at [p, p + n).

@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(kCullThreads)
         counters[CNT_WORK_COLOR] = 0u;
         counters[CNT_DONE] = 0u;
         counters[CNT_CHUNKS] = off_c + total_chunks;
+        counters[CNT_CHUNK_POINTS] = a.chunk_points;
         counters[CNT_POINTS] = off_p + total_points;
     }
     if (threadIdx.x == 0) {
@@ -565,9 +566,10 @@ cr_status launch_cull(cr_cloud *cloud, const CullUniforms &u, cudaStream_t s,
     const uint32_t most = (uint32_t)std::max(cloud->ctx->chunk_points, kMinChunkPoints);
     const bool few = (uint64_t)cloud->resident * cloud->cap.pointsPerBatch <=
                      5ull * (uint32_t)cloud->ctx->sm_count * 2048u;
-    const uint32_t cp = few ? std::min(most, 1024u) : most;
+    // No batch has more than pointsPerBatch points, and no record need have.
+    const uint32_t cp = std::min(few ? std::min(most, 1024u) : most,
+                                 std::max<uint32_t>(cloud->cap.pointsPerBatch, kMinChunkPoints));
     const uint32_t ctas = (n + kCullThreads - 1) / kCullThreads;
-    cloud->cull_chunk_points = cp;
     CullArgs a{cloud->d_batches,  n,
                cloud->d_files,    (uint32_t)cloud->files.size(),
                cloud->d_cull_tmp, cloud->d_cull_cta,

@@ -1290,6 +1290,12 @@ __device__ __forceinline__ void splat_to_frame(const RasterArgs &a, const ViewRe
                                     (zc.y >> 16) & 0xffu, 1u);
         }
 }
+// Steps per chunk record, from the size that the cull gave its records.  The
+// records' steps are no more than two and a half times the records at the
+// smallest size, of which the fragment counts have room for kFragCounts.
+__device__ __forceinline__ uint32_t splat_steps(const uint32_t *counters) {
+    return (counters[CNT_CHUNK_POINTS] + kSplatPoints - 1) / kSplatPoints;
+}
 // Steps are claimed from the cloud's work cursor, as the point passes claim
 // their records; the last CTA resets it.
 __device__ __forceinline__ void splat_finish(const RasterArgs &a) {
@@ -1303,7 +1309,7 @@ __device__ __forceinline__ void splat_finish(const RasterArgs &a) {
 }
 
 __global__ void __launch_bounds__(kThreads, 4)
-    splat_depth(const __grid_constant__ RasterArgs a, uint32_t steps, uint32_t most) {
+    splat_depth(const __grid_constant__ RasterArgs a) {
     __shared__ uint32_t tile[kSplatPx];
     __shared__ SplatShared ss;
     __shared__ __align__(16) float sfile[kInlineFiles][32];  // transform, world
@@ -1318,7 +1324,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     const crd::PointSize ps{a.u.pointSizeMode, a.u.minimumPointSize, a.u.maximumPointSize,
                             a.u.pointSizeScale};
     const int lane = threadIdx.x & 31;
-    const uint32_t total = min(a.counters[CNT_CHUNKS] * steps, most);
+    const uint32_t steps = splat_steps(a.counters), total = a.counters[CNT_CHUNKS] * steps;
     uint32_t *cursor = a.counters + CNT_WORK_DEPTH;
     if (threadIdx.x == 0) {
         ss.next = atomicAdd(cursor, 1u);
@@ -1425,7 +1431,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 // keep every field below its width) and the pixels' visibility thresholds.
 constexpr int kSplatColorBytes = kSplatPx * 16;
 __global__ void __launch_bounds__(kThreads, 5)
-    splat_color(const __grid_constant__ RasterArgs a, uint32_t steps, uint32_t most) {
+    splat_color(const __grid_constant__ RasterArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t *acc = reinterpret_cast<uint32_t *>(smem);
     float *thr = reinterpret_cast<float *>(acc + 3 * kSplatPx);
@@ -1434,7 +1440,7 @@ __global__ void __launch_bounds__(kThreads, 5)
     crd::launch_dependents();
     const ViewRegsT<false> vr(a);
     const int W = a.u.width, H = a.u.height;
-    const uint32_t total = min(a.counters[CNT_CHUNKS] * steps, most);
+    const uint32_t steps = splat_steps(a.counters), total = a.counters[CNT_CHUNKS] * steps;
     uint32_t *cursor = a.counters + CNT_WORK_DEPTH;
     if (threadIdx.x == 0) {
         ss.next = atomicAdd(cursor, 1u);
@@ -1539,8 +1545,7 @@ struct RedoArgs {
     float *depthf;
     uint32_t npix;
     ResolveUniforms ru;
-    uint32_t splat_steps[kRedoMaxClouds];  // splats: steps per chunk record; 0: single pixels
-    uint32_t splat_most[kRedoMaxClouds];   // and their bound
+    int splats;  // the fragments are the splat passes'
 };
 
 __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
@@ -1560,9 +1565,8 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
         a.frag_zc = const_cast<uint2 *>(r.clouds[ci].frag_zc);
         const ViewRegsT<false> vr(a);
         const uint32_t nchunks = r.clouds[ci].counters[CNT_CHUNKS];
-        const uint32_t steps = r.splat_steps[ci];
-        if (steps) {
-            const uint32_t total = min(nchunks * steps, r.splat_most[ci]);
+        if (r.splats) {
+            const uint32_t steps = splat_steps(r.clouds[ci].counters), total = nchunks * steps;
             for (uint32_t v = 0; v < total; ++v) {
                 const uint32_t k = v / steps;
                 const uint32_t base = a.chunks[k].first + (v - k * steps) * kSplatPoints;
@@ -1599,8 +1603,8 @@ __global__ void __launch_bounds__(kThreads, 5)
 
 // The differentiable passes of one view with single-pixel footprints (depth
 // plane, FP32 colour sums, adjoint): 512 points of a chunk record to a step,
-// two to a thread, `steps` steps to a record; the grid strides over all of
-// them.  A training view holds a million points or so, of which the
+// two to a thread, as many steps to a record as the size that the cull gave
+// its records takes; the grid strides over all of them.  A training view holds a million points or so, of which the
 // four-points-a-thread passes make two rounds in the few hundred chunks that
 // there are: half of the SMs' warps had no work, and each waited for its
 // chain of loads (record, words, depth, colour) alone.  Steps spread the work
@@ -1613,7 +1617,7 @@ static_assert(kStepEach % 2 == 0, "points are projected in pairs");
 constexpr int kStepPoints = kStepEach * kThreads;
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 6)
-    point_pass(const __grid_constant__ RasterArgs a, uint32_t steps) {
+    point_pass(const __grid_constant__ RasterArgs a) {
     // The inline files' transforms; a larger table is read where it is.
     __shared__ __align__(16) float sT[kInlineFiles][16];
     for (uint32_t t = threadIdx.x; t < 16u * a.ifiles.n; t += kThreads)
@@ -1623,6 +1627,7 @@ __global__ void __launch_bounds__(kThreads, 6)
     __syncthreads();
     const ViewRegsT<false> vr(a);
     const int W = a.u.width;
+    const uint32_t steps = (a.counters[CNT_CHUNK_POINTS] + kStepPoints - 1) / kStepPoints;
     const uint32_t total = a.counters[CNT_CHUNKS] * steps;
     for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
         const uint32_t k = v / steps, local0 = (v - k * steps) * kStepPoints + threadIdx.x;
@@ -1821,19 +1826,6 @@ RasterArgs make_args(cr_cloud *cloud, const RasterUniforms &u, const RasterTarge
     return a;
 }
 
-// Steps per chunk record of the splat passes.  A batch has at most
-// pointsPerBatch points, so the steps of all records are no more than the
-// records at the smallest chunk size, which the fragment counts have room for.
-uint32_t splat_steps(const cr_cloud *cloud) {
-    const uint32_t most = std::min(cloud->cull_chunk_points, cloud->cap.pointsPerBatch);
-    return (most + kSplatPoints - 1) / kSplatPoints;
-}
-// The room itself, for the records of a replayed capture whose cull had another
-// chunk size than the cloud's last one.
-uint32_t splat_most(const cr_cloud *cloud) {
-    return (uint32_t)std::min<uint64_t>(cloud->chunk_cap * kFragCounts, 0xffffffffu);
-}
-
 // One-view passes start while the previous kernel drains (programmatic
 // dependent launch); batched views, captured in a graph, launch plainly.
 template <int PASS, bool MV>
@@ -1884,18 +1876,17 @@ cr_status launch_splats(cr_cloud *cloud, bool color, const RasterUniforms &u,
         const cr_status st = ensure_device_files(cloud);
         if (st) return st;
     }
-    const uint32_t steps = splat_steps(cloud), most = splat_most(cloud);
     cr_context *ctx = cloud->ctx;
     if (color) {
         if (ctx->blocks_per_sm_splat[1] == 0)
             ctx->blocks_per_sm_splat[1] = resident_blocks(splat_color, kSplatColorBytes);
         CR_CUDA(launch_programmatic(splat_color, dim3(ctx->sm_count * ctx->blocks_per_sm_splat[1]),
-                                    dim3(kThreads), (size_t)kSplatColorBytes, s, a, steps, most));
+                                    dim3(kThreads), (size_t)kSplatColorBytes, s, a));
     } else {
         if (ctx->blocks_per_sm_splat[0] == 0)
             ctx->blocks_per_sm_splat[0] = resident_blocks(splat_depth, 0);
         CR_CUDA(launch_programmatic(splat_depth, dim3(ctx->sm_count * ctx->blocks_per_sm_splat[0]),
-                                    dim3(kThreads), 0, s, a, steps, most));
+                                    dim3(kThreads), 0, s, a));
     }
     return CR_OK;
 }
@@ -1911,9 +1902,8 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
     for (uint32_t i = 0; i < nclouds; ++i) {
         r.clouds[i] = RedoCloud{clouds[i]->d_chunks,   clouds[i]->d_counters, clouds[i]->d_frag_count,
                                 clouds[i]->d_frag_xy, clouds[i]->d_frag_zc};
-        r.splat_steps[i] = splats ? splat_steps(clouds[i]) : 0u;
-        r.splat_most[i] = splat_most(clouds[i]);
     }
+    r.splats = splats ? 1 : 0;
     r.nclouds = nclouds;
     r.redo = t.redo;
     r.rgba = f->d_rgba[0];
@@ -1927,15 +1917,12 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
 
 uint32_t hqs_redo_max_clouds() { return kRedoMaxClouds; }
 
-// A step to a CTA while there are CTAs.  No chunk record of the cloud's last
-// cull has more than chunk_points points.
+// A step to a CTA while there are CTAs.
 template <int PASS>
-cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, uint32_t chunk_points,
-                              cudaStream_t s) {
-    const uint32_t steps = (chunk_points + kStepPoints - 1) / kStepPoints;
+cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, cudaStream_t s) {
     return launch_programmatic(point_pass<PASS>,
                                dim3(ctx->sm_count * point_pass_blocks_per_sm<PASS>()),
-                               dim3(kThreads), 0, s, a, steps);
+                               dim3(kThreads), 0, s, a);
 }
 
 cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
@@ -1953,10 +1940,9 @@ cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUnifor
     a.fgrad = grad;
     cr_context *ctx = cloud->ctx;
     if (a.radius_zero) {
-        const uint32_t cp = cloud->cull_chunk_points;
-        CR_CUDA(pass == PASS_DEPTH       ? launch_point_pass<PASS_DEPTH>(a, ctx, cp, s)
-                : pass == PASS_COLOR_F32 ? launch_point_pass<PASS_COLOR_F32>(a, ctx, cp, s)
-                                         : launch_point_pass<PASS_GRAD>(a, ctx, cp, s));
+        CR_CUDA(pass == PASS_DEPTH       ? launch_point_pass<PASS_DEPTH>(a, ctx, s)
+                : pass == PASS_COLOR_F32 ? launch_point_pass<PASS_COLOR_F32>(a, ctx, s)
+                                         : launch_point_pass<PASS_GRAD>(a, ctx, s));
         return CR_OK;
     }
     if (pass == PASS_DEPTH) return launch_raster(cloud, pass, u, t, s);

@@ -36,7 +36,6 @@ struct VariantArgs {
     const uint8_t *levels;
     const cr_raster_file *files;
     InlineFiles ifiles;  // the file table, when small (else n = 0: files)
-    uint32_t steps;      // per chunk record
     int packed;          // two 64-bit adds per sample (not with coverage)
     int radius_zero;     // every footprint is a single pixel
     const float4 *disp, *prev_disp, *tint;  // null: zeros (prev_disp null: disp)
@@ -82,14 +81,15 @@ __global__ void __launch_bounds__(kThreads, COLOR ? 4 : 6)
     crd::grid_wait();
     crd::launch_dependents();
     __syncthreads();
-    const uint32_t total = a.counters[CNT_CHUNKS] * a.steps;
+    const uint32_t steps = (a.counters[CNT_CHUNK_POINTS] + kThreads - 1) / kThreads;  // a record
+    const uint32_t total = a.counters[CNT_CHUNKS] * steps;
     const int W = a.u.width, H = a.u.height;
     const crd::PointSize ps{a.u.pointSizeMode, a.u.minimumPointSize, a.u.maximumPointSize,
                             a.u.pointSizeScale};
     const bool mb_on = a.motion_blur > 0.0f;
     const bool oit = a.coverage_mode || mb_on;
     for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
-        const uint32_t k = v / a.steps, local = (v - k * a.steps) * kThreads + threadIdx.x;
+        const uint32_t k = v / steps, local = (v - k * steps) * kThreads + threadIdx.x;
         ChunkRec c;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -272,7 +272,6 @@ cr_status launch_variant_pass(cr_cloud *cloud, bool color, const RasterUniforms 
     a.ifiles = inline_files(cloud);
     if (!a.ifiles.n)
         if (const cr_status st = ensure_device_files(cloud)) return st;
-    a.steps = (cloud->cull_chunk_points + kThreads - 1) / kThreads;
     a.packed = t.packed;
     a.radius_zero = fmaxf(u.minimumPointSize, u.maximumPointSize) <= 1.0f ? 1 : 0;
     a.disp = cloud->d_disp;
