@@ -688,6 +688,7 @@ cr_status grow(T **p, uint64_t &cap, uint64_t want_elems) {
 }
 
 // Keys are sized for 64-bit words so either key width fits.
+constexpr uint64_t kPointScratch = 2 * sizeof(float4) + 2 * 8 + 3 * 4 + 1;  // bytes a point
 cr_status ensure_points(PackScratch &s, uint64_t n) {
     if (s.cap_points >= n && s.keys[0]) return CR_OK;
     pack_scratch_free(s);
@@ -768,6 +769,23 @@ cr_status lod_args(PackSeg &sg, const float bmin[3], const float ext[3], int lev
     }
     *cells_out = total;
     return CR_OK;
+}
+
+// Device memory that a wave of several jobs may take anew for each kind of its
+// scratch: an eighth of what is free, so that chunks beside a nearly full pool
+// are packed one at a time, as in no more memory than the largest of them needs.
+cr_status wave_share(uint64_t *bytes) {
+    size_t free_b = 0, total_b = 0;
+    CR_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    *bytes = free_b / 8;
+    return CR_OK;
+}
+
+// Bytes of a job's host input, staged on the device.
+uint64_t staged_bytes(const PackJob &job, int on_device) {
+    return on_device ? 0
+                     : job.count * ((uint64_t)job.in->positionStrideBytes +
+                                    job.in->colorStrideBytes);
 }
 
 // Packs jobs [0, njobs) in one run; *done = the jobs packed, fewer than
@@ -898,7 +916,7 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
     const int divs = std::max(1, prm->coarseVoxelDivisions);
     const uint32_t max_level = (uint32_t)(L - 1);
     std::vector<uint64_t> cells(njobs, 0);
-    uint64_t cell_sum = 0;
+    uint64_t cell_sum = 0, cell_limit = 0;
     uint32_t nseg = 0;
     cr_status refused = CR_OK;
     for (uint32_t j = 0; j < njobs; ++j) {
@@ -915,7 +933,16 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
             sg.m.scale[k] = sg.m.top / ext[k];
         }
         if ((refused = lod_args(sg, bmin, ext, L, divs, &cells[j]))) break;
-        if (j > 0 && cell_sum + cells[j] > kLodCellCap) break;
+        // Grids of several jobs together: in the memory that there is, or in new
+        // memory up to the wave's share.
+        if (j > 0 && cell_sum + cells[j] > sc.cap_grid) {
+            if (cell_limit == 0) {
+                uint64_t bytes = 0;
+                if ((st = wave_share(&bytes))) return st;
+                cell_limit = std::max(sc.cap_grid, std::min(kLodCellCap, bytes / 4));
+            }
+            if (cell_sum + cells[j] > cell_limit) break;
+        }
         cell_sum += cells[j];
         nseg = j + 1;
     }
@@ -1009,26 +1036,42 @@ void pack_scratch_free(PackScratch &s) {
 // context stream; one synchronisation per wave reads the segments' bounds
 // back to size the Morton scales and the LOD grids.  src_idx_host (one job
 // only): the input index of every packed point.  A wave takes jobs while
-// they hold at most kWavePoints points together, so that a long list of
-// chunks needs no more scratch than one chunk of that size.
+// they hold at most kWavePoints points and kWaveStaged bytes of host input
+// together, so that a long list of chunks needs no more scratch than one chunk
+// of that size, and takes fewer where their scratch would be more than its share
+// of the free memory, or is refused.
 cr_status pack_run(cr_context *ctx, cr_cloud *cloud, const std::vector<PackJob> &jobs,
                    const cr_pack_params *prm, int on_device, uint32_t *src_idx_host) {
     constexpr uint64_t kWavePoints = 1ull << 24;
     constexpr size_t kWaveJobs = 4096;  // the launches' second grid dimension is bounded
+    constexpr uint64_t kWaveStaged = 1ull << 29;
     if (src_idx_host && jobs.size() != 1)
         return cri::fail(CR_ERR_INTERNAL, "pack_run: source indices of one job only");
     size_t first = 0;
     while (first < jobs.size()) {
-        size_t last = first;
-        uint64_t points = 0;
-        do {
-            points += padded(jobs[last].count);
-            ++last;
-        } while (last < jobs.size() && last - first < kWaveJobs &&
-                 points + padded(jobs[last].count) <= kWavePoints);
+        size_t last = first + 1;
+        uint64_t points = padded(jobs[first].count), staged = staged_bytes(jobs[first], on_device);
+        uint64_t share = 0;
+        for (; last < jobs.size() && last - first < kWaveJobs; ++last) {
+            const uint64_t p = points + padded(jobs[last].count);
+            const uint64_t b = staged + staged_bytes(jobs[last], on_device);
+            if (p > kWavePoints || b > kWaveStaged) break;
+            if (p > ctx->pack->cap_points || b > ctx->pack->cap_raw_bytes) {
+                if (share == 0)
+                    if (const cr_status st = wave_share(&share)) return st;
+                if (p * kPointScratch > share || b > share) break;
+            }
+            points = p;
+            staged = b;
+        }
         uint32_t done = 0;
-        const cr_status st = pack_wave(ctx, cloud, jobs.data() + first, (uint32_t)(last - first),
-                                       prm, on_device, src_idx_host, &done);
+        cr_status st;
+        for (;;) {
+            st = pack_wave(ctx, cloud, jobs.data() + first, (uint32_t)(last - first), prm, on_device,
+                           src_idx_host, &done);
+            if (st != CR_ERR_OUT_OF_MEMORY || last - first == 1) break;
+            last = first + (last - first) / 2;
+        }
         if (st) return st;
         first += done;
     }

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from scenes import blob_cloud
+from test_gpu_pack import check_region
 from test_gpu_render import assert_same, camera, make_cloud, render_both
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,41 @@ def test_fp32_planes_after_running_out_of_memory(cr, orc, ctx):
     assert covered.any()
     want = np.where(covered[..., None], np.array([1.0, 0.5, 0.0], np.float32), np.float32(0.0))
     assert np.abs(img.download() - want).max() <= 1e-4
+
+
+@pytest.mark.parametrize("host", [False, True])
+def test_chunks_beside_a_full_gpu(cr, orc, host):
+    """Thirteen nodes whose LOD grids (78 MB each at the default divisions)
+    fit one at a time, not together: packed, each as the CPU packs it."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(17)
+    nodes = []
+    for k in range(13):
+        n = 2000 + 37 * k
+        nodes.append((rng.uniform(-1.0, 1.0, (n, 3)).astype(np.float32),
+                      rng.integers(0, 1 << 32, n, dtype=np.uint32)))
+    given = nodes
+    if not host:
+        given = [(torch.from_numpy(p).cuda(), torch.from_numpy(c.view("int32")).cuda())
+                 for p, c in nodes]
+        torch.cuda.synchronize()
+    warm = cr.Context(0)  # loads the kernels; its scratch goes with it
+    spare = cr.ComputeRasteriserPointCloud(warm, cr.ComputeRasteriserCapacity(6, 1000))
+    for some in (given[:2], given[:1]):
+        spare.addRawChunksGPU(cr.GPUPacker(warm, coarseVoxelDivisions=4), some)
+    spare.close()
+    warm.close()
+    ctx = cr.Context(0)
+    cloud = cr.ComputeRasteriserPointCloud(ctx, cr.ComputeRasteriserCapacity(3 * 13, 1000))
+    with LeaveFree(cr, ctx, 200 * MB):
+        first = cloud.addRawChunksGPU(cr.GPUPacker(ctx), given)
+        assert len(first) == 13
+        for f, (pos, rgba) in zip(first, nodes):
+            ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=1000)
+            check_region(cloud, ref, f, 1000)
+    # With memory back the nodes go together.
+    cloud.clearAllBatches()
+    assert cloud.addRawChunksGPU(cr.GPUPacker(ctx), given) == first
+    for f, (pos, rgba) in zip(first, nodes):
+        ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=1000)
+        check_region(cloud, ref, f, 1000)
