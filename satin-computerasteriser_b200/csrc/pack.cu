@@ -348,14 +348,22 @@ __device__ __forceinline__ const uint32_t *final_index(const Sorted &so, uint32_
     return sorted_index(so.vals[0], so.vals[1], set, begin);
 }
 
-// Places of a CTA's keys among the keys that agree with them above `low` bits:
-// a key moves back by the keys before it with larger low bits and on by the
-// keys after it with smaller ones (equal keys keep their order).  The CTA's
-// keys are staged in shared memory; a run that leaves it is read on in place.
+// Places of a CTA's keys among the keys that agree with them above `low` (at
+// most 32) bits: in a run of such keys, which are neighbours, a key stands after
+// those with smaller low bits and the equal ones before it.  The CTA's keys are
+// staged in shared memory; a run that leaves it is read in place.  Most runs are
+// of a few keys, which are looked at one after the other.  A longer run's ends are
+// searched for, its keys being sorted above the low bits, and its low words, which
+// differ in those bits alone, are counted with nothing to decide between two
+// reads.  A pack of 600 thousand points of which 700 agree took 408 us key by key,
+// 258 so (310 with every digit sorted); of 100M points of which three thousand
+// agree 9.65 ms, 8.99 so (10.9).
 __device__ __forceinline__ void tie_places(const unsigned long long *__restrict__ keys, uint32_t n,
                                            uint64_t first, uint32_t low, unsigned long long *skey,
                                            uint32_t (&place)[kEach]) {
     const uint32_t count = (uint32_t)min((uint64_t)n - first, (uint64_t)kPointsPerCta);
+    const uint32_t base = (uint32_t)first;
+    constexpr uint32_t kNear = 7;
 #pragma unroll
     for (int k = 0; k < kEach; ++k) {
         const uint32_t t = threadIdx.x + k * kThreads;
@@ -363,28 +371,70 @@ __device__ __forceinline__ void tie_places(const unsigned long long *__restrict_
     }
     __syncthreads();
     auto key_at = [&](uint32_t i) {
-        const uint32_t t = i - (uint32_t)first;  // wraps below the CTA's keys
+        const uint32_t t = i - base;  // wraps below the CTA's keys
         return t < count ? skey[t] : __ldg(keys + i);
     };
     const unsigned long long mask = (1ull << low) - 1ull;
+    uint32_t runs = 0;  // bit k: key k's run goes on past kNear keys on a side
 #pragma unroll
     for (int k = 0; k < kEach; ++k) {
-        const uint32_t i = (uint32_t)first + threadIdx.x + k * kThreads;
+        const uint32_t t = threadIdx.x + k * kThreads, i = base + t;
         place[k] = i;
-        if (threadIdx.x + k * kThreads >= count) continue;
-        const unsigned long long mine = skey[threadIdx.x + k * kThreads];
-        uint32_t at = i;
+        if (t >= count) continue;
+        const unsigned long long mine = skey[t];
+        uint32_t at = i, far = 0u;
         for (uint32_t j = i; j > 0u; --j) {
             const unsigned long long other = key_at(j - 1u);
             if ((other ^ mine) & ~mask) break;
             at -= (other & mask) > (mine & mask) ? 1u : 0u;
+            if (i - j == kNear) {
+                far = 1u;
+                break;
+            }
         }
         for (uint32_t j = i + 1u; j < n; ++j) {
             const unsigned long long other = key_at(j);
             if ((other ^ mine) & ~mask) break;
             at += (other & mask) < (mine & mask) ? 1u : 0u;
+            if (j - i > kNear) {
+                far = 1u;
+                break;
+            }
         }
         place[k] = at;
+        if (far) runs |= 1u << k;
+    }
+    for (; runs; runs &= runs - 1u) {
+        const int which = __ffs(runs) - 1;
+        const uint32_t i = base + threadIdx.x + which * kThreads;
+        const unsigned long long mine = skey[i - base];
+        auto agrees = [&](uint32_t j) { return ((key_at(j) ^ mine) >> low) == 0ull; };
+        uint32_t s = i, e = i + 1u;  // the run is [s, e)
+        uint32_t step = 1u;
+        for (; step <= s && agrees(s - step); step <<= 1) s -= step;
+        while (step >>= 1)
+            if (step <= s && agrees(s - step)) s -= step;
+        step = 1u;
+        for (; step <= n - e && agrees(e - 1u + step); step <<= 1) e += step;
+        while (step >>= 1)
+            if (step <= n - e && agrees(e - 1u + step)) e += step;
+        const uint32_t my = (uint32_t)mine;
+        uint32_t before = 0;
+        auto rank = [&](auto low_at) {
+#pragma unroll 8
+            for (uint32_t j = s; j < i; ++j) before += low_at(j) <= my ? 1u : 0u;
+#pragma unroll 8
+            for (uint32_t j = i + 1u; j < e; ++j) before += low_at(j) < my ? 1u : 0u;
+        };
+        if (s >= base && e - base <= count)
+            rank([&](uint32_t j) { return (uint32_t)skey[j - base]; });
+        else
+            rank([&](uint32_t j) {
+                return __ldg(reinterpret_cast<const uint32_t *>(keys) + 2 * (size_t)j);
+            });
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+            if (k == which) place[k] = s + before;
     }
 }
 

@@ -27,7 +27,8 @@
 // many agree, and when they are few those passes are left out: the segment's
 // tie word then says how many low bits were not sorted, and the reader of the
 // sorted keys orders each run of keys that agree above them (its cost grows
-// with the runs' lengths, which the sample bounds).
+// with the square of a run's length: the sample bounds their mean and the
+// longest).
 // Nothing is read back: which of the two buffers a segment's pass reads
 // follows from the segment's set of digits (bit p: pass p runs), and so does
 // where its sorted keys and indices end up.
@@ -91,18 +92,23 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
 }
 
 // How many pairs of kSamples keys, drawn with replacement from all n, agree
-// above their low 24 (and 32) bits: a hash table of 39-bit (31-bit) values per
-// choice, each slot a value and the samples that had it.  n times the chance
-// that two keys agree is the mean length of the run that a key is in.
+// above their low 24 (and 32) bits, and how many samples at most agree with one
+// another: a hash table of 39-bit (31-bit) values per choice, each slot a value
+// and the samples that had it.  n times the chance that two keys agree is the
+// mean length of the run that a key is in; a run of r keys has about
+// r * kSamples / n samples.
+// found: the pairs of each choice, then the largest counts before a sample.
 constexpr uint32_t kSamples = 1u << 16;
 constexpr int kSampleSlotBits = 18;
 constexpr int kSampleChoices = 2;
 __global__ void __launch_bounds__(kThreads)
     radix_sample(const unsigned long long *__restrict__ keys, uint32_t n,
-                 unsigned long long *__restrict__ table, unsigned long long *__restrict__ pairs) {
+                 unsigned long long *__restrict__ table, unsigned long long *__restrict__ found) {
     constexpr uint32_t kMask = (1u << kSampleSlotBits) - 1u;
     const uint32_t s = blockIdx.x * kThreads + threadIdx.x;
-    uint32_t h = s * 0x9e3779b9u + 0x7f4a7c15u;  // a spread of the sample's number
+    // A spread of the sample's number: Weyl's sequence by the golden ratio, and
+    // the first steps of MurmurHash3's 32-bit finaliser.
+    uint32_t h = s * 0x9e3779b9u + 0x7f4a7c15u;
     h ^= h >> 16;
     h *= 0x85ebca6bu;
     h ^= h >> 13;
@@ -122,25 +128,34 @@ __global__ void __launch_bounds__(kThreads)
             break;
         }
         const uint32_t sum = __reduce_add_sync(0xffffffffu, agree);
-        if ((threadIdx.x & 31) == 0 && sum) atomicAdd(pairs + v, (unsigned long long)sum);
+        const uint32_t most = __reduce_max_sync(0xffffffffu, agree);
+        if ((threadIdx.x & 31) == 0 && sum) {
+            atomicAdd(found + v, (unsigned long long)sum);
+            atomicMax(found + kSampleChoices + v, (unsigned long long)most);
+        }
     }
 }
 
 // Low passes to leave out given the sample: those whose bits separate runs of
-// at most kMaxMeanRun keys in the mean.
-constexpr unsigned long long kMaxMeanRun = 6;
-__device__ __forceinline__ uint32_t passes_left_out(const unsigned long long *pairs, uint32_t n) {
+// at most kMaxMeanRun keys in the mean and, by the samples of one run, of about
+// kMaxRun keys (or kMaxRunSamples samples, where one stands for more keys).  By
+// the mean alone, 100M points with 24 thousand in one cell were packed in 17.9 ms,
+// 10.9 with every digit sorted.
+constexpr unsigned long long kMaxMeanRun = 6, kMaxRun = 1024, kMaxRunSamples = 4;
+__device__ __forceinline__ uint32_t passes_left_out(const unsigned long long *found, uint32_t n) {
+    const unsigned long long longest = max(kMaxRunSamples, kMaxRun * kSamples / n);
     for (int v = kSampleChoices - 1; v >= 0; --v)
-        if (2ull * pairs[v] * n <= kMaxMeanRun * ((unsigned long long)kSamples * kSamples))
+        if (2ull * found[v] * n <= kMaxMeanRun * ((unsigned long long)kSamples * kSamples) &&
+            found[kSampleChoices + v] < longest)
             return 3u + (uint32_t)v;
     return 0u;
 }
 
 // A segment's digit bases, the set of its passes and its tie word: one CTA per
-// segment, a thread per digit.  pairs: the sample (null: none was taken).
+// segment, a thread per digit.  sampled: radix_sample's (null: none was taken).
 __global__ void __launch_bounds__(kThreads)
     radix_bases(const uint32_t *__restrict__ hist, const RadixSeg *__restrict__ segs, int passes,
-                const unsigned long long *__restrict__ pairs, uint32_t *__restrict__ bases,
+                const unsigned long long *__restrict__ sampled, uint32_t *__restrict__ bases,
                 uint32_t *__restrict__ runs, uint32_t *__restrict__ ties) {
     __shared__ uint32_t sums[kRadixMaxPasses][kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -167,7 +182,7 @@ __global__ void __launch_bounds__(kThreads)
         if (p < passes) bases[row + p * 256 + threadIdx.x] = base;
     }
     if (threadIdx.x == 0) {
-        const uint32_t out = pairs ? passes_left_out(pairs, n) : 0u;
+        const uint32_t out = sampled ? passes_left_out(sampled, n) : 0u;
         runs[blockIdx.x] = set & ~((1u << out) - 1u);
         ties[blockIdx.x] = 8u * out;
     }
@@ -501,19 +516,19 @@ cr_status radix_sort(const RadixBuffers<K> &buf, const RadixSeg *segs, uint32_t 
     // A sample is taken of one large segment of 64-bit keys: the passes left
     // out then save more than the sample costs (15 us; at half a million keys
     // two passes take that long).
-    const unsigned long long *pairs = nullptr;
+    const unsigned long long *sampled = nullptr;
     if constexpr (sizeof(K) == 8) {
         if (ties_ok && nseg == 1 && n0 >= kSampleMinKeys) {
-            const size_t words = ((size_t)kSampleChoices << kSampleSlotBits) + kSampleChoices;
+            const size_t words = ((size_t)kSampleChoices << kSampleSlotBits) + 2 * kSampleChoices;
             if (!rs.sample) CR_CUDA(cudaMalloc((void **)&rs.sample, words * 8));
             CR_CUDA(cudaMemsetAsync(rs.sample, 0, words * 8, s));
             unsigned long long *found = rs.sample + ((size_t)kSampleChoices << kSampleSlotBits);
             radix_sample<<<kSamples / kThreads, kThreads, 0, s>>>(buf.keys[0], n0, rs.sample, found);
             CR_CUDA(cudaGetLastError());
-            pairs = found;
+            sampled = found;
         }
     }
-    radix_bases<<<nseg, kThreads, 0, s>>>(rs.hist, segs, passes, pairs, rs.bases, rs.runs, rs.ties);
+    radix_bases<<<nseg, kThreads, 0, s>>>(rs.hist, segs, passes, sampled, rs.bases, rs.runs, rs.ties);
     CR_CUDA(cudaGetLastError());
     const size_t smem = onesweep_smem_bytes<K>();
     CR_CUDA(cudaFuncSetAttribute(radix_onesweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,

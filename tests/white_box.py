@@ -14,6 +14,7 @@ extern "C" {
 void set_sort_wait_limit(cr_context *c, uint32_t polls) { c->sort_wait_limit = polls; }
 uint32_t get_sort_wait_limit(const cr_context *c) { return c->sort_wait_limit; }
 void *sort_indices(const cr_context *c, int k) { return c->pack->idx[k]; }
+void *sort_ties(const cr_context *c) { return c->pack->radix.ties; }
 }
 """
 
@@ -34,4 +35,6 @@ def build(tmp_path, cr):
     lib.get_sort_wait_limit.restype = C.c_uint32
     lib.sort_indices.argtypes = [C.c_void_p, C.c_int]
     lib.sort_indices.restype = C.c_void_p
+    lib.sort_ties.argtypes = [C.c_void_p]
+    lib.sort_ties.restype = C.c_void_p
     return lib
