@@ -1588,8 +1588,12 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
     }
 }
 
+// The nearest pass of larger footprints asks for four CTAs per SM: left to the
+// compiler it has 48 registers, some spilled, and 5M points of 4 m splats at
+// 1080p take 1268 us, 1052 so (1028 at three, but 20M points of 0.5 m splats 161
+// instead of 147).
 template <int PASS, bool MV>
-__global__ void __launch_bounds__(kThreads) raster_kernel(const __grid_constant__ RasterArgs a) {
+__global__ void __launch_bounds__(kThreads, PASS == PASS_NEAREST ? 4 : 1) raster_kernel(const __grid_constant__ RasterArgs a) {
     raster_body<PASS, MV, true>(a);
 }
 
