@@ -1929,6 +1929,15 @@ cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, cudaSt
                                dim3(kThreads), 0, s, a);
 }
 
+// Many points to a pixel meet in their atomics: past this many resident points a
+// pixel the depth plane is drawn by depth_kernel, whose screen tiles send a pixel
+// to the frame once a record.  Terrains, four views: 100M points at 256 x 256
+// 3.88 ms with point_pass and 2.11 so, 20M at 512 x 512 (76 a pixel) 749 and 649
+// us, 5M at 256 x 256 (76) 274 and 254; below, 10M at 512 x 512 (38) 426 and 405
+// but 16 views of square patches 1094 and 1139, 5M at 512 x 512 (19) 263 and 274,
+// 2M at 640 x 512 (6) 172 and 188.
+constexpr uint64_t kDensePoints = 64;
+
 cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUniforms &u,
                             const RasterTargets &t, const float *colors, const float *dldimg,
                             float *grad, cudaStream_t s) {
@@ -1943,7 +1952,9 @@ cr_status launch_raster_f32(cr_cloud *cloud, RasterPass pass, const RasterUnifor
     a.dldimg = dldimg;
     a.fgrad = grad;
     cr_context *ctx = cloud->ctx;
-    if (a.radius_zero) {
+    const bool dense = (uint64_t)cloud->resident * cloud->cap.pointsPerBatch >
+                       kDensePoints * (uint64_t)u.width * (uint64_t)u.height;
+    if (a.radius_zero && !(dense && pass == PASS_DEPTH)) {
         CR_CUDA(pass == PASS_DEPTH       ? launch_point_pass<PASS_DEPTH>(a, ctx, s)
                 : pass == PASS_COLOR_F32 ? launch_point_pass<PASS_COLOR_F32>(a, ctx, s)
                                          : launch_point_pass<PASS_GRAD>(a, ctx, s));
