@@ -37,7 +37,6 @@ struct VariantArgs {
     const cr_raster_file *files;
     InlineFiles ifiles;  // the file table, when small (else n = 0: files)
     int packed;          // two 64-bit adds per sample (not with coverage)
-    int radius_zero;     // every footprint is a single pixel
     const float4 *disp, *prev_disp, *tint;  // null: zeros (prev_disp null: disp)
     uint32_t *depth;
     uint32_t *accum;  // R, G, B, count per pixel
@@ -66,7 +65,8 @@ __device__ __forceinline__ void red_add64(uint32_t *p, uint32_t lo, uint32_t hi)
                  : "memory");
 }
 
-template <bool COLOR>
+// PIXELS: every footprint is a single pixel.
+template <bool COLOR, bool PIXELS>
 __global__ void __launch_bounds__(kThreads, COLOR ? 4 : 6)
     variant_pass(const __grid_constant__ VariantArgs a) {
     // The inline files' transform, world and previous transform.
@@ -82,14 +82,23 @@ __global__ void __launch_bounds__(kThreads, COLOR ? 4 : 6)
     crd::launch_dependents();
     __syncthreads();
     const uint32_t steps = (a.counters[CNT_CHUNK_POINTS] + kThreads - 1) / kThreads;  // a record
-    const uint32_t total = a.counters[CNT_CHUNKS] * steps;
+    const uint32_t nchunks = a.counters[CNT_CHUNKS], total = nchunks * steps;
     const int W = a.u.width, H = a.u.height;
     const crd::PointSize ps{a.u.pointSizeMode, a.u.minimumPointSize, a.u.maximumPointSize,
                             a.u.pointSizeScale};
     const bool mb_on = a.motion_blur > 0.0f;
     const bool oit = a.coverage_mode || mb_on;
     for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
-        const uint32_t k = v / steps, local = (v - k * steps) * kThreads + threadIdx.x;
+        // The CTAs at work together take steps of different records where footprints
+        // are single pixels: those of one record meet in its few pixels' atomics
+        // (10M points at 256 x 256 with coverage: 240 us with a record's steps after
+        // one another, 187 so; 5M at 1080p 132 and 117).  Larger footprints find the
+        // record's pixels in the cache instead (1M points of 4 m splats at 1080p with
+        // motion blur: 915 us, 1000 with steps of different records).
+        const uint32_t outer = v / (PIXELS ? nchunks : steps);
+        const uint32_t inner = v - outer * (PIXELS ? nchunks : steps);
+        const uint32_t k = PIXELS ? inner : outer;
+        const uint32_t local = (PIXELS ? outer : inner) * kThreads + threadIdx.x;
         ChunkRec c;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -140,9 +149,9 @@ __global__ void __launch_bounds__(kThreads, COLOR ? 4 : 6)
             iy = H - 1 - iy;
             if (!COLOR) {
                 const uint32_t depth = crd::depth_to_uint(nz);
-                const int rad = a.radius_zero ? 0
-                                              : crd::footprint_radius(px, py, pz, world, a.u.view,
-                                                                      a.u.proj, H, ps);
+                const int rad = PIXELS ? 0
+                                       : crd::footprint_radius(px, py, pz, world, a.u.view,
+                                                               a.u.proj, H, ps);
                 for (int oy = -rad; oy <= rad; ++oy)
                     for (int ox = -rad; ox <= rad; ++ox) {
                         if (!crd::inside_footprint(ox, oy, rad)) continue;
@@ -177,9 +186,9 @@ __global__ void __launch_bounds__(kThreads, COLOR ? 4 : 6)
                 }
             }
             if (oit && cov <= 0.0f) continue;
-            const int rad = a.radius_zero ? 0
-                                          : crd::footprint_radius(px, py, pz, world, a.u.view,
-                                                                  a.u.proj, H, ps);
+            const int rad = PIXELS ? 0
+                                   : crd::footprint_radius(px, py, pz, world, a.u.view, a.u.proj,
+                                                           H, ps);
             // Motion blur: smear back toward the previous screen position
             // (ColorPass/Shaders.metal:149-171).
             int samples = 1;
@@ -273,7 +282,6 @@ cr_status launch_variant_pass(cr_cloud *cloud, bool color, const RasterUniforms 
     if (!a.ifiles.n)
         if (const cr_status st = ensure_device_files(cloud)) return st;
     a.packed = t.packed;
-    a.radius_zero = fmaxf(u.minimumPointSize, u.maximumPointSize) <= 1.0f ? 1 : 0;
     a.disp = cloud->d_disp;
     a.prev_disp = cloud->d_prev_disp;
     a.tint = cloud->d_tint;
@@ -287,17 +295,15 @@ cr_status launch_variant_pass(cr_cloud *cloud, bool color, const RasterUniforms 
     a.motion_blur = cfg.motionBlur > 0.0f ? cfg.motionBlur : 0.0f;
     a.mb_samples = cfg.motionBlurSamples;
     a.mb_max_spread = cfg.motionBlurMaxSpread;
+    const bool pixels = fmaxf(u.minimumPointSize, u.maximumPointSize) <= 1.0f;
+    const auto kernel = color ? (pixels ? variant_pass<true, true> : variant_pass<true, false>)
+                              : (pixels ? variant_pass<false, true> : variant_pass<false, false>);
     cr_context *ctx = cloud->ctx;
-    int &blocks = ctx->blocks_per_sm_variant[color ? 1 : 0];
-    if (blocks == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &blocks, color ? variant_pass<true> : variant_pass<false>, kThreads, 0) !=
-                cudaSuccess ||
-            blocks < 1)
-            blocks = 1;
-    }
-    const dim3 grid(ctx->sm_count * blocks);
-    CR_CUDA(color ? launch_programmatic(variant_pass<true>, grid, dim3(kThreads), 0, s, a)
-                  : launch_programmatic(variant_pass<false>, grid, dim3(kThreads), 0, s, a));
+    int &blocks = ctx->blocks_per_sm_variant[color ? 1 : 0][pixels ? 1 : 0];
+    if (blocks == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kThreads, 0) !=
+                            cudaSuccess ||
+                        blocks < 1))
+        blocks = 1;
+    CR_CUDA(launch_programmatic(kernel, dim3(ctx->sm_count * blocks), dim3(kThreads), 0, s, a));
     return CR_OK;
 }
