@@ -539,7 +539,13 @@ __global__ void __launch_bounds__(kThreads)
 // NL: the levels there can be (4, the default, or 8): a ballot each in both
 // passes.
 constexpr int kBatchRounds = 4;
-constexpr int kBatchThreads = 512;
+// A warp for every kBatchRounds rounds of the largest batch, up to this many
+// threads (5M points in batches of 64: the pack 3180 us with 512 threads to every
+// batch, 2000 so).
+constexpr uint32_t kBatchThreads = 512;
+uint32_t batch_threads(uint32_t ppb) {
+    return std::min(kBatchThreads, 32u * ((ppb + 32u * kBatchRounds - 1u) / (32u * kBatchRounds)));
+}
 template <int NL, bool ONE>
 __global__ void __launch_bounds__(kBatchThreads)
     pack_batches(const __grid_constant__ Segs segs, const float4 *__restrict__ sorted,
@@ -548,11 +554,10 @@ __global__ void __launch_bounds__(kBatchThreads)
                  uint32_t *__restrict__ low, uint32_t *__restrict__ med,
                  uint32_t *__restrict__ high, uint32_t *__restrict__ colors,
                  uint8_t *__restrict__ levels, uint32_t *__restrict__ src_out) {
-    constexpr int kWarps = kBatchThreads / 32;
     constexpr unsigned kFull = 0xffffffffu;
-    __shared__ uint32_t red[6][kWarps];
-    __shared__ uint32_t wcnt[kWarps][NL];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ uint32_t red[6][kBatchThreads / 32];
+    __shared__ uint32_t wcnt[kBatchThreads / 32][NL];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t si = seg_of<ONE, &PackSeg::batch0>(segs, blockIdx.x);
     const PackSeg &sg = seg_at<ONE>(segs, si);
@@ -561,7 +566,7 @@ __global__ void __launch_bounds__(kBatchThreads)
     const uint32_t total = (uint32_t)min((uint64_t)sg.n - start, (uint64_t)ppb);
     const uint32_t slot = sg.first_slot + batch;
     const uint64_t pool = (uint64_t)slot * ppb;
-    const uint32_t seg = (total + kWarps - 1u) / kWarps;
+    const uint32_t seg = (total + warps - 1u) / warps;
     const uint32_t s0 = min(total, (uint32_t)warp * seg);
     const uint32_t s1 = min(total, (uint32_t)(warp + 1) * seg);
     const float4 *bsorted = sorted + sg.begin + start;
@@ -635,7 +640,7 @@ __global__ void __launch_bounds__(kBatchThreads)
         uint32_t acc = 0;
 #pragma unroll
         for (int L = 0; L < NL; ++L) {
-            const uint32_t x = lane < kWarps ? wcnt[lane][L] : 0u;
+            const uint32_t x = lane < warps ? wcnt[lane][L] : 0u;
             const uint32_t tot = __reduce_add_sync(kFull, x);
             const uint32_t before = __reduce_add_sync(kFull, lane < warp ? x : 0u);
             run[L] = acc + before;
@@ -648,8 +653,8 @@ __global__ void __launch_bounds__(kBatchThreads)
     float bmin[3], size[3], bmax[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        bmin[a] = unflip(__reduce_min_sync(kFull, lane < kWarps ? red[a][lane] : 0xffffffffu));
-        bmax[a] = unflip(__reduce_max_sync(kFull, lane < kWarps ? red[3 + a][lane] : 0u));
+        bmin[a] = unflip(__reduce_min_sync(kFull, lane < warps ? red[a][lane] : 0xffffffffu));
+        bmax[a] = unflip(__reduce_max_sync(kFull, lane < warps ? red[3 + a][lane] : 0u));
         size[a] = fmaxf(bmax[a] - bmin[a], 0.000001f);
     }
     if (threadIdx.x == 0) {
@@ -1056,12 +1061,12 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
     // indices only when asked for.
     uint32_t *src = src_idx_host ? sc.src_idx : nullptr;
     if (L <= 4)
-        PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<4, true>),
+        PACK_LAUNCH(nseg, (unsigned)batches, batch_threads(ppb), s, (pack_batches<4, true>),
                     (pack_batches<4, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, so,
                     cloud->d_batches, cloud->d_low, cloud->d_med,
                     cloud->d_high, cloud->d_colors, cloud->d_levels, src);
     else
-        PACK_LAUNCH(nseg, (unsigned)batches, kBatchThreads, s, (pack_batches<8, true>),
+        PACK_LAUNCH(nseg, (unsigned)batches, batch_threads(ppb), s, (pack_batches<8, true>),
                     (pack_batches<8, false>), arg, sc.sorted, sc.lv_morton, max_level, ppb, so,
                     cloud->d_batches, cloud->d_low, cloud->d_med,
                     cloud->d_high, cloud->d_colors, cloud->d_levels, src);

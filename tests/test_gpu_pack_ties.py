@@ -91,3 +91,19 @@ def test_a_long_run_keeps_every_digit(cr, orc, inside):
     ties = cr.DeviceView(ctx, inside.sort_ties(ctx.handle), (1,), np.uint32).download()
     assert ties[0] == 0
     check_region(cloud, ref, 0, 10240, src)
+
+
+@pytest.mark.parametrize("n,ppb", [(1000, 2), (5000, 127), (5000, 128), (5000, 129), (9000, 1920),
+                                   (9000, 1921), (9000, 2049)])
+@pytest.mark.parametrize("lod", [4, 6])
+def test_batches_by_warps(cr, orc, n, ppb, lod):
+    """Batches on either side of the sizes at which their kernel takes another
+    warp, from one warp to all of them."""
+    ctx = cr.Context(0)
+    rng = np.random.default_rng(n + ppb)
+    pos = rng.uniform(-1.0, 1.0, (n, 3)).astype(np.float32)
+    rgba = rng.integers(0, 1 << 32, n, dtype=np.uint32)
+    ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=ppb, lodLevels=lod,
+                   coarseVoxelDivisions=3)
+    cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, ppb=ppb, lod=lod, divs=3)
+    check_region(cloud, ref, 0, ppb, src)
