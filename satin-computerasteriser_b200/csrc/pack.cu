@@ -506,7 +506,11 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int k = 0; k < kEach; ++k) {
         cell[k] = lod_cell(p[k], a);
-        holder[k] = left[k] ? __ldcg(a.grid + cell[k]) : 0u;
+        // Through L1: the claims are the kernel's before, and of what is written
+        // now, no value but its own index matters to a point.  A pack of 20M points
+        // in one place takes 3.75 ms with the voxels read from L2, 2.41 so; of
+        // 100M points of terrain 8.85 and 8.75.
+        holder[k] = left[k] ? a.grid[cell[k]] : 0u;
     }
 #pragma unroll
     for (int k = 0; k < kEach; ++k) {
@@ -591,7 +595,7 @@ __global__ void __launch_bounds__(kBatchThreads)
 #pragma unroll
             for (int k = 0; k < kBatchRounds; ++k) {
                 cell[k] = lod_cell(p[k], a);
-                holder[k] = l[k] == max_level ? __ldcg(a.grid + cell[k]) : 0xffffffffu;
+                holder[k] = l[k] == max_level ? a.grid[cell[k]] : 0xffffffffu;
             }
 #pragma unroll
             for (int k = 0; k < kBatchRounds; ++k) {

@@ -107,3 +107,19 @@ def test_batches_by_warps(cr, orc, n, ppb, lod):
                    coarseVoxelDivisions=3)
     cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, ppb=ppb, lod=lod, divs=3)
     check_region(cloud, ref, 0, ppb, src)
+
+
+@pytest.mark.parametrize("share", [0.5, 1.0])
+def test_points_in_one_place(cr, orc, inside, share):
+    """Half of the cloud, or all of it, in one place: every sample meets the
+    others, every claim of a level the same voxel."""
+    rng = np.random.default_rng(5)
+    pos = rng.uniform(-1.0, 1.0, (N, 3)).astype(np.float32)
+    pos[rng.permutation(N)[:int(share * N)]] = (0.25, -0.5, 0.125)
+    rgba = rng.integers(0, 1 << 32, N, dtype=np.uint32)
+    ctx = cr.Context(0)
+    ref = orc.pack(pos, colors_rgba8=rgba, pointsPerBatch=10240, morton_bits=21, threads=8)
+    cloud, src = gpu_pack(cr, ctx, pos, rgba=rgba, bits=21)
+    ties = cr.DeviceView(ctx, inside.sort_ties(ctx.handle), (1,), np.uint32).download()
+    assert ties[0] == 0
+    check_region(cloud, ref, 0, 10240, src)
