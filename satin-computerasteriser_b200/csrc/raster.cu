@@ -551,7 +551,7 @@ __device__ __forceinline__ void emit_footprint(const RasterArgs &a, const ViewRe
 }
 
 // A chunk's points are split over the CTA's warps in contiguous pieces of
-// whole 128-point rounds (warp_span points a warp, the same split in every
+// whole rounds (warp_span points a warp, the same split in every
 // pass): each warp packs the fragments of its piece from the piece's own
 // start, counting them in a register, and leaves its count beside the other
 // warps' (kFragWarps per chunk record); the colour pass walks each piece with
@@ -562,8 +562,12 @@ __device__ __forceinline__ void emit_footprint(const RasterArgs &a, const ViewRe
 // points 9.30 -> 9.12 ms.
 constexpr uint32_t kFragWarps = kThreads / 32;
 static_assert(kFragWarps == kFragCounts, "the count arrays have a word per warp");
-__device__ __forceinline__ uint32_t warp_span(uint32_t count) {
-    return 128u * ((count + 128u * kFragWarps - 1u) / (128u * kFragWarps));
+// A round is 128 points, four to a lane, or 32 where the chunk starts unaligned
+// and is read a point to a lane (2M points in batches of 257 at 1080p: 71 us with
+// pieces of 128, 58 so).
+__device__ __forceinline__ uint32_t warp_span(uint32_t first, uint32_t count) {
+    const uint32_t round = (first & 3u) == 0u ? 128u : 32u;
+    return round * ((count + round * kFragWarps - 1u) / (round * kFragWarps));
 }
 
 // Appends the warp's kept points at fragment `at`, lanes placed by ballot
@@ -865,7 +869,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         // 1.0f; 0.5f without dither): (thr - L) + 0.5f only grows as L falls.
         const bool all_keep = (a.u.lodDither ? 1.0f : 0.5f) < (c.thr - 7.0f) + 0.5f;
         // The warp's piece of the chunk and its fragments' place.
-        const uint32_t span = warp_span(c.count), piece = (threadIdx.x >> 5) * span;
+        const uint32_t span = warp_span(c.first, c.count), piece = (threadIdx.x >> 5) * span;
         // Passes without fragments take rounds of the whole CTA in turn.
         constexpr bool kPieces = PASS == PASS_DEPTH_FRAG;
         const uint32_t end = kPieces ? min(piece + span, c.count) : c.count;
@@ -1023,7 +1027,7 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
                                            uint32_t base, int W, const uint32_t *depth) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = __ldg(a.frag_count + slot * kFragWarps + warp);
-    base += warp * warp_span(__ldg(&a.chunks[slot].count));
+    base += warp * warp_span(__ldg(&a.chunks[slot].first), __ldg(&a.chunks[slot].count));
     if ((base & 3u) == 0u) {
         // Two neighbouring fragments per lane and half round: a piece's last
         // round then fills whole half warps before it leaves lanes idle.

@@ -83,3 +83,32 @@ def test_adjoint_after_a_replayed_forward(cr, orc, ctx):
     assert (want > 0).any(1).sum() > 148 * 10240 // 4
     replay()
     assert np.array_equal(adjoint(), want)
+
+
+@pytest.mark.parametrize("chunk", [256, 300, 2048])
+@pytest.mark.parametrize("ppb", [1, 3, 31, 33, 64, 255, 257, 1025, 2051])
+def test_fragments_of_batches_that_start_unaligned(cr, orc, ctx, ppb, chunk):
+    """One-view and batched frames of single pixels, whose fragments each warp
+    packs for the same warp of the colour pass: bit for bit against the oracle."""
+    from test_gpu_render import assert_same, render_both
+    cloud, _ = make_cloud(cr, orc, ctx, *blob_cloud(700 if ppb < 4 else 9000, 12), ppb=ppb)
+    w, h = 97, 61
+    cam = camera(cr, (0.2, 0.1, 1.6), w=w, h=h)
+    cfg = cr.ComputeRasteriserConfiguration(depthTolerance=0.3)
+    before = ctx.tuning()["chunkPoints"]
+    try:
+        ctx.set_tuning(chunkPoints=chunk)
+        _, gpu, ref = render_both(cr, orc, ctx, [cloud], cfg, cam, w, h)
+        assert_same(cr, cfg, gpu, ref)
+        mv = cr.MultiViewRasteriser(ctx, [(w, h)] * 2)
+        mv.configuration = cfg
+        mv.addPointCloud(cloud)
+        mv.render([cam, cam])
+        for v in (0, 1):
+            px = mv.pixels(v)
+            assert np.array_equal(px["depth"], ref.depth)
+            assert np.array_equal(np.stack([px[k] for k in ("red", "green", "blue", "count")], -1),
+                                  ref.accum)
+        mv.close()
+    finally:
+        ctx.set_tuning(chunkPoints=before)
