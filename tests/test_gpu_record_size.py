@@ -112,3 +112,20 @@ def test_fragments_of_batches_that_start_unaligned(cr, orc, ctx, ppb, chunk):
         mv.close()
     finally:
         ctx.set_tuning(chunkPoints=before)
+
+
+@pytest.mark.parametrize("ppb", [1, 4, 16, 255, 256, 257, 260])
+@pytest.mark.parametrize("tiles", [False, True])
+def test_nearest_frames_of_small_records(cr, orc, ctx, ppb, tiles):
+    """Records of as many points as a CTA has threads, fewer and more."""
+    from test_gpu_render import assert_same, render_both
+    cloud, _ = make_cloud(cr, orc, ctx, *blob_cloud(700 if ppb < 4 else 6000, 13), ppb=ppb)
+    try:
+        ctx.set_tuning(useTiles=tiles)
+        for w, h in ((97, 61), (16, 9)):
+            cfg = cr.ComputeRasteriserConfiguration(mode=cr.MODE_NEAREST)
+            _, gpu, ref = render_both(cr, orc, ctx, [cloud], cfg,
+                                      camera(cr, (0.2, 0.1, 1.6), w=w, h=h), w, h)
+            assert_same(cr, cfg, gpu, ref)
+    finally:
+        ctx.set_tuning(useTiles=True)
