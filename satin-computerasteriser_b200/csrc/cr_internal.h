@@ -97,6 +97,7 @@ struct cr_context {
     int blocks_per_sm_views[7] = {};  // the same, batched-view kernels
     int blocks_per_sm_hash_views = 0;  // the batched-view colour hash kernel
     int blocks_per_sm_splat[2] = {};   // the splat depth and colour passes
+    int blocks_per_sm_point[7] = {};   // the FP32 passes of single pixels (per RasterPass)
     int blocks_per_sm_nearest = 0;     // the nearest pass of single-pixel points
     int blocks_per_sm_variant[2][2] = {};  // the colour variants' passes: colour, single pixels
     int chunk_points = 2048;           // points per chunk work record

@@ -1751,15 +1751,6 @@ int resident_blocks(Kernel k, int smem) {
     return n < 1 ? 1 : n;
 }
 
-template <int PASS>
-int point_pass_blocks_per_sm() {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, point_pass<PASS>, kThreads, 0) !=
-        cudaSuccess)
-        n = 1;
-    return n < 1 ? 1 : n;
-}
-
 template <int PASS, bool MV>
 int blocks_per_sm_for() {
     int n = 0;
@@ -1932,10 +1923,11 @@ uint32_t hqs_redo_max_clouds() { return kRedoMaxClouds; }
 
 // A step to a CTA while there are CTAs.
 template <int PASS>
-cudaError_t launch_point_pass(const RasterArgs &a, const cr_context *ctx, cudaStream_t s) {
-    return launch_programmatic(point_pass<PASS>,
-                               dim3(ctx->sm_count * point_pass_blocks_per_sm<PASS>()),
-                               dim3(kThreads), 0, s, a);
+cudaError_t launch_point_pass(const RasterArgs &a, cr_context *ctx, cudaStream_t s) {
+    int &blocks = ctx->blocks_per_sm_point[PASS];
+    if (blocks == 0) blocks = resident_blocks(point_pass<PASS>, 0);
+    return launch_programmatic(point_pass<PASS>, dim3(ctx->sm_count * blocks), dim3(kThreads), 0, s,
+                               a);
 }
 
 // Many points to a pixel meet in their atomics: past this many resident points a
