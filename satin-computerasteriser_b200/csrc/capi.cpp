@@ -466,8 +466,6 @@ CR_API cr_status cr_context_create(int device, cr_context **out) {
         e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->d_status), ctx->h_status, 0);
     if (e != cudaSuccess) {
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
-    if (ctx->h_pick) cudaFreeHost(ctx->h_pick);
-    if (ctx->d_pick) cudaFree(ctx->d_pick);
         cudaStreamDestroy(ctx->stream);
         delete ctx->pack;
         delete ctx;

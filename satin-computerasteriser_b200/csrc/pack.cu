@@ -98,7 +98,6 @@ struct LodArgs {
     float bmin[3];
     float inv;
     uint32_t dims[3];
-    uint32_t level;
     uint32_t *grid;  // this level's voxels
 };
 
@@ -823,7 +822,6 @@ cr_status lod_args(PackSeg &sg, const float bmin[3], const float ext[3], int lev
         if (cells > kLodCellCap)
             return cri::fail(CR_ERR_CAPACITY,
                              "LOD grid of " + std::to_string(cells) + " cells exceeds the cap");
-        a.level = (uint32_t)level;
         total += cells;
     }
     *cells_out = total;

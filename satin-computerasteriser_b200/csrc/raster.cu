@@ -75,13 +75,22 @@ struct TileCfg<PASS_DEPTH_FRAG> {
     static constexpr int kPx = 4096;
     static constexpr int kBytes = kPx * 4;
 };
-template <>
-struct TileCfg<PASS_COLOR_F32> {  // no screen tiles
-    static constexpr int kPx = 0;
-    static constexpr int kBytes = 0;
-};
-template <>
-struct TileCfg<PASS_GRAD> : TileCfg<PASS_COLOR_F32> {};
+// The kernels that draw footprints of more than a pixel only, and so have no
+// screen tiles: other kernels draw single pixels in the nearest pass (FP false),
+// the one-view colour pass (from fragments), the batched views' depth pass (with
+// fragments) and the FP32 passes.
+template <int PASS, bool MV, bool FP>
+__host__ __device__ constexpr bool footprints_only() {
+    return (PASS == PASS_NEAREST && FP) || (PASS == PASS_COLOR && !MV) ||
+           (PASS == PASS_DEPTH && MV) || PASS == PASS_COLOR_F32 || PASS == PASS_GRAD;
+}
+template <int PASS, bool MV>
+constexpr int tile_bytes() {
+    if constexpr (footprints_only<PASS, MV, true>())
+        return 0;
+    else
+        return TileCfg<PASS>::kBytes;
+}
 
 __host__ __device__ constexpr bool is_depth(int p) { return p == PASS_DEPTH || p == PASS_DEPTH_FRAG; }
 __host__ __device__ constexpr bool is_color(int p) { return p == PASS_COLOR; }
@@ -461,15 +470,6 @@ __device__ __forceinline__ void emit_direct(const RasterArgs &a, const ViewRegsT
         if (vis)
             color_global<MV>(a, vr, pix, o.color & 0xffu, (o.color >> 8) & 0xffu, (o.color >> 16) & 0xffu,
                          1u);
-    } else if (PASS == PASS_COLOR_F32 || PASS == PASS_GRAD) {
-        const uint32_t closest = o.ok ? vdepth<MV>(vr)[pix] : 0u;
-        const bool vis = closest != 0u && o.nz >= crd::uint_to_depth(closest) * a.keep_scale;
-        if (PASS == PASS_COLOR_F32 && vis) color_f32_sample(a, pix, o.pointIndex);
-        if (PASS == PASS_GRAD && vis) {
-            float g[3] = {0.0f, 0.0f, 0.0f};
-            grad_sample(a, pix, g);
-            grad_store(a, o.pointIndex, g);
-        }
     } else {
         if (o.ok) red_max_u64(&vnearest<MV>(vr)[pix], nearest_key(o.depth, o.pointIndex));
     }
@@ -602,12 +602,16 @@ __device__ __forceinline__ void do_point(const RasterArgs &a, const ViewRegsT<MV
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
     project_point<PASS, MV>(a, vr, sb.T, c, lo, me, hi, o);
     if (!is_depth(PASS) && !__any_sync(kFull, o.ok)) return;
-    if (FP && !a.radius_zero)
+    if constexpr (footprints_only<PASS, MV, FP>()) {
         emit_footprint<PASS, MV>(a, vr, sb, o);
-    else if (tiled)
-        emit_tile<PASS, MV>(a, vr, c, smem, o);
-    else
-        emit_direct<PASS, MV>(a, vr, o);
+    } else {
+        if (FP && !a.radius_zero)
+            emit_footprint<PASS, MV>(a, vr, sb, o);
+        else if (tiled)
+            emit_tile<PASS, MV>(a, vr, c, smem, o);
+        else
+            emit_direct<PASS, MV>(a, vr, o);
+    }
     if (PASS == PASS_DEPTH_FRAG && emit) frag_at += emit_fragment(a, frag_at, o);
 }
 
@@ -815,10 +819,11 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         cp_async_commit();
         const uint32_t file_id = MV ? cur_view * a.nfiles + c.file : c.file;
         const bool new_file = file_id != sb.file;
-        const bool tiled = a.use_tiles && a.radius_zero && c.tw > 0 &&
-                           c.tw * c.th <= TileCfg<PASS>::kPx &&
-                           c.tw * c.th <= (int)c.count &&
-                           (!is_color(PASS) || c.count < 4096u);
+        bool tiled = false;
+        if constexpr (!footprints_only<PASS, MV, FP>())
+            tiled = a.use_tiles && a.radius_zero && c.tw > 0 &&
+                    c.tw * c.th <= TileCfg<PASS>::kPx && c.tw * c.th <= (int)c.count &&
+                    (!is_color(PASS) || c.count < 4096u);
         if (new_file || tiled) {
             __syncthreads();  // everyone has read sb.file (and the view state)
             if (new_file) {
@@ -851,7 +856,8 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
                 loaded_view = cur_view;
                 if (tiled) __syncthreads();  // the tile's set-up reads the view state
             }
-            if (tiled) tile_init<PASS, MV>(a, c, smem);
+            if constexpr (!footprints_only<PASS, MV, FP>())
+                if (tiled) tile_init<PASS, MV>(a, c, smem);
             __syncthreads();
         }
         // The view's size and planes: registers (batched views, read once
@@ -954,10 +960,11 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         }
         if (PASS == PASS_DEPTH_FRAG && (threadIdx.x & 31) == 0)
             a.frag_count[fslot * kFragWarps + (threadIdx.x >> 5)] = frag_at - frag0;
-        if (tiled) {
-            __syncthreads();
-            tile_flush<PASS, MV>(a, vr, c, smem);
-        }
+        if constexpr (!footprints_only<PASS, MV, FP>())
+            if (tiled) {
+                __syncthreads();
+                tile_flush<PASS, MV>(a, vr, c, smem);
+            }
     }
     cp_async_wait_all();
     finish();
@@ -1598,8 +1605,8 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
 }
 
 // The nearest pass of larger footprints asks for four CTAs per SM: left to the
-// compiler it has 48 registers, some spilled, and 5M points of 4 m splats at
-// 1080p take 1268 us, 1052 so (1028 at three, but 20M points of 0.5 m splats 161
+// compiler it had 48 registers, some spilled, and 5M points of 4 m splats at
+// 1080p took 1268 us, 1052 so (1028 at three, but 20M points of 0.5 m splats 161
 // instead of 147).
 template <int PASS, bool MV>
 __global__ void __launch_bounds__(kThreads, PASS == PASS_NEAREST ? 4 : 1) raster_kernel(const __grid_constant__ RasterArgs a) {
@@ -1701,7 +1708,7 @@ __global__ void __launch_bounds__(kThreads, 6)
 }
 
 // The one-view depth passes fit 64 registers without spilling, so four CTAs
-// (and their 32 KB screen tiles) share an SM.
+// (and their screen tiles, 16 KB with fragments and 32 without) share an SM.
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 4) depth_kernel(const __grid_constant__ RasterArgs a) {
     raster_body<PASS, false, PASS != PASS_DEPTH_FRAG>(a);
@@ -1709,16 +1716,17 @@ __global__ void __launch_bounds__(kThreads, 4) depth_kernel(const __grid_constan
 
 // The batched-view depth passes at five CTAs per SM (48 registers, a dozen
 // spilled): 64 views of 50M points 8.83 ms, 9.05 ms at four, 9.13 ms with the
-// chunk record in registers (9.41 ms at five).
+// chunk record in registers (9.41 ms at five).  With footprints 16 views of 20M
+// points 2.86 ms, 2.88 at four.
 template <int PASS>
 __global__ void __launch_bounds__(kThreads, 5)
     depth_views_kernel(const __grid_constant__ RasterArgs a) {
     raster_body<PASS, true, PASS != PASS_DEPTH_FRAG>(a);
 }
 
-// The colour pass that decodes the points holds a 64 KB screen tile, so at
-// most three CTAs share an SM whatever their registers; saying so lets the
-// compiler use up to 85 registers per thread instead of spilling.
+// The batched views' colour pass that decodes the points holds a 64 KB screen
+// tile, so at most three CTAs share an SM whatever their registers; saying so
+// lets the compiler use up to 85 registers per thread instead of spilling.
 template <bool MV>
 __global__ void __launch_bounds__(kThreads, 3) raster_kernel_color(const __grid_constant__ RasterArgs a) {
     raster_body<PASS_COLOR, MV, true>(a);
@@ -1755,9 +1763,9 @@ template <int PASS, bool MV>
 int blocks_per_sm_for() {
     int n = 0;
     constexpr auto k = kernel_for<PASS, MV>();
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TileCfg<PASS>::kBytes);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, TileCfg<PASS>::kBytes) !=
-        cudaSuccess)
+    constexpr int kBytes = tile_bytes<PASS, MV>();
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, kBytes) != cudaSuccess)
         n = 1;
     return n < 1 ? 1 : n;
 }
@@ -1835,10 +1843,10 @@ RasterArgs make_args(cr_cloud *cloud, const RasterUniforms &u, const RasterTarge
 template <int PASS, bool MV>
 void launch_pass(const RasterArgs &a, int grid, cudaStream_t s) {
     if constexpr (MV)
-        kernel_for<PASS, MV>()<<<grid, kThreads, TileCfg<PASS>::kBytes, s>>>(a);
+        kernel_for<PASS, MV>()<<<grid, kThreads, (tile_bytes<PASS, MV>()), s>>>(a);
     else
         launch_programmatic(kernel_for<PASS, MV>(), dim3(grid), dim3(kThreads),
-                            (size_t)TileCfg<PASS>::kBytes, s, a);
+                            (size_t)tile_bytes<PASS, MV>(), s, a);
 }
 
 }  // namespace
