@@ -1021,19 +1021,15 @@ def run_packer(args, cr, ctx, torch, dist):
     cloud.close()
     ctx.trim()
     bit_exact = pack_parity(args, cr, ctx) if args.pack_check_points > 0 else None
-    # Bytes per point of a pack that sorts every digit (63-bit keys, 4 LOD
-    # levels; a yardstick: the packer leaves out digits that all keys share
-    # and low ones that few keys need, and moves fewer): 8 radix passes
-    # moving a 64-bit key and a 32-bit index in and out (192 B), the gather
-    # (16 B in, 12 B of sorted position out), 3 LOD levels (12 B each), the
-    # quantisation (12 B in, 12 B out) and the colour (4 B): 284 B.
-    bpp = 8 * 2 * (8 + 4) + (16 + 12) + 3 * 12 + (12 + 12) + 4
+    # Bytes per point that a pack cannot do without: the 16-byte record in, and
+    # three words, the colour and the level byte out.
+    bpp = 16 + 12 + 4 + 1
     peak, peak_kind = measured_peaks()
     achieved = n * bpp / (ms / 1e3) / 1e9
     return {"points": n, "morton_bits": 63, "batches": int(len(res)),
             "pack_ms": round(ms, 2), "gpts_per_s": round(n / (ms / 1e3) / 1e9, 3),
             "roofline": {"bound": "hbm", "bytes_per_point": bpp,
-                         "bytes_model": "a pack that sorts all eight digits",
+                         "bytes_model": "each record read once, each packed point written once",
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "peak_source": peak_kind},
             "checks": checks, "bit_exact": bit_exact,
