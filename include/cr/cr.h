@@ -527,7 +527,8 @@ CR_API cr_status cr_host_free(void *host_ptr);
 /* Per-pass timing (the reference's labelled encoders, ComputeRasteriser.swift:379-428) */
 /* ------------------------------------------------------------------------ */
 typedef enum cr_pass_id {
-    CR_PASS_CLEAR = 0,
+    CR_PASS_CLEAR = 0,   /* frames with no cloud to cull; the planes are cleared in the
+                          * cull's launch otherwise, in both modes */
     CR_PASS_CULL = 1,
     CR_PASS_DEPTH = 2,   /* HQS depth, or the fused nearest depth/index pass */
     CR_PASS_COLOR = 3,
@@ -551,8 +552,9 @@ CR_API cr_status cr_context_pass_times(cr_context *ctx, int32_t nframes, float *
 /* Launch tuning of the point passes                                         */
 /* ------------------------------------------------------------------------ */
 /* chunkPoints: most survivor points per work record of the depth / colour /
- * nearest passes (>= 256; a small cloud's records have fewer); useTiles: accumulate compact batches in
- * shared-memory screen tiles.  Results do not depend on either value. */
+ * nearest passes (>= 256; a small cloud's records have fewer); useTiles:
+ * accumulate compact batches in shared-memory screen tiles.  Results do not
+ * depend on either value. */
 typedef struct cr_tuning {
     int32_t chunkPoints;     /* default 2048 */
     int32_t useTiles;        /* default 1    */

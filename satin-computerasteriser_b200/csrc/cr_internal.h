@@ -320,7 +320,11 @@ struct CullArgs {
 
 // Launches a kernel that may begin while the previous kernel on the stream
 // finishes (programmatic stream serialisation); the kernel orders itself
-// after that kernel with crd::grid_wait().
+// after that kernel with crd::grid_wait().  What it reads before that wait must
+// not be written by any kernel that the stream may run before it without a copy
+// or a synchronisation in between.  The cull reads the batch records and the file
+// table so (cull.cu): a new kernel that writes either has to be followed by
+// one, as the packer is by the copy of its batches to the host.
 template <typename... Params, typename... Args>
 cudaError_t launch_programmatic(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                                 cudaStream_t s, Args &&...args) {
