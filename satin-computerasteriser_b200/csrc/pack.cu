@@ -994,12 +994,14 @@ cr_status pack_wave(cr_context *ctx, cr_cloud *cloud, const PackJob *jobs, uint3
         }
         if ((refused = lod_args(sg, bmin, ext, L, divs, &cells[j]))) break;
         // Grids of several jobs together: in the memory that there is, or in new
-        // memory up to the wave's share.
+        // memory up to the wave's share (asked for only where it can decide: 200
+        // nodes in several waves 2350 us a call with a query in each, 2140 without).
+        if (j > 0 && cell_sum + cells[j] > std::max(sc.cap_grid, kLodCellCap)) break;
         if (j > 0 && cell_sum + cells[j] > sc.cap_grid) {
             if (cell_limit == 0) {
                 uint64_t bytes = 0;
                 if ((st = wave_share(&bytes))) return st;
-                cell_limit = std::max(sc.cap_grid, std::min(kLodCellCap, bytes / 4));
+                cell_limit = std::max(sc.cap_grid, bytes / 4);
             }
             if (cell_sum + cells[j] > cell_limit) break;
         }
