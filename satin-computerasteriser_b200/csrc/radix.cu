@@ -418,8 +418,8 @@ __global__ void __launch_bounds__(kThreads, kSortBlocksPerSM)
         // inclusive prefix; a word not yet published is polled (bounded).
         constexpr unsigned long long kCountMask = (1ull << 46) - 1ull;
         bool gave_up = wait_limit == 0u;
-        int64_t t = (int64_t)tile - 1;
-        while (t >= 0 && !gave_up) {
+        int64_t t = gave_up ? -1 : (int64_t)tile - 1;
+        while (t >= 0) {
             const int nb = t + 1 < kLookbackBatch ? (int)(t + 1) : kLookbackBatch;
             unsigned long long v[kLookbackBatch];
 #pragma unroll
