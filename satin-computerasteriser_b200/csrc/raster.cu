@@ -134,7 +134,8 @@ struct RasterArgs {
     F2Consts two;      // 1 and -0, twice each
     int radius_zero;   // every footprint is a single pixel
     int use_tiles;
-    uint32_t *frag_xy;  // pixel x | row << 16
+    uint32_t round_shift;  // of the fragment passes' rounds (warp_span)
+    uint32_t *frag_xy;     // pixel x | row << 16
     uint2 *frag_zc;     // NDC z bits, RGBA8: two stores per fragment
     uint32_t *frag_count;
     // Differentiable colours: learnable colours, dL/dpixel, gradient (3 floats each).
@@ -562,12 +563,13 @@ __device__ __forceinline__ void emit_footprint(const RasterArgs &a, const ViewRe
 // points 9.30 -> 9.12 ms.
 constexpr uint32_t kFragWarps = kThreads / 32;
 static_assert(kFragWarps == kFragCounts, "the count arrays have a word per warp");
-// A round is 128 points, four to a lane, or 32 where the chunk starts unaligned
-// and is read a point to a lane (2M points in batches of 257 at 1080p: 71 us with
-// pieces of 128, 58 so).
-__device__ __forceinline__ uint32_t warp_span(uint32_t first, uint32_t count) {
-    const uint32_t round = (first & 3u) == 0u ? 128u : 32u;
-    return round * ((count + round * kFragWarps - 1u) / (round * kFragWarps));
+// A round is 128 points, four to a lane, or 32 where pointsPerBatch is no
+// multiple of four: most batches then start unaligned and are read a point to a
+// lane (2M points in batches of 257 at 1080p: 71 us with pieces of 128, 58 so).
+// round_shift: its logarithm, the same for all of a cloud's passes.
+__device__ __forceinline__ uint32_t warp_span(uint32_t round_shift, uint32_t count) {
+    static_assert(kFragWarps == 8, "a round for every warp is eight rounds");
+    return (((count - 1u) >> (round_shift + 3)) + 1u) << round_shift;
 }
 
 // Appends the warp's kept points at fragment `at`, lanes placed by ballot
@@ -875,7 +877,7 @@ __device__ __forceinline__ void raster_body(const RasterArgs &a) {
         // 1.0f; 0.5f without dither): (thr - L) + 0.5f only grows as L falls.
         const bool all_keep = (a.u.lodDither ? 1.0f : 0.5f) < (c.thr - 7.0f) + 0.5f;
         // The warp's piece of the chunk and its fragments' place.
-        const uint32_t span = warp_span(c.first, c.count), piece = (threadIdx.x >> 5) * span;
+        const uint32_t span = warp_span(a.round_shift, c.count), piece = (threadIdx.x >> 5) * span;
         // Passes without fragments take rounds of the whole CTA in turn.
         constexpr bool kPieces = PASS == PASS_DEPTH_FRAG;
         const uint32_t end = kPieces ? min(piece + span, c.count) : c.count;
@@ -1039,7 +1041,7 @@ __device__ __forceinline__ void hash_frags(const RasterArgs &a, const ViewRegsT<
                                            uint32_t base, int W, const uint32_t *depth) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = __ldg(a.frag_count + slot * kFragWarps + warp);
-    base += warp * warp_span(__ldg(&a.chunks[slot].first), __ldg(&a.chunks[slot].count));
+    base += warp * warp_span(a.round_shift, __ldg(&a.chunks[slot].count));
     if ((base & 3u) == 0u) {
         // Two neighbouring fragments per lane and half round: a piece's last
         // round then fills whole half warps before it leaves lanes idle.
@@ -1550,6 +1552,7 @@ struct RedoCloud {
     const ChunkRec *chunks;
     const uint32_t *counters, *frag_count, *frag_xy;
     const uint2 *frag_zc;
+    uint32_t round_shift;
 };
 constexpr uint32_t kRedoMaxClouds = 32;
 struct RedoArgs {
@@ -1579,6 +1582,7 @@ __global__ void __launch_bounds__(kThreads) hqs_redo_kernel(RedoArgs r) {
         a.frag_count = const_cast<uint32_t *>(r.clouds[ci].frag_count);
         a.frag_xy = const_cast<uint32_t *>(r.clouds[ci].frag_xy);
         a.frag_zc = const_cast<uint2 *>(r.clouds[ci].frag_zc);
+        a.round_shift = r.clouds[ci].round_shift;
         const ViewRegsT<false> vr(a);
         const uint32_t nchunks = r.clouds[ci].counters[CNT_CHUNKS];
         if (r.splats) {
@@ -1822,6 +1826,7 @@ RasterArgs make_args(cr_cloud *cloud, const RasterUniforms &u, const RasterTarge
     // upper bound is 1 every radius is 0 whatever the distance.
     a.radius_zero = fmaxf(u.minimumPointSize, u.maximumPointSize) <= 1.0f ? 1 : 0;
     a.use_tiles = cloud->ctx->use_tiles ? 1 : 0;
+    a.round_shift = cloud->cap.pointsPerBatch % 4u == 0u ? 7u : 5u;
     a.frag_xy = cloud->d_frag_xy;
     a.frag_zc = cloud->d_frag_zc;
     a.frag_count = cloud->d_frag_count;
@@ -1913,7 +1918,8 @@ cr_status launch_hqs_redo(cr_frame *f, cr_cloud *const *clouds, uint32_t nclouds
     r.a = make_args(clouds[0], u, t);
     for (uint32_t i = 0; i < nclouds; ++i) {
         r.clouds[i] = RedoCloud{clouds[i]->d_chunks,   clouds[i]->d_counters, clouds[i]->d_frag_count,
-                                clouds[i]->d_frag_xy, clouds[i]->d_frag_zc};
+                                clouds[i]->d_frag_xy, clouds[i]->d_frag_zc,
+                                make_args(clouds[i], u, t).round_shift};
     }
     r.splats = splats ? 1 : 0;
     r.nclouds = nclouds;
